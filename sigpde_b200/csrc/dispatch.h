@@ -85,21 +85,27 @@ size_t dgemm_inc_pipe_smem(int64_t d);
 // null for dim > 32
 // out64: float64 matrix (float64 cells), else float32 (float32 cells)
 StaticIncFn get_static_inc_kernel(int kind, int64_t dim, bool out64);
-// backward pass (grad.cuh): forward-with-derivatives and adjoint wavefronts for R rows a lane,
-// order O (R >= 2^O); null members where the combination is not built
+// backward pass (grad.cuh): recording forward and adjoint wavefronts for R rows and `cols` columns a
+// lane step at order O (R >= 2^O), ccols coarse columns a step; null members where not built
 struct GradFns {
     void (*fwd)(GradParams);
     void (*bwd)(GradParams);
+    int cols, ccols, ctas; // ctas: resident CTAs per SM
+    int rec;               // doubles of a warp step's record
+    size_t bwd_smem;       // dynamic shared memory of bwd
 };
-GradFns get_grad_kernels(int R, int O);
+// wide: steps of twice the columns (null where not built)
+GradFns get_grad_kernels(int R, int O, bool wide);
 struct GradAuxFns {
     void (*pair_inc)(const double *, const double *, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, double *);
     void (*gx)(GradContractParams);
     void (*gy)(GradContractParams);
     void (*reduce)(const double *, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, double *);
     void (*points)(const double *, int64_t, int64_t, int64_t, double, const void *, int, void *);
-    void (*rows)(const double *, int64_t, int64_t, int64_t, int64_t, double *);
+    void (*rows)(const double *, int64_t, int64_t, int64_t, int64_t, int, double *);
+    void (*gx_gram)(GradContractParams);
     void (*gy_gram)(GradContractParams);
+    void (*gy_reduce)(const double *, int64_t, int64_t, double *);
     void (*inc_blocks)(const void *, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t,
                        const void *, const void *, double *, void *, int);
 };

@@ -15,18 +15,16 @@
 //   A'(c) = 1/2 + c/6,  B'(c) = -c/6.
 //
 // Kernels
-//   grad_fwd_kernel  one warp per pair: the forward wavefront (R rows a lane,
-//                    one fine column a step, bands of 32R rows) storing the
-//                    top input of every lane step and each lane's rows at the
-//                    start of every segment of T = 32/R steps;
-//   grad_bwd_kernel  one warp per pair: per segment (last first), each lane
-//                    recomputes its rows' K and D over the segment on its own
-//                    (no cross-lane dependency: its inputs were stored), then
-//                    the adjoint runs the same schedule in reverse for
-//                    Lambda, summing Lambda D per coarse cell; each coarse
-//                    cell's rows belong to one lane (R >= 2^order), so the
-//                    sum is written once, over the cell's increment in the
-//                    increment matrix (which then holds dk/dc);
+//   grad_fwd_kernel  the forward wavefront over a run of pairs a warp, writing
+//                    what enters every lane step: the values above the
+//                    lane's block, left of it and above-left of it;
+//   grad_bwd_kernel  the same lane steps in reverse time: each lane recomputes
+//                    its block's D from that record alone (no other lane is
+//                    asked), then runs the adjoint over the block, summing
+//                    Lambda D per coarse cell; each coarse cell's rows belong
+//                    to one lane (R >= 2^order), so the sum is written once,
+//                    over the cell's increment in the increment matrix (which
+//                    then holds dk/dc);
 //   grad_gx_kernel / grad_gy_kernel   contractions of dk/dc with the scaled
 //                    differences of the other side: the gradients with
 //                    respect to the coarse differences;
@@ -45,274 +43,538 @@ struct GradParams {
     int64_t ncx, ncy;
     int order;
     int64_t nitems;       // pairs in this chunk
+    int64_t per_warp;     // pairs a warp (a contiguous run)
+    int nb, nsteps, period; // bands a pair, lane steps a band, steps from one band's start to the next
     int64_t ny;           // Gram: y paths
     const void *w;        // weights (grad_out): pairwise (n,), Gram (n_x, n_y) row-major; input dtype
     int in64;
     int64_t x0;           // first x path of the chunk
-    double *dbuf;         // per pair and band grad_band_doubles(m, R): top inputs and segment checkpoints
-    double *bnd;          // per pair 2 * (m + 2) doubles: band boundary rows
+    double *rec;          // per warp grad_warp_steps(...) records of what enters its lane steps
+    double *bnd;          // per warp bnd_stride doubles: rows handed from band to band
+    int64_t bnd_stride;
+    int bnd_smem;         // forward: those rows are in dynamic shared memory instead
 };
 
-// pair `it` of the chunk: its x path (global), y path, and its increment block
-__device__ __forceinline__ void grad_item(const GradParams &p, int64_t it, int64_t &xi, int64_t &yj, double *&base,
-                                          int64_t &row_ld)
+// Lane-step shape.  A lane owns R rows and takes C columns a step: the cells of
+// an R x C block are independent along anti-diagonals, and a step's loads,
+// shuffles, control and record are paid once for all of them (one column a step
+// with the same R spent 33 instructions a cell, 10 of them float64; the adjoint
+// then ran at 35% of the float64 pipe).  A block's D stays in registers: 32
+// cells at three CTAs an SM (W = 1), or 64 at two (W = 2, long runs: 128 x 128
+// pairs, L = 128, order 2 run 4.12 + 2.25 ms backward + forward against
+// 4.64 + 3.13, with 4 columns; short runs pay the wider pipeline fill).  Orders
+// 3 and 4 may split a coarse column over several steps; orders 0 and 1 take
+// several whole coarse columns a step.
+template <int R, int O, int W>
+struct GradShape {
+    static constexpr int C = (O == 0 || O == 4) ? 2 : 4 * W;
+    static constexpr int RC = R >> O;                        // coarse rows a lane
+    static constexpr int CC = (C >> O) > 0 ? (C >> O) : 1;   // coarse columns a step
+    static constexpr bool WHOLE = (C >> O) > 0;              // steps hold whole coarse columns
+    static constexpr int NV2 = (R + C) / 2;                  // 16-byte parts of a lane step's record
+    static constexpr int REC = NV2 * 64 + 32;                // doubles of a warp step's record
+    static constexpr int INC = CC * RC * 32;                 // doubles of a warp step's increments
+    static constexpr int CTAS = W == 1 ? 3 : 2;              // resident CTAs an SM
+    static_assert(R >= (1 << O) && R % 2 == 0 && C % 2 == 0, "a lane's rows hold whole coarse rows");
+    __host__ __device__ static constexpr int cc_of(int c) { return CC == 1 ? 0 : c >> O; }
+};
+
+// Warp schedule, shared by both kernels (the backward kernel runs it in
+// reverse).  A warp walks a run of pairs, each in nb bands of 32 R rows; lane
+// l does step q of the run's v-th band at warp step s = v * period + q + l, so
+// the lane pipeline does not drain between bands and pairs.  A band needs the
+// row that lane 31 of the band above wrote 31 steps after lane 0 took the same
+// columns: with several bands the period is at least kGradMinPeriod, which
+// leaves room to load that row one step ahead.
+constexpr int kGradMinPeriod = 34;
+constexpr int kGradFwdRing = 4; // steps of increments in shared memory: one in use, three in flight
+constexpr int kGradRing = 3;    // backward: one step of records and increments in use, two in flight
+
+__host__ __device__ __forceinline__ int64_t grad_warp_steps(int64_t pairs, int nb, int period)
 {
-    if (p.op == kOpPairwise) {
-        xi = p.x0 + it;
-        yj = xi;
-        base = p.mat + it * p.ncy * p.rows_x;
-        row_ld = p.rows_x;
-    } else {
-        const int64_t il = it / p.ny;
-        xi = p.x0 + il;
-        yj = it - il * p.ny;
-        base = p.mat + yj * p.ncy * p.ld + il * p.rows_x;
-        row_ld = p.ld;
-    }
+    return pairs * nb * period + 31;
 }
 
-// Steps per recompute segment: T * R = 32 doubles of D per lane in shared memory.
-template <int R>
-constexpr int grad_seg() { return 32 / R; }
-
-// Per pair and band, the forward pass stores what the adjoint needs to
-// recompute any segment of T steps lane by lane: the top input K(p0-1, q)
-// each lane used at every step ([step][lane]) and each lane's K(rows, q-1)
-// at the start of every segment ([segment][row][lane]).
-__host__ __device__ __forceinline__ int64_t grad_band_doubles(int m, int R)
+template <int R, int O, int W>
+constexpr size_t grad_bwd_smem()
 {
-    const int64_t S = m + 31, T = 32 / R, NS = (S + T - 1) / T;
-    return S * 32 + NS * R * 32;
+    using GS = GradShape<R, O, W>;
+    return (size_t)kWarpsPerBlock * kGradRing * (GS::REC + GS::INC) * sizeof(double);
 }
 
-// Coefficients of the lane's coarse rows for coarse column cj.
-template <int RC>
-__device__ __forceinline__ void grad_coefs(const double *base, int64_t row_ld, int ci0, int64_t ncx, int cj,
-                                           double (&A)[RC], double (&B)[RC], double (&Ad)[RC], double (&Bd)[RC])
-{
-#pragma unroll
-    for (int rc = 0; rc < RC; ++rc) {
-        const int ci = ci0 + rc;
-        const double c = ci < ncx ? base[(int64_t)cj * row_ld + ci] : 0.0;
-        stencil_coefs(c, A[rc], B[rc]);
-        Ad[rc] = fma(c, 1.0 / 6.0, 0.5);
-        Bd[rc] = c * (-1.0 / 6.0);
-    }
-}
-
-// One forward step of the lane's R rows at a column: left holds K(rows, q-1)
-// and becomes K(rows, q); D of each row goes to d[r * 32].  Rows beyond n
-// (coarse rows >= ncx, c = 0) copy row n and carry Lambda = 0 in the adjoint:
-// they need no masking.
-template <int R, int O, bool WANT_D>
-__device__ __forceinline__ void grad_lane_step(double (&left)[R], double top, double diag, const double *A,
-                                               const double *B, const double *Ad, const double *Bd, double *d)
-{
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int rc = r >> O;
-        const double sum = left[r] + top;
-        const double k = sum * A[rc] - diag * B[rc];
-        if constexpr (WANT_D) d[r * 32] = sum * Ad[rc] - diag * Bd[rc];
-        diag = left[r];
-        left[r] = k;
-        top = k;
-    }
-}
+// A lane's place in the warp's run: step q of the period (idle from nsteps on),
+// band b and pair (yj, and the first of its own coarse rows in the pair's
+// increment block).
+struct GradPos {
+    int q, b;
+    int64_t yj;
+    double *rows; // increment (ci0, 0) of the band's coarse rows ci0 of this lane
+    int ci0;
+};
 
 template <int R, int O>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) grad_fwd_kernel(GradParams p)
+__device__ __forceinline__ GradPos grad_pos(const GradParams &p, int64_t it, int b, int q, int lane)
 {
-    static_assert(R >= (1 << O), "a lane's rows hold whole coarse rows");
-    constexpr int RC = R >> O;
-    constexpr int T = grad_seg<R>();
-    const int lane = threadIdx.x & 31;
-    const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int n = (int)(p.ncx << p.order), m = (int)(p.ncy << p.order);
-    const int nb = (n + 32 * R - 1) / (32 * R);
-    const int S = m + 31;
-    const int64_t band_doubles = grad_band_doubles(m, R);
-    for (int64_t it = gwarp; it < p.nitems; it += nwarps) {
-        int64_t xi, yj, row_ld;
-        double *base;
-        grad_item(p, it, xi, yj, base, row_ld);
-        double *bnd = p.bnd + it * 2 * (int64_t)(m + 2); // K of the row above the band, columns 0..m
-        for (int b = 0; b < nb; ++b) {
-            double *tops = p.dbuf + (it * nb + b) * band_doubles + lane;
-            double *ck = tops + (int64_t)S * 32;
-            const int p0 = b * 32 * R + lane * R + 1; // this lane's first fine row (1-based)
-            const int ci0 = (p0 - 1) >> O;            // its first coarse row
-            double left[R];
+    GradPos w;
+    const int64_t xi = p.op == kOpPairwise ? it : it / p.ny;
+    w.yj = p.op == kOpPairwise ? 0 : it - xi * p.ny;
+    w.q = q;
+    w.b = b;
+    w.ci0 = ((b * 32 + lane) * R) >> O;
+    w.rows = (p.op == kOpPairwise ? p.mat + it * p.ncy * p.rows_x : p.mat + w.yj * p.ncy * p.ld + xi * p.rows_x) + w.ci0;
+    return w;
+}
+
+// the band after (q is the caller's)
+template <int R, int O>
+__device__ __forceinline__ void grad_next_band(const GradParams &p, GradPos &w, int lane)
+{
+    w.rows += (32 * R) >> O;
+    w.ci0 += (32 * R) >> O;
+    if (++w.b < p.nb) return;
+    w.b = 0;
+    w.rows -= w.ci0; // back to the pair's first rows
+    w.ci0 = (lane * R) >> O;
+    w.rows += w.ci0;
+    if (p.op == kOpPairwise) {
+        w.rows += p.ncy * p.rows_x;
+    } else if (++w.yj < p.ny) {
+        w.rows += p.ncy * p.ld;
+    } else {
+        w.yj = 0;
+        w.rows += p.rows_x - (p.ny - 1) * p.ncy * p.ld;
+    }
+}
+
+// the band before
+template <int R, int O>
+__device__ __forceinline__ void grad_prev_band(const GradParams &p, GradPos &w, int lane)
+{
+    w.rows -= (32 * R) >> O;
+    w.ci0 -= (32 * R) >> O;
+    if (--w.b >= 0) return;
+    w.b = p.nb - 1;
+    w.rows -= w.ci0;
+    w.ci0 = ((w.b * 32 + lane) * R) >> O;
+    w.rows += w.ci0;
+    if (p.op == kOpPairwise) {
+        w.rows -= p.ncy * p.rows_x;
+    } else if (--w.yj >= 0) {
+        w.rows -= p.ncy * p.ld;
+    } else {
+        w.yj = p.ny - 1;
+        w.rows += (p.ny - 1) * p.ncy * p.ld - p.rows_x;
+    }
+}
+
+__device__ __forceinline__ void grad_cp_async16(void *dst, const void *src)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(src) : "memory");
+}
+
+// n bytes copied, the rest of the 16 (8) filled with 0
+__device__ __forceinline__ void grad_cp_async16z(void *dst, const void *src, int n)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(n) : "memory");
+}
+
+__device__ __forceinline__ void grad_cp_async8z(void *dst, const void *src, int n)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(a), "l"(src), "r"(n) : "memory");
+}
+
+// The increments of a lane step (CC coarse columns of RC rows) come through a
+// shared-memory ring several steps ahead: one step ahead in registers left the
+// forward pass waiting on HBM (37% of its issue bound).  Cells beyond the
+// pair's rows and columns, and steps outside the run (`run` false), are filled
+// with 0; a path's rows are padded to a multiple of 4 with zeros, so a 16-byte
+// copy that starts inside a path stays inside its padding.
+template <int R, int O, int W>
+__device__ __forceinline__ void grad_fetch_incs(const GradParams &p, const GradPos &w, bool run, int64_t row_ld,
+                                                double *slot, int lane)
+{
+    using GS = GradShape<R, O, W>;
+    run = run && w.q < p.nsteps;
+    const int cj0 = (w.q * GS::C) >> O;
 #pragma unroll
-            for (int r = 0; r < R; ++r) left[r] = 1.0; // K(p, 0)
-            double bot = 1.0, corner = 1.0;            // lane l-1's last row at q-1 (as received), at q-2
-            double A[RC], B[RC], Ad[RC], Bd[RC];
-            __syncwarp();
-            for (int s = 0; s < S; ++s) {
-                const double from_above = __shfl_up_sync(0xffffffffu, bot, 1);
-                if (s % T == 0) {
+    for (int cc = 0; cc < GS::CC; ++cc) {
+        const bool in = run && cj0 + cc < (int)p.ncy;
+        const double *col = w.rows + (int64_t)(cj0 + cc) * row_ld;
+        if constexpr (GS::RC == 1) {
+            const bool ok = in && w.ci0 < (int)p.ncx;
+            grad_cp_async8z(slot + cc * 32 + lane, ok ? col : p.mat, ok ? 8 : 0);
+        } else {
 #pragma unroll
-                    for (int r = 0; r < R; ++r) ck[((int64_t)(s / T) * R + r) * 32] = left[r];
-                }
-                const int q = s - lane + 1;
-                double top = 1.0;
-                if (q >= 1 && q <= m) {
-                    double diag;
-                    if (lane == 0) {
-                        top = b == 0 ? 1.0 : bnd[q];
-                        diag = b == 0 ? 1.0 : bnd[q - 1];
-                    } else {
-                        top = from_above;
-                        diag = q == 1 ? 1.0 : corner;
-                    }
-                    if (((q - 1) & ((1 << O) - 1)) == 0) // a new coarse column
-                        grad_coefs<RC>(base, row_ld, ci0, p.ncx, (q - 1) >> O, A, B, Ad, Bd);
-                    grad_lane_step<R, O, false>(left, top, diag, A, B, Ad, Bd, nullptr);
-                    if (lane == 31 && b + 1 < nb) bnd[q] = left[R - 1];
-                    corner = from_above;
-                    bot = left[R - 1];
-                }
-                tops[(int64_t)s * 32] = top;
+            for (int h = 0; h < GS::RC / 2; ++h) {
+                const bool ok = in && w.ci0 + 2 * h < (int)p.ncx;
+                grad_cp_async16z(slot + 2 * ((cc * (GS::RC / 2) + h) * 32 + lane), ok ? col + 2 * h : p.mat, ok ? 16 : 0);
             }
-            __syncwarp();
-            if (lane == 31 && b + 1 < nb) bnd[0] = 1.0;
-            __syncwarp();
         }
     }
 }
 
-template <int R, int O>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) grad_bwd_kernel(GradParams p)
+template <int R, int O, int W>
+__device__ __forceinline__ void grad_read_incs(const double *slot, int lane,
+                                               double (&c)[GradShape<R, O, W>::CC][GradShape<R, O, W>::RC])
 {
-    static_assert(R >= (1 << O), "a lane's rows hold whole coarse rows");
-    constexpr int RC = R >> O;
-    constexpr int T = grad_seg<R>();
-    __shared__ double dsm[kWarpsPerBlock][T][R][32]; // D of the current segment, per lane
-    const int lane = threadIdx.x & 31;
-    const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int n = (int)(p.ncx << p.order), m = (int)(p.ncy << p.order);
-    const int nb = (n + 32 * R - 1) / (32 * R);
-    const int S = m + 31, NS = (S + T - 1) / T;
-    const int64_t band_doubles = grad_band_doubles(m, R);
-    double *dl = &dsm[threadIdx.x >> 5][0][0][lane];
-    for (int64_t it = gwarp; it < p.nitems; it += nwarps) {
-        int64_t xi, yj, row_ld;
-        double *base;
-        grad_item(p, it, xi, yj, base, row_ld);
-        const int64_t widx = p.op == kOpPairwise ? xi : xi * p.ny + yj;
-        const double w = p.in64 ? reinterpret_cast<const double *>(p.w)[widx]
-                                : (double)reinterpret_cast<const float *>(p.w)[widx];
-        double *bP = p.bnd + it * 2 * (int64_t)(m + 2); // P and Q of the row below the band, columns 0..m+1
-        double *bQ = bP + (m + 2);
-        for (int b = nb - 1; b >= 0; --b) {
-            const double *tops = p.dbuf + (it * nb + b) * band_doubles + lane;
-            const double *ck = tops + (int64_t)S * 32;
-            const int p0 = b * 32 * R + lane * R + 1;
-            const int ci0 = (p0 - 1) >> O;
-            double Pr[R], Qr[R]; // P, Q of the lane's rows at column q + 1
-            // the seed Lambda(n, m) = w enters as the right neighbour of row n at column m
-            const int rseed = n - p0;
+    using GS = GradShape<R, O, W>;
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                Pr[r] = r == rseed ? w : 0.0;
-                Qr[r] = 0.0;
+    for (int cc = 0; cc < GS::CC; ++cc) {
+        if constexpr (GS::RC == 1) {
+            c[cc][0] = slot[cc * 32 + lane];
+        } else {
+#pragma unroll
+            for (int h = 0; h < GS::RC / 2; ++h) {
+                const double2 v = *reinterpret_cast<const double2 *>(slot + 2 * ((cc * (GS::RC / 2) + h) * 32 + lane));
+                c[cc][2 * h] = v.x;
+                c[cc][2 * h + 1] = v.y;
             }
-            double g[RC];
+        }
+    }
+}
+
+// grad_fwd_kernel is bound by its record: (R + C + 1) / (R C) doubles a cell,
+// written once, against 3 float64 operations (128 x 128 pairs, L = 128, order 2:
+// 9.1 GB in 2.26 ms; the kernel before it, one column a step, took 3.48 ms).
+template <int R, int O, int W>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, (GradShape<R, O, W>::CTAS)) grad_fwd_kernel(GradParams p)
+{
+    using GS = GradShape<R, O, W>;
+    constexpr int C = GS::C, RC = GS::RC, CC = GS::CC;
+    extern __shared__ __align__(16) unsigned char grad_smem[]; // the warps' boundary rows, if they fit
+    __shared__ __align__(16) double incs[kWarpsPerBlock][kGradFwdRing][GS::INC];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
+    const int64_t first = gwarp * p.per_warp;
+    if (first >= p.nitems) return; // warp-uniform
+    const int cnt = (int)(p.nitems - first < p.per_warp ? p.nitems - first : p.per_warp);
+    const int nsteps = p.nsteps, period = p.period;
+    const int64_t row_ld = p.op == kOpPairwise ? p.rows_x : p.ld;
+    const int run = cnt * p.nb * period, steps = run + 31;
+    double *rec = p.rec + gwarp * grad_warp_steps(p.per_warp, p.nb, period) * GS::REC;
+    // K of the row above the next band, columns 1..nsteps * C
+    double *bnd = p.bnd_smem ? reinterpret_cast<double *>(grad_smem) + wib * nsteps * C : p.bnd + gwarp * p.bnd_stride;
+    double(*ring)[GS::INC] = incs[wib];
+
+    GradPos w = grad_pos<R, O>(p, first, 0, 0, lane), f = w; // f: the step whose increments are fetched
+    auto fetch = [&](int s) { // of warp step s; called for s = 0, 1, ...
+        if (s >= lane) {
+            grad_fetch_incs<R, O, W>(p, f, s - lane < run, row_ld, ring[s & (kGradFwdRing - 1)], lane);
+            if (++f.q == period) {
+                f.q = 0;
+                grad_next_band<R, O>(p, f, lane);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    fetch(1);
+    fetch(2);
+    double tn[C]; // lane 0: the row above its next step
+    double left[R], bot[C], corner = 1.0;
 #pragma unroll
-            for (int rc = 0; rc < RC; ++rc) g[rc] = 0.0;
-            double topP = 0.0, topQ = 0.0; // this lane's row 0 P, Q at its last column (published)
-            double belowQ_prev = 0.0;      // lane l+1's row 0 Q at column q + 1
-            double A[RC], B[RC], Ad[RC], Bd[RC];
-            __syncwarp();
-            for (int k = NS - 1; k >= 0; --k) {
-                const int s0 = k * T;
-                // phase A: recompute this segment's steps lane by lane from the checkpoint and the
-                // stored top inputs, keeping D in shared memory
-                {
-                    double left[R], tp[T + 1];
+    for (int r = 0; r < R; ++r) left[r] = 1.0;
 #pragma unroll
-                    for (int r = 0; r < R; ++r) left[r] = ck[((int64_t)k * R + r) * 32];
+    for (int c = 0; c < C; ++c) {
+        bot[c] = 1.0;
+        tn[c] = 1.0;
+    }
+    for (int s = 0; s < steps; ++s) {
+        fetch(s + 3);
+        asm volatile("cp.async.wait_group 3;" ::: "memory"); // step s has arrived
+        double top[C];
 #pragma unroll
-                    for (int t = 0; t <= T; ++t) {
-                        const int st = s0 - 1 + t;
-                        tp[t] = (st >= 0 && st < S) ? tops[(int64_t)st * 32] : 1.0;
+        for (int c = 0; c < C; ++c) top[c] = __shfl_up_sync(kFullMask, bot[c], 1);
+        if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) top[c] = tn[c];
+        }
+        if ((unsigned)(s - lane) < (unsigned)run) {
+            if (w.q < nsteps) {
+                double A[CC][RC], B[CC][RC];
+                grad_read_incs<R, O, W>(ring[s & (kGradFwdRing - 1)], lane, A);
+#pragma unroll
+                for (int cc = 0; cc < CC; ++cc)
+#pragma unroll
+                    for (int rc = 0; rc < RC; ++rc) stencil_coefs(A[cc][rc], A[cc][rc], B[cc][rc]);
+                double *rs = rec + (int64_t)s * GS::REC;
+                double2 *rs2 = reinterpret_cast<double2 *>(rs) + lane;
+#pragma unroll
+                for (int c = 0; c < C / 2; ++c) __stcs(rs2 + c * 32, make_double2(top[2 * c], top[2 * c + 1]));
+#pragma unroll
+                for (int r = 0; r < R / 2; ++r) __stcs(rs2 + (C / 2 + r) * 32, make_double2(left[2 * r], left[2 * r + 1]));
+                __stcs(rs + GS::NV2 * 64 + lane, corner);
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const int cc = GS::cc_of(c);
+                    double up = top[c], dg = c == 0 ? corner : top[c - 1];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const double l = left[r], a = A[cc][r >> O];
+                        up = fma(up, a, fma(l, a, -(dg * B[cc][r >> O])));
+                        dg = l;
+                        left[r] = up;
                     }
-                    bool have = false;
+                    bot[c] = up;
+                }
+                corner = top[C - 1];
+                if (lane == 31 && w.b + 1 < p.nb) {
 #pragma unroll
-                    for (int t = 0; t < T; ++t) {
-                        const int q = s0 + t - lane + 1;
-                        if (q >= 1 && q <= m) {
-                            if (!have || ((q - 1) & ((1 << O) - 1)) == 0)
-                                grad_coefs<RC>(base, row_ld, ci0, p.ncx, (q - 1) >> O, A, B, Ad, Bd);
-                            have = true;
-                            grad_lane_step<R, O, true>(left, tp[t + 1], q == 1 ? 1.0 : tp[t], A, B, Ad, Bd,
-                                                       dl + t * R * 32);
+                    for (int c = 0; c < C; ++c) bnd[w.q * C + c] = bot[c];
+                }
+            }
+            if (++w.q == period) { // the next band starts
+                w.q = 0;
+                grad_next_band<R, O>(p, w, lane);
+#pragma unroll
+                for (int r = 0; r < R; ++r) left[r] = 1.0;
+                corner = 1.0;
+            }
+            if (lane == 0 && w.q < nsteps) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) tn[c] = w.b > 0 ? bnd[w.q * C + c] : 1.0;
+            }
+        }
+        __syncwarp(); // orders lane 31's boundary stores before lane 0's loads
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// grad_bwd_kernel: per cell 5 float64 operations for D (K of the block and
+// dK/dc in one pass), 3 for Lambda and 1 for the sum.  The record and the
+// increments come through shared-memory rings of cp.async copies, two steps
+// ahead.  Lambda of a cell is
+//   A(right) Lambda(right) + A(below) Lambda(below) - B(diagonal) Lambda(diagonal),
+// three operations with the coefficients of the three cells' coarse cells:
+// those of the column to the right are kept from the previous step (AR, BR),
+// those of the row below come from lane l + 1 with its Lambda.  An SM
+// sub-partition issues a float64 instruction in two slots and any other in one,
+// so the bound is 18 slots a cell plus the step's rest; 128 x 128 pairs,
+// L = 128, order 2: 4.20 ms, 2.05 of them float64 (one column a step: 9.48 ms).
+template <int R, int O, int W>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, (GradShape<R, O, W>::CTAS)) grad_bwd_kernel(GradParams p)
+{
+    using GS = GradShape<R, O, W>;
+    constexpr int C = GS::C, RC = GS::RC, CC = GS::CC, NV2 = GS::NV2;
+    extern __shared__ __align__(16) unsigned char grad_smem[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
+    const int64_t first = gwarp * p.per_warp;
+    if (first >= p.nitems) return; // warp-uniform
+    const int cnt = (int)(p.nitems - first < p.per_warp ? p.nitems - first : p.per_warp);
+    const int ncx = (int)p.ncx, ncy = (int)p.ncy, nsteps = p.nsteps, period = p.period;
+    const int n = ncx << O;
+    const int64_t row_ld = p.op == kOpPairwise ? p.rows_x : p.ld;
+    const int run = cnt * p.nb * period, steps = run + 31;
+    const double *rec = p.rec + gwarp * grad_warp_steps(p.per_warp, p.nb, period) * GS::REC;
+    double *ring = reinterpret_cast<double *>(grad_smem) + wib * kGradRing * (GS::REC + GS::INC);
+    // the first row of the band below: Lambda of its columns, then A and B of its coarse columns
+    double *bL = p.bnd + gwarp * p.bnd_stride, *bA = bL + nsteps * C, *bB = bA + nsteps * CC;
+
+    GradPos w = grad_pos<R, O>(p, first + cnt - 1, p.nb - 1, period - 1, lane), f = w;
+    int64_t wi = (p.op == kOpPairwise ? p.x0 : p.x0 * p.ny) + first + cnt - 1; // the pair's weight
+    auto fetch = [&](int s, int slot) { // of warp step s; called for s = steps - 1, steps - 2, ...
+        double *dst = ring + slot * (GS::REC + GS::INC);
+        if (s >= 0) {
+            const double *src = rec + (int64_t)s * GS::REC;
+#pragma unroll
+            for (int i = 0; i < NV2; ++i) grad_cp_async16(dst + 2 * (i * 32 + lane), src + 2 * (i * 32 + lane));
+            grad_cp_async8z(dst + NV2 * 64 + lane, src + NV2 * 64 + lane, 8);
+        }
+        if (s - lane < run) {
+            grad_fetch_incs<R, O, W>(p, f, s >= lane, row_ld, dst + GS::REC, lane);
+            if (--f.q < 0) {
+                f.q = period - 1;
+                grad_prev_band<R, O>(p, f, lane);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(steps - 1, 0);
+    fetch(steps - 2, 1);
+    int slot = 0;
+
+    double Lr[R];                        // Lambda of the lane's rows at the column right of the block
+    double AR[RC], BR[RC], bBR;          // A, B of that column (bBR: B of the row below)
+    double g[CC][RC];
+    double topL[C], tA[CC], tB[CC];     // Lambda and coefficients of the lane's first row, for lane l - 1
+    double below0;                       // Lambda below-right of the block
+    auto start_band = [&]() { // nothing lies to the right of the band's last column
+        const int rseed = w.b == p.nb - 1 ? n - 1 - (w.b * 32 + lane) * R : -1;
+        double wt = 0.0;
+        if (rseed >= 0 && rseed < R) // Lambda(n, m) = the pair's weight, as row n's right neighbour
+            wt = p.in64 ? reinterpret_cast<const double *>(p.w)[wi] : (double)reinterpret_cast<const float *>(p.w)[wi];
+#pragma unroll
+        for (int r = 0; r < R; ++r) Lr[r] = r == rseed ? wt : 0.0;
+#pragma unroll
+        for (int rc = 0; rc < RC; ++rc) {
+            AR[rc] = 1.0;
+            BR[rc] = 0.0;
+        }
+        bBR = 0.0;
+        below0 = 0.0;
+    };
+    start_band();
+#pragma unroll
+    for (int c = 0; c < C; ++c) topL[c] = 0.0;
+#pragma unroll
+    for (int cc = 0; cc < CC; ++cc) {
+        tA[cc] = 1.0;
+        tB[cc] = 1.0;
+#pragma unroll
+        for (int rc = 0; rc < RC; ++rc) g[cc][rc] = 0.0;
+    }
+
+    for (int s = steps - 1; s >= 0; --s) {
+        fetch(s - 2, slot == 0 ? kGradRing - 1 : slot - 1); // the slot of step s + 1
+        asm volatile("cp.async.wait_group 2;" ::: "memory"); // step s has arrived
+        double bl[C], bAc[CC], bBc[CC]; // the row below: Lambda and coefficients
+#pragma unroll
+        for (int c = 0; c < C; ++c) bl[c] = __shfl_down_sync(kFullMask, topL[c], 1);
+#pragma unroll
+        for (int cc = 0; cc < CC; ++cc) {
+            bAc[cc] = __shfl_down_sync(kFullMask, tA[cc], 1);
+            bBc[cc] = __shfl_down_sync(kFullMask, tB[cc], 1);
+        }
+        if ((unsigned)(s - lane) < (unsigned)run) {
+            if (w.q < nsteps) {
+                if (lane == 31) {
+                    const bool has = w.b + 1 < p.nb;
+#pragma unroll
+                    for (int c = 0; c < C; ++c) bl[c] = has ? bL[w.q * C + c] : 0.0;
+#pragma unroll
+                    for (int cc = 0; cc < CC; ++cc) {
+                        bAc[cc] = has ? bA[w.q * CC + cc] : 1.0;
+                        bBc[cc] = has ? bB[w.q * CC + cc] : 1.0;
+                    }
+                }
+                const double *rs = ring + slot * (GS::REC + GS::INC);
+                double A[CC][RC], B[CC][RC], Ad[CC][RC], Bd[CC][RC];
+                grad_read_incs<R, O, W>(rs + GS::REC, lane, A);
+#pragma unroll
+                for (int cc = 0; cc < CC; ++cc)
+#pragma unroll
+                    for (int rc = 0; rc < RC; ++rc) {
+                        const double c = A[cc][rc];
+                        stencil_coefs(c, A[cc][rc], B[cc][rc]);
+                        Ad[cc][rc] = fma(c, 1.0 / 6.0, 0.5);
+                        Bd[cc][rc] = c * (1.0 / 6.0); // -B'
+                    }
+                double D[R][C];
+                { // D of the block from the record
+                    double left[R], top[C];
+                    const double2 *rs2 = reinterpret_cast<const double2 *>(rs) + lane;
+#pragma unroll
+                    for (int c = 0; c < C / 2; ++c) {
+                        const double2 v = rs2[c * 32];
+                        top[2 * c] = v.x;
+                        top[2 * c + 1] = v.y;
+                    }
+#pragma unroll
+                    for (int r = 0; r < R / 2; ++r) {
+                        const double2 v = rs2[(C / 2 + r) * 32];
+                        left[2 * r] = v.x;
+                        left[2 * r + 1] = v.y;
+                    }
+                    const double corner = rs[NV2 * 64 + lane];
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        const int cc = GS::cc_of(c);
+                        double up = top[c], dg = c == 0 ? corner : top[c > 0 ? c - 1 : 0];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            const int rc = r >> O;
+                            const double l = left[r], sum = l + up;
+                            D[r][c] = fma(sum, Ad[cc][rc], dg * Bd[cc][rc]);
+                            up = fma(sum, A[cc][rc], -(dg * B[cc][rc]));
+                            dg = l;
+                            left[r] = up;
                         }
                     }
                 }
-                // phase B: the adjoint over the same steps in reverse
-                bool have = false;
-#pragma unroll 1
-                for (int t = T - 1; t >= 0; --t) {
-                    const int s = s0 + t;
-                    if (s >= S) continue; // uniform: the last segment may be short
-                    const double belowP = __shfl_down_sync(0xffffffffu, topP, 1);
-                    const double belowQ = __shfl_down_sync(0xffffffffu, topQ, 1);
-                    const int q = s - lane + 1;
-                    if (q >= 1 && q <= m) {
-                        double dP, dQ; // P(p+1, q) and Q(p+1, q+1) for the lane's last row
-                        if (lane == 31) {
-                            const bool last = b + 1 >= nb;
-                            dP = last ? 0.0 : bP[q];
-                            dQ = last ? 0.0 : bQ[q + 1];
-                        } else {
-                            dP = belowP;
-                            dQ = q == m ? 0.0 : belowQ_prev;
-                        }
-                        const int cj = (q - 1) >> O;
-                        if (!have || q == m || (q & ((1 << O) - 1)) == 0)
-                            grad_coefs<RC>(base, row_ld, ci0, p.ncx, cj, A, B, Ad, Bd);
-                        have = true;
-                        const double *dq = dl + t * R * 32;
 #pragma unroll
-                        for (int r = R - 1; r >= 0; --r) {
-                            const int rc = r >> O;
-                            const double lam = Pr[r] + dP - dQ;
-                            g[rc] = fma(lam, dq[r * 32], g[rc]);
-                            const double P = A[rc] * lam, Q = B[rc] * lam;
-                            dQ = Qr[r]; // Q(p, q+1) is the diagonal of the row above
-                            dP = P;
-                            Pr[r] = P;
-                            Qr[r] = Q;
-                        }
-                        topP = Pr[0];
-                        topQ = Qr[0];
-                        if (lane == 0 && b > 0) {
-                            bP[q] = Pr[0];
-                            bQ[q] = Qr[0];
-                        }
-                        if (((q - 1) & ((1 << O) - 1)) == 0) { // leaving the coarse column: dk/dc is complete
+                for (int c = C - 1; c >= 0; --c) {
+                    const bool edge_r = c == C - 1;
+                    const int cc = GS::cc_of(c), cr = edge_r ? 0 : GS::cc_of(c + 1);
+                    double dn = bl[c], dgl = edge_r ? below0 : bl[edge_r ? 0 : c + 1];
 #pragma unroll
-                            for (int rc = 0; rc < RC; ++rc) {
-                                const int ci = ci0 + rc;
-                                if (ci < p.ncx) base[(int64_t)cj * row_ld + ci] = g[rc];
-                                g[rc] = 0.0;
+                    for (int r = R - 1; r >= 0; --r) {
+                        const bool edge_d = r == R - 1;
+                        const int rc = r >> O, rb = edge_d ? 0 : (r + 1) >> O; // rb: coarse row below
+                        const double ad = edge_d ? bAc[cc] : A[cc][rb];
+                        const double ar = edge_r ? AR[rc] : A[cr][rc];
+                        const double bg = edge_r ? (edge_d ? bBR : BR[rb]) : (edge_d ? bBc[cr] : B[cr][rb]);
+                        const double lr = Lr[r];
+                        const double lam = fma(ad, dn, fma(ar, lr, -(bg * dgl)));
+                        // the coarse cell's first fine cell in this order starts its sum
+                        const bool starts = GS::WHOLE && (edge_d || rc != rb) && (edge_r || cc != cr);
+                        g[cc][rc] = starts ? lam * D[r][c] : fma(lam, D[r][c], g[cc][rc]);
+                        dgl = lr;
+                        dn = lam;
+                        Lr[r] = lam;
+                    }
+                    topL[c] = dn;
+                }
+                below0 = bl[0];
+                bBR = bBc[0];
+#pragma unroll
+                for (int rc = 0; rc < RC; ++rc) {
+                    AR[rc] = A[0][rc];
+                    BR[rc] = B[0][rc];
+                }
+#pragma unroll
+                for (int cc = 0; cc < CC; ++cc) {
+                    tA[cc] = A[cc][0];
+                    tB[cc] = B[cc][0];
+                }
+                if (lane == 0 && w.b > 0) {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) bL[w.q * C + c] = topL[c];
+#pragma unroll
+                    for (int cc = 0; cc < CC; ++cc) {
+                        bA[w.q * CC + cc] = tA[cc];
+                        bB[w.q * CC + cc] = tB[cc];
+                    }
+                }
+                if (GS::WHOLE || ((w.q * C) & ((1 << O) - 1)) == 0) { // dk/dc of the coarse columns is complete
+                    const int cj0 = (w.q * C) >> O;
+#pragma unroll
+                    for (int cc = 0; cc < CC; ++cc) {
+                        double *col = w.rows + (int64_t)(cj0 + cc) * row_ld;
+                        if (CC == 1 || cj0 + cc < ncy) {
+                            if constexpr (RC == 1) {
+                                if (w.ci0 < ncx) col[0] = g[cc][0];
+                            } else {
+#pragma unroll
+                                for (int h = 0; h < RC / 2; ++h) {
+                                    if (w.ci0 + 2 * h + 1 < ncx)
+                                        *reinterpret_cast<double2 *>(col + 2 * h) = make_double2(g[cc][2 * h], g[cc][2 * h + 1]);
+                                    else if (w.ci0 + 2 * h < ncx)
+                                        col[2 * h] = g[cc][2 * h];
+                                }
                             }
                         }
+                        if constexpr (!GS::WHOLE) {
+#pragma unroll
+                            for (int rc = 0; rc < RC; ++rc) g[cc][rc] = 0.0;
+                        }
                     }
-                    belowQ_prev = belowQ;
                 }
             }
-            __syncwarp();
-            if (lane == 0 && b > 0) {
-                bP[m + 1] = 0.0;
-                bQ[m + 1] = 0.0;
+            if (--w.q < 0) {
+                w.q = period - 1;
+                if (w.b == 0) --wi;
+                grad_prev_band<R, O>(p, w, lane);
+                if (s > lane) start_band();
             }
-            __syncwarp();
         }
+        slot = slot == kGradRing - 1 ? 0 : slot + 1;
+        __syncwarp(); // orders lane 0's boundary stores before lane 31's loads
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Increments of pairwise pairs (x path = y path = x0 + item) in per-pair
@@ -383,28 +645,44 @@ struct GradContractParams {
     int64_t ld, rows_x, ncx, ncy;
     int64_t nrows_m;       // Gram: ld; pairwise: nitems * rows_x
     int64_t ncols_n;       // Gram: ny * ncy; pairwise: ncy (per pair)
-    const double *dxt;     // x differences, rows m of the chunk: [m][k]
+    const double *dxt;     // pairwise: x differences, rows m of the chunk: [m][k]
+    const double *dxk;     // Gram: the same, dimension-major: [k][m] (leading dimension ld)
     const double *dyt;     // y differences, all y cells: [y path * ncy + cj][k]
     int64_t d;
-    double *part;          // gx: [slice][nrows_m][d] partial sums
-    int64_t slice;         // columns per slice
+    double *part;          // gx: [slice][nrows_m][d], gy of a Gram: [range of m][ncols_n][d] partial sums
+    int64_t slice;         // gx: columns per slice
+    int64_t mslice;        // gy of a Gram: m per range (a multiple of kGyTile)
     double *gdy;           // gy: (ny, ncy, d) accumulated (+=) over chunks
     int64_t x0;
 };
 
-// Row layout of scaled differences: dst[(path * rows + r) * d + k] =
-// src[(path * d + k) * nc + r] for r < nc, 0 for nc <= r < rows.
+// Scaled differences src[(path * d + k) * nc + r] with `rows` rows a path
+// (0 for nc <= r < rows): row layout dst[(path * rows + r) * d + k], or
+// dimension-major over all paths, dst[k * (npaths * rows) + path * rows + r].
 template <int V = 0> // instantiated once, in kernels_grad.cu
-__global__ void grad_rows_kernel(const double *src, int64_t npaths, int64_t nc, int64_t rows, int64_t d, double *dst)
+__global__ void grad_rows_kernel(const double *src, int64_t npaths, int64_t nc, int64_t rows, int64_t d, int dim_major,
+                                 double *dst)
 {
     const int64_t total = npaths * rows * d;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t path = e / (rows * d), rem = e - path * rows * d, r = rem / d, k = rem - r * d;
+        int64_t path, r, k;
+        if (dim_major) {
+            k = e / (npaths * rows);
+            const int64_t rem = e - k * npaths * rows;
+            path = rem / rows;
+            r = rem - path * rows;
+        } else {
+            path = e / (rows * d);
+            const int64_t rem = e - path * rows * d;
+            r = rem / d;
+            k = rem - r * d;
+        }
         dst[e] = r < nc ? src[(path * d + k) * nc + r] : 0.0;
     }
 }
 
+// pairwise
 template <int V = 0> // instantiated once, in kernels_grad.cu
 __global__ void grad_gx_kernel(GradContractParams p)
 {
@@ -412,19 +690,9 @@ __global__ void grad_gx_kernel(GradContractParams p)
     if (mm >= p.nrows_m) return;
     const int64_t n0 = (int64_t)blockIdx.y * p.slice;
     const int64_t n1 = n0 + p.slice < p.ncols_n ? n0 + p.slice : p.ncols_n;
-    const double *col;     // G[n][mm] = col[n * stride]
-    int64_t stride;
-    const double *dyt;     // dyt[n * d + k] for the n of this row
-    if (p.op == kOpPairwise) {
-        const int64_t item = mm / p.rows_x, ci = mm - item * p.rows_x;
-        col = p.mat + item * p.ncy * p.rows_x + ci;
-        stride = p.rows_x;
-        dyt = p.dyt + (p.x0 + item) * p.ncy * p.d; // the pair's own y path
-    } else {
-        col = p.mat + mm;
-        stride = p.ld;
-        dyt = p.dyt;
-    }
+    const int64_t item = mm / p.rows_x, ci = mm - item * p.rows_x;
+    const double *col = p.mat + item * p.ncy * p.rows_x + ci;  // G[n][mm] = col[n * rows_x]
+    const double *dyt = p.dyt + (p.x0 + item) * p.ncy * p.d;   // the pair's own y path, [n][k]
     double *out = p.part + ((int64_t)blockIdx.y * p.nrows_m + mm) * p.d;
     for (int64_t k0 = 0; k0 < p.d; k0 += 8) {
         double acc[8];
@@ -432,7 +700,7 @@ __global__ void grad_gx_kernel(GradContractParams p)
         for (int k = 0; k < 8; ++k) acc[k] = 0.0;
         const double *yk = dyt + k0;
         for (int64_t n = n0; n < n1; ++n) {
-            const double gv = col[n * stride];
+            const double gv = col[n * p.rows_x];
             const double *yn = yk + n * p.d;
 #pragma unroll
             for (int k = 0; k < 8; ++k)
@@ -444,35 +712,85 @@ __global__ void grad_gx_kernel(GradContractParams p)
     }
 }
 
-// gy: one warp per y cell n (Gram: n = y path * ncy + cj over all y paths;
-// pairwise: n = pair * ncy + cj), lanes over the x cells paired with it.
+// Gram: a tall, skinny product that should cost one read of G.  A thread owns
+// two neighbouring rows m (16-byte loads) and 8 dimensions; the y rows of a
+// tile sit in shared memory, read by the whole warp at one address.  The loads
+// of 8 columns are issued together: with one in flight the kernel waited 28
+// issue slots per instruction on them.
+constexpr int kGxThreads = 128;
+constexpr int kGxTile = 64; // y cells staged at a time
+
+template <int V = 0> // instantiated once, in kernels_grad.cu
+__global__ void __launch_bounds__(kGxThreads) grad_gx_gram_kernel(GradContractParams p)
+{
+    __shared__ double2 ys[kGxTile][4];
+    const int64_t mm = 2 * ((int64_t)blockIdx.x * kGxThreads + threadIdx.x);
+    const bool own = mm < p.nrows_m;
+    const int64_t n0 = (int64_t)blockIdx.y * p.slice;
+    const int64_t n1 = n0 + p.slice < p.ncols_n ? n0 + p.slice : p.ncols_n;
+    const double *col = p.mat + (own ? mm : 0);
+    double *out = p.part + ((int64_t)blockIdx.y * p.nrows_m + mm) * p.d;
+    for (int64_t k0 = 0; k0 < p.d; k0 += 8) {
+        const int kn = (int)(p.d - k0 < 8 ? p.d - k0 : 8);
+        double2 acc[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] = make_double2(0.0, 0.0);
+        for (int64_t nt = n0; nt < n1; nt += kGxTile) {
+            __syncthreads();
+            for (int e = threadIdx.x; e < kGxTile * 8; e += kGxThreads) {
+                const int j = e >> 3, k = e & 7;
+                reinterpret_cast<double *>(ys)[e] = nt + j < n1 && k < kn ? p.dyt[(nt + j) * p.d + k0 + k] : 0.0;
+            }
+            __syncthreads();
+            const int cnt = (int)(n1 - nt < kGxTile ? n1 - nt : kGxTile);
+            const double *g = col + nt * p.ld;
+            for (int j0 = 0; j0 < cnt; j0 += 8) {
+                double2 gv[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { // columns beyond the slice: 0
+                    gv[j] = make_double2(0.0, 0.0);
+                    if (j0 + j < cnt) gv[j] = *reinterpret_cast<const double2 *>(g + (j0 + j) * p.ld);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const double2 y = ys[j0 + j][k];
+                        acc[2 * k].x = fma(gv[j].x, y.x, acc[2 * k].x);
+                        acc[2 * k].y = fma(gv[j].y, y.x, acc[2 * k].y);
+                        acc[2 * k + 1].x = fma(gv[j].x, y.y, acc[2 * k + 1].x);
+                        acc[2 * k + 1].y = fma(gv[j].y, y.y, acc[2 * k + 1].y);
+                    }
+                }
+            }
+        }
+        if (own) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k < kn) {
+                    out[k0 + k] = acc[k].x;
+                    out[p.d + k0 + k] = acc[k].y;
+                }
+        }
+    }
+}
+
+// pairwise gy: one warp per y cell n = pair * ncy + cj, lanes over the pair's x cells.
 template <int V = 0> // instantiated once, in kernels_grad.cu
 __global__ void grad_gy_kernel(GradContractParams p)
 {
     const int lane = threadIdx.x & 31;
     const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nrows = p.op == kOpPairwise ? (p.nrows_m / p.rows_x) * p.ncy : p.ncols_n;
-    if (n >= nrows) return;
-    const double *row;
-    const double *xt;
-    int64_t mlen, yrow;
-    if (p.op == kOpPairwise) {
-        const int64_t item = n / p.ncy, cj = n - item * p.ncy;
-        row = p.mat + item * p.ncy * p.rows_x + cj * p.rows_x;
-        mlen = p.rows_x;
-        xt = p.dxt + item * p.rows_x * p.d;
-        yrow = (p.x0 + item) * p.ncy + cj;
-    } else {
-        row = p.mat + n * p.ld;
-        mlen = p.ld;
-        xt = p.dxt;
-        yrow = n;
-    }
+    if (n >= (p.nrows_m / p.rows_x) * p.ncy) return;
+    const int64_t item = n / p.ncy, cj = n - item * p.ncy;
+    const double *row = p.mat + item * p.ncy * p.rows_x + cj * p.rows_x;
+    const double *xt = p.dxt + item * p.rows_x * p.d;
+    const int64_t yrow = (p.x0 + item) * p.ncy + cj;
     for (int64_t k0 = 0; k0 < p.d; k0 += 8) {
         double acc[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) acc[k] = 0.0;
-        for (int64_t mm = lane; mm < mlen; mm += 32) {
+        for (int64_t mm = lane; mm < p.rows_x; mm += 32) {
             const double gv = row[mm]; // padding rows hold 0, as do their differences
             const double *xm = xt + mm * p.d + k0;
 #pragma unroll
@@ -483,62 +801,103 @@ __global__ void grad_gy_kernel(GradContractParams p)
         for (int k = 0; k < 8; ++k) {
             double v = acc[k];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFullMask, v, off);
             if (lane == 0 && k0 + k < p.d) p.gdy[yrow * p.d + k0 + k] += v;
         }
     }
 }
 
-// gy for the Gram: gdy[n][k] += sum_m G[n][m] dxt[m][k], a tall-skinny GEMM
-// (rows n: all y cells, m: the chunk's x cells, k < d).  A CTA owns 32 rows
-// and k-chunks of up to 32; m goes in tiles of 64 staged in shared memory
-// (G rows coalesced along m; dxt transposed to [k][m] with a padded stride so
-// that the 8 k-groups of a warp hit different banks).  Each (n, k) has one
-// owner thread, so the sum over chunks stays in order.
-constexpr int kGyRows = 32, kGyTile = 64, kGyK = 32;
+// gy for the Gram: partial sums over a range of m of G[n][m] dx[m][k], n over all
+// y cells, m over the chunk's x cells, k < d, again one read of G.  A warp owns
+// kGyRows rows and 8 dimensions; its lanes take two neighbouring m each (16-byte
+// loads, the next ones in flight), the differences of a tile of m come from
+// shared memory (dimension-major [k][m], two tiles), and the lanes' sums meet in
+// a fixed shuffle tree.  grad_gy_reduce_kernel adds the ranges of m in order.
+// (One fma per shared-memory load, or the differences read from the L2 by each
+// warp, cost 2.39 and 1.76 ms for the 2.1 GB of a 128 x 128 gradient.)
+constexpr int kGyRows = 8;
+constexpr int kGyWarps = 4;
+constexpr int kGyTile = 128; // m per tile
 
 template <int V = 0> // instantiated once, in kernels_grad.cu
-__global__ void __launch_bounds__(256) grad_gy_gram_kernel(GradContractParams p)
+__global__ void __launch_bounds__(kGyWarps * 32, 2) grad_gy_gram_kernel(GradContractParams p)
 {
-    __shared__ double gs[kGyRows][kGyTile + 1];
-    __shared__ double xs[kGyK][kGyTile + 1];
-    const int tid = threadIdx.x;
-    const int row = tid >> 3, kg = tid & 7; // 32 rows x 8 k-groups; k = kg + 8 j
-    const int64_t n0 = (int64_t)blockIdx.x * kGyRows;
-    const int64_t nrows = p.ncols_n;
-    for (int64_t k0 = 0; k0 < p.d; k0 += kGyK) {
-        const int kn = (int)((p.d - k0) < kGyK ? (p.d - k0) : kGyK);
-        double acc[kGyK / 8];
+    __shared__ __align__(16) double xs[2][8][kGyTile];
+    const int lane = threadIdx.x & 31;
+    const int64_t n0 = ((int64_t)blockIdx.x * kGyWarps + (threadIdx.x >> 5)) * kGyRows;
+    const int64_t mb = (int64_t)blockIdx.y * p.mslice;
+    const int64_t me = mb + p.mslice < p.ld ? mb + p.mslice : p.ld; // both multiples of 4
+    const double *row[kGyRows];
 #pragma unroll
-        for (int j = 0; j < kGyK / 8; ++j) acc[j] = 0.0;
-        for (int64_t m0 = 0; m0 < p.ld; m0 += kGyTile) {
-            __syncthreads();
-            for (int e = tid; e < kGyRows * kGyTile; e += 256) {
-                const int r = e / kGyTile, mm = e - r * kGyTile;
-                const int64_t n = n0 + r, m = m0 + mm;
-                gs[r][mm] = (n < nrows && m < p.ld) ? p.mat[n * p.ld + m] : 0.0;
-            }
-            for (int e = tid; e < kGyTile * kn; e += 256) {
-                const int mm = e / kn, k = e - mm * kn;
-                const int64_t m = m0 + mm;
-                xs[k][mm] = m < p.ld ? p.dxt[m * p.d + k0 + k] : 0.0;
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int mm = 0; mm < kGyTile; ++mm) {
-                const double gv = gs[row][mm];
+    for (int r = 0; r < kGyRows; ++r) // rows beyond the last repeat it (not written)
+        row[r] = p.mat + (n0 + r < p.ncols_n ? n0 + r : p.ncols_n - 1) * p.ld;
+    auto load_g = [&](int64_t m, double2 (&v)[kGyRows]) {
 #pragma unroll
-                for (int j = 0; j < kGyK / 8; ++j)
-                    if (kg + 8 * j < kn) acc[j] = fma(gv, xs[kg + 8 * j][mm], acc[j]);
+        for (int r = 0; r < kGyRows; ++r) {
+            v[r] = make_double2(0.0, 0.0);
+            if (m < me) v[r] = *reinterpret_cast<const double2 *>(row[r] + m);
+        }
+    };
+    for (int64_t k0 = 0; k0 < p.d; k0 += 8) {
+        const int kn = (int)(p.d - k0 < 8 ? p.d - k0 : 8);
+        auto stage = [&](int64_t m0, int buf) {
+            for (int e = threadIdx.x; e < 8 * kGyTile / 2; e += kGyWarps * 32) {
+                const int k = e / (kGyTile / 2), i = 2 * (e - k * (kGyTile / 2));
+                const bool in = k < kn && m0 + i < me;
+                grad_cp_async16z(&xs[buf][k][i], in ? p.dxk + (k0 + k) * p.ld + m0 + i : p.dxk, in ? 16 : 0);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        double acc[kGyRows][8];
+#pragma unroll
+        for (int r = 0; r < kGyRows; ++r)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[r][k] = 0.0;
+        double2 gn[kGyRows];
+        load_g(mb + 2 * lane, gn);
+        __syncthreads(); // the previous dimensions are done with the tiles
+        stage(mb, 0);
+        int buf = 0;
+        for (int64_t m0 = mb; m0 < me; m0 += kGyTile, buf ^= 1) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads(); // this tile is visible; the other is free
+            if (m0 + kGyTile < me) stage(m0 + kGyTile, buf ^ 1);
+#pragma unroll
+            for (int h = 0; h < kGyTile / 64; ++h) {
+                double2 g[kGyRows];
+#pragma unroll
+                for (int r = 0; r < kGyRows; ++r) g[r] = gn[r];
+                load_g(m0 + 64 * (h + 1) + 2 * lane, gn);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const double2 x = *reinterpret_cast<const double2 *>(&xs[buf][k][64 * h + 2 * lane]);
+#pragma unroll
+                    for (int r = 0; r < kGyRows; ++r) acc[r][k] = fma(g[r].y, x.y, fma(g[r].x, x.x, acc[r][k]));
+                }
             }
         }
-        const int64_t n = n0 + row;
-        if (n < nrows) {
 #pragma unroll
-            for (int j = 0; j < kGyK / 8; ++j)
-                if (kg + 8 * j < kn) p.gdy[n * p.d + k0 + kg + 8 * j] += acc[j];
-        }
+        for (int r = 0; r < kGyRows; ++r)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                double v = acc[r][k];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFullMask, v, off);
+                if (lane == 0 && k < kn && n0 + r < p.ncols_n)
+                    p.part[((int64_t)blockIdx.y * p.ncols_n + n0 + r) * p.d + k0 + k] = v;
+            }
     }
+}
+
+// gdy[e] += sum over the ranges of m of part[range][e], in order.
+template <int V = 0> // instantiated once, in kernels_grad.cu
+__global__ void grad_gy_reduce_kernel(const double *part, int64_t nranges, int64_t total, double *gdy)
+{
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    double s = 0.0;
+    for (int64_t i = 0; i < nranges; ++i) s += part[i * total + e];
+    gdy[e] += s;
 }
 
 // gdx[(x0 + il) * ncx + ci][k] = sum over slices of part (rows ci < ncx).

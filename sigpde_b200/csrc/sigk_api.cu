@@ -986,52 +986,104 @@ int run_pairs_static(const TcPlan &t, int op, int kind, double param, const void
 
 // ------------------------------------------------------------------ backward pass
 // Gradients of sum w * k with respect to the points (grad.cuh).  Pairs are
-// processed in chunks of x paths so that the per-cell derivatives D (one
-// float64 per fine cell of every pair in the chunk) and the chunk's increment
-// matrix stay under kGradChunkBytes (SIGK_GRAD_CHUNK_MB overrides).
+// processed in equal chunks of x paths so that the records of the forward pass
+// and the chunk's increment matrix stay under kGradChunkBytes
+// (SIGK_GRAD_CHUNK_MB overrides).
 // Workspace: zero word | x, y differences | dk/d(x diff), dk/d(y diff) |
-// partial sums of the x contraction | increment matrix | D | boundary rows.
+// partial sums of the x contraction | increment matrix | records | boundary rows.
 constexpr size_t kGradChunkBytes = 8ull << 30;
 constexpr int kGradMaxOrder = 4;
 constexpr int64_t kGradSlices = 64;
+constexpr size_t kGradFwdBndBytes = 16 * 1024;    // a CTA's boundary rows stay in shared memory up to this
 
 struct GradPlan {
     bool ok = false;
-    int R = 0, O = 0, nb = 0;
-    int64_t rows_x = 0, chunk = 0, nchunks = 0, slice = 0, nslices = 0;
-    size_t dx_off = 0, dy_off = 0, gdx_off = 0, gdy_off = 0, part_off = 0, mat_off = 0, d_off = 0, bnd_off = 0,
+    int R = 0, O = 0, nb = 0, nsteps = 0, period = 0;
+    bool wide = false;
+    int64_t rows_x = 0, chunk = 0, nchunks = 0, per_warp = 0, slice = 0, nslices = 0, mslice = 0, bnd_stride = 0;
+    size_t dx_off = 0, dy_off = 0, gdx_off = 0, gdy_off = 0, part_off = 0, mat_off = 0, rec_off = 0, bnd_off = 0,
            xt_off = 0, yt_off = 0, ws_bytes = 0;
 };
 
-GradPlan make_grad_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order)
+// Pairs a warp of the backward wavefronts: a run as long as the resident warps make it.
+int64_t grad_per_warp(int64_t items, int ctas)
 {
-    GradPlan g;
-    if (order > kGradMaxOrder) return g;
+    const int64_t warps = (int64_t)sm_count() * ctas * kWarpsPerBlock;
+    return (items + warps - 1) / warps;
+}
+
+// Rows per lane, lane steps and chunks of a backward pass over nx * items_per_x pairs.
+bool grad_shape(GradPlan &g, int64_t nx, int64_t items_per_x, int64_t ncx, int64_t ncy, int order)
+{
+    if (order > kGradMaxOrder) return false;
     const int64_t n = ncx << order, m = ncy << order;
-    // rows per lane: the smallest power of two with 32R >= n, at most 8 (bands of 256 rows keep the
-    // adjoint's registers near 128), and at least 2^order (a lane holds whole coarse rows)
-    int R = 1;
-    while (R < 8 && 32 * R < n) R *= 2;
+    // rows per lane: the smallest power of two with 32R >= n, from 2 to 8 (the adjoint's block of 8 x 4
+    // cells stays within 168 registers), and at least 2^order (a lane holds whole coarse rows)
+    int R = 2;
+    while (R < (order < 2 ? 4 : 8) && 32 * R < n) R *= 2;
     while (R < (1 << order)) R *= 2;
+    g.nb = (int)((n + 32 * R - 1) / (32 * R));
+    GradFns kf = get_grad_kernels(R, order, true);
+    const GradFns narrow = get_grad_kernels(R, order, false);
+    if (kf.fwd) {
+        // warp steps of the whole call (its longest warp); a wide step costs about 1.15 narrow ones (128 x 128
+        // pairs, L = 128, order 2: 1823 steps in 6.46 ms against 2602 in 7.78; 40 x 40 pairs, L = 60 / 75, order 2:
+        // 105 steps in 341 us against 105 in 320; 30 x 30, L = 100, order 2: 131 in 444 against 229 in 457)
+        auto steps = [&](const GradFns &f) {
+            const int64_t q = (m + f.cols - 1) / f.cols;
+            const int64_t period = g.nb > 1 && q < kGradMinPeriod ? kGradMinPeriod : q;
+            return grad_warp_steps(grad_per_warp(nx * items_per_x, f.ctas), g.nb, (int)period);
+        };
+        g.wide = !narrow.fwd || 23 * steps(kf) < 20 * steps(narrow);
+    }
+    if (!g.wide) kf = narrow;
+    if (!kf.fwd) return false;
+    const int64_t nsteps = (m + kf.cols - 1) / kf.cols;
     g.R = R;
     g.O = order;
-    g.nb = (int)((n + 32 * R - 1) / (32 * R));
+    g.nsteps = (int)nsteps;
+    g.period = g.nb > 1 && g.nsteps < kGradMinPeriod ? kGradMinPeriod : g.nsteps;
     g.rows_x = (ncx + 3) / 4 * 4;
-    const size_t dbytes = (size_t)g.nb * grad_band_doubles((int)m, R) * sizeof(double);
-    const size_t bbytes = 2 * (size_t)(m + 2) * sizeof(double);
-    const size_t mbytes = (size_t)ncy * g.rows_x * sizeof(double);
-    const int64_t items_per_x = op == kOpPairwise ? 1 : ny;
-    const size_t per_x = (size_t)items_per_x * (dbytes + bbytes + mbytes);
+    g.bnd_stride = g.nb > 1 ? nsteps * (kf.cols + 2 * kf.ccols) : 0;
+    // chunk: records and increments of a pair, both within the cap; chunks of equal size
+    const size_t step_bytes = (size_t)kf.rec * sizeof(double);
+    const size_t per_item = (size_t)g.nb * g.period * step_bytes + (size_t)ncy * g.rows_x * sizeof(double);
     size_t cap = kGradChunkBytes;
     if (const char *v = getenv("SIGK_GRAD_CHUNK_MB")) {
         const long long mb = atoll(v);
         if (mb > 0) cap = (size_t)mb << 20;
     }
-    int64_t chunk = (int64_t)(cap / per_x);
+    int64_t chunk = (int64_t)(cap / (per_item * (size_t)items_per_x));
     if (chunk < 1) chunk = 1;
     if (chunk > nx) chunk = nx;
-    g.chunk = chunk;
     g.nchunks = (nx + chunk - 1) / chunk;
+    g.chunk = (nx + g.nchunks - 1) / g.nchunks;
+    g.nchunks = (nx + g.chunk - 1) / g.chunk;
+    return true;
+}
+
+// Increment matrix, records and boundary rows of a chunk from offset `off` on; returns the end.
+size_t grad_wave_layout(GradPlan &g, int64_t items, int64_t ncy, size_t off)
+{
+    const GradFns kf = get_grad_kernels(g.R, g.O, g.wide);
+    // every chunk runs with the full chunk's pairs a warp, so a smaller last one fits the same records
+    const int64_t pw = grad_per_warp(items, kf.ctas), warps = (items + pw - 1) / pw;
+    g.per_warp = pw;
+    g.mat_off = off;
+    off += align256((size_t)items * (size_t)ncy * g.rows_x * sizeof(double));
+    g.rec_off = off;
+    off += align256((size_t)warps * (size_t)grad_warp_steps(pw, g.nb, g.period) * (size_t)kf.rec * sizeof(double));
+    g.bnd_off = off;
+    off += align256((size_t)warps * (size_t)g.bnd_stride * sizeof(double));
+    return off;
+}
+
+GradPlan make_grad_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order)
+{
+    GradPlan g;
+    const int64_t items_per_x = op == kOpPairwise ? 1 : ny;
+    if (!grad_shape(g, nx, items_per_x, ncx, ncy, order)) return g;
+    const int64_t chunk = g.chunk;
     const int64_t ncols = op == kOpPairwise ? ncy : ny * ncy;
     g.slice = (ncols + kGradSlices - 1) / kGradSlices;
     if (g.slice < 32) g.slice = ncols < 32 ? ncols : 32;
@@ -1046,21 +1098,55 @@ GradPlan make_grad_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy
     off += align256((size_t)nx * ncx * d * sizeof(double));
     g.gdy_off = off;
     off += align256((size_t)ny_paths * ncy * d * sizeof(double));
-    g.part_off = off;
-    off += align256((size_t)g.nslices * chunk * g.rows_x * d * sizeof(double));
-    g.xt_off = off; // the chunk's x differences in row layout
+    // y contraction of a Gram: ranges of m, enough of them for several waves of CTAs, at least 4 tiles each
+    const int64_t ld = chunk * g.rows_x, row_ctas = (ncols + kGyRows * kGyWarps - 1) / (kGyRows * kGyWarps);
+    int64_t ranges = (int64_t)sm_count() * 2 * 6 / row_ctas;
+    const int64_t most = ld / (4 * kGyTile);
+    if (ranges > most) ranges = most;
+    if (ranges < 1) ranges = 1;
+    g.mslice = ((ld + ranges - 1) / ranges + kGyTile - 1) / kGyTile * kGyTile;
+    ranges = (ld + g.mslice - 1) / g.mslice;
+    g.part_off = off; // partial sums of the x contraction, then of a Gram's y contraction
+    size_t part = (size_t)g.nslices * ld * d;
+    if (op != kOpPairwise && part < (size_t)ranges * ncols * d) part = (size_t)ranges * ncols * d;
+    off += align256(part * sizeof(double));
+    g.xt_off = off; // the chunk's x differences: row layout (pairwise) or dimension-major (Gram)
     off += align256((size_t)chunk * g.rows_x * d * sizeof(double));
     g.yt_off = off; // all y differences in row layout
     off += align256((size_t)ny_paths * ncy * d * sizeof(double));
-    g.mat_off = off;
-    off += align256((size_t)chunk * items_per_x * mbytes);
-    g.d_off = off;
-    off += align256((size_t)chunk * items_per_x * dbytes);
-    g.bnd_off = off;
-    off += align256((size_t)chunk * items_per_x * bbytes);
-    g.ws_bytes = off;
+    g.ws_bytes = grad_wave_layout(g, chunk * items_per_x, ncy, off);
     g.ok = true;
     return g;
+}
+
+// The recording forward pass and the adjoint over one chunk (gp: pairs and matrix set by the caller).
+int launch_grad_wavefronts(const GradPlan &g, GradParams gp, unsigned char *wsb, cudaStream_t stream)
+{
+    const GradFns kf = get_grad_kernels(g.R, g.O, g.wide);
+    if (!kf.fwd || !kf.bwd) return fail(SIGK_EUNSUPPORTED, "no backward kernels for R=%d order=%d", g.R, g.O);
+    gp.rows_x = g.rows_x;
+    gp.order = g.O;
+    gp.per_warp = g.per_warp;
+    gp.nb = g.nb;
+    gp.nsteps = g.nsteps;
+    gp.period = g.period;
+    gp.rec = reinterpret_cast<double *>(wsb + g.rec_off);
+    gp.bnd = reinterpret_cast<double *>(wsb + g.bnd_off);
+    gp.bnd_stride = g.bnd_stride;
+    const int64_t warps = (gp.nitems + gp.per_warp - 1) / gp.per_warp;
+    const unsigned blocks = (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    int nb = 0, st = blocks_per_sm((const void *)kf.bwd, kf.bwd_smem, &nb); // opts the kernel in to its shared memory
+    if (st) return st;
+    const size_t rows = g.nb > 1 ? (size_t)kWarpsPerBlock * g.nsteps * kf.cols * sizeof(double) : 0;
+    gp.bnd_smem = rows <= kGradFwdBndBytes;
+    kf.fwd<<<blocks, kWarpsPerBlock * 32, gp.bnd_smem ? rows : 0, stream>>>(gp);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "backward forward-pass launch");
+    kf.bwd<<<blocks, kWarpsPerBlock * 32, kf.bwd_smem, stream>>>(gp);
+    count_launch();
+    e = cudaGetLastError();
+    return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "adjoint launch");
 }
 
 int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_t nx, int64_t ny, int64_t lx,
@@ -1095,22 +1181,17 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
     if ((st = run_delta(y, ny_paths, ly, 1.0, sy, dy))) return st;
     double *dxt = reinterpret_cast<double *>(wsb + g.xt_off);
     double *dyt = reinterpret_cast<double *>(wsb + g.yt_off);
-    auto run_rows = [&](const double *src, int64_t npaths, int64_t nc, int64_t rows, double *dst) -> int {
+    auto run_rows = [&](const double *src, int64_t npaths, int64_t nc, int64_t rows, bool dim_major, double *dst) -> int {
         const int64_t total = npaths * rows * d;
         int64_t blocks = (total + 255) / 256;
         if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-        get_grad_aux_kernels().rows<<<(unsigned)blocks, 256, 0, stream>>>(src, npaths, nc, rows, d, dst);
+        get_grad_aux_kernels().rows<<<(unsigned)blocks, 256, 0, stream>>>(src, npaths, nc, rows, d, dim_major, dst);
         count_launch();
         cudaError_t e2 = cudaGetLastError();
         return e2 == cudaSuccess ? SIGK_OK : cuda_fail(e2, "row-layout launch");
     };
-    if ((st = run_rows(dy, ny_paths, ncy, ncy, dyt))) return st;
-    GradFns kf = get_grad_kernels(g.R, g.O);
+    if ((st = run_rows(dy, ny_paths, ncy, ncy, false, dyt))) return st;
     GradAuxFns aux = get_grad_aux_kernels();
-    if (!kf.fwd || !kf.bwd) return fail(SIGK_EUNSUPPORTED, "no backward kernels for R=%d order=%d", g.R, g.O);
-    int nbf = 0, nbb = 0;
-    if ((st = blocks_per_sm((const void *)kf.fwd, 0, &nbf)) || (st = blocks_per_sm((const void *)kf.bwd, 0, &nbb)))
-        return st;
     auto launched = [&](const char *what) -> int {
         count_launch();
         cudaError_t e2 = cudaGetLastError();
@@ -1143,31 +1224,19 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
             gp.ld = ld;
             if ((st = launch_dgemm_inc(gp, stream))) return st;
         }
-        if ((st = run_rows(dx + i0 * d * ncx, nxc, ncx, g.rows_x, dxt))) return st;
+        if ((st = run_rows(dx + i0 * d * ncx, nxc, ncx, g.rows_x, op != kOpPairwise, dxt))) return st;
         GradParams gp{};
         gp.op = op;
         gp.mat = mat;
         gp.ld = ld;
-        gp.rows_x = g.rows_x;
         gp.ncx = ncx;
         gp.ncy = ncy;
-        gp.order = order;
         gp.nitems = items;
         gp.ny = ny;
         gp.w = w;
         gp.in64 = in64;
         gp.x0 = i0;
-        gp.dbuf = reinterpret_cast<double *>(wsb + g.d_off);
-        gp.bnd = reinterpret_cast<double *>(wsb + g.bnd_off);
-        auto grid_for = [&](int nb) -> unsigned {
-            int64_t warps = (int64_t)sm_count() * nb * kWarpsPerBlock;
-            if (warps > items) warps = items;
-            return (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
-        };
-        kf.fwd<<<grid_for(nbf), kWarpsPerBlock * 32, 0, stream>>>(gp);
-        if ((st = launched("backward forward-pass launch"))) return st;
-        kf.bwd<<<grid_for(nbb), kWarpsPerBlock * 32, 0, stream>>>(gp);
-        if ((st = launched("adjoint launch"))) return st;
+        if ((st = launch_grad_wavefronts(g, gp, wsb, stream))) return st;
         // contractions: x side (partial slices, then their ordered sum) and y side
         GradContractParams cp{};
         cp.op = op;
@@ -1179,6 +1248,7 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
         cp.nrows_m = op == kOpPairwise ? items * g.rows_x : ld;
         cp.ncols_n = op == kOpPairwise ? ncy : ny * ncy;
         cp.dxt = dxt;
+        cp.dxk = dxt;
         cp.dyt = dyt;
         cp.d = d;
         cp.part = part;
@@ -1186,8 +1256,13 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
         cp.gdy = gdy;
         cp.x0 = i0;
         const int64_t nsl = (cp.ncols_n + g.slice - 1) / g.slice;
+        cp.mslice = g.mslice;
         if (gx) {
-            aux.gx<<<dim3((unsigned)((cp.nrows_m + 127) / 128), (unsigned)nsl), 128, 0, stream>>>(cp);
+            if (op == kOpPairwise)
+                aux.gx<<<dim3((unsigned)((cp.nrows_m + 127) / 128), (unsigned)nsl), 128, 0, stream>>>(cp);
+            else
+                aux.gx_gram<<<dim3((unsigned)((cp.nrows_m + 2 * kGxThreads - 1) / (2 * kGxThreads)), (unsigned)nsl),
+                              kGxThreads, 0, stream>>>(cp);
             if ((st = launched("x contraction launch"))) return st;
             const int64_t tot = cp.nrows_m * d;
             aux.reduce<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(part, nsl, cp.nrows_m, g.rows_x, ncx, d, i0,
@@ -1199,7 +1274,12 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
                 const int64_t rows = items * ncy;
                 aux.gy<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, stream>>>(cp);
             } else {
-                aux.gy_gram<<<(unsigned)((ny * ncy + kGyRows - 1) / kGyRows), 256, 0, stream>>>(cp);
+                const int64_t per_cta = kGyRows * kGyWarps, ranges = (cp.ld + g.mslice - 1) / g.mslice;
+                aux.gy_gram<<<dim3((unsigned)((ny * ncy + per_cta - 1) / per_cta), (unsigned)ranges), kGyWarps * 32, 0,
+                              stream>>>(cp);
+                if ((st = launched("y contraction launch"))) return st;
+                const int64_t tot = ny * ncy * d;
+                aux.gy_reduce<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(part, ranges, tot, gdy);
             }
             if ((st = launched("y contraction launch"))) return st;
         }
@@ -1222,21 +1302,10 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
 // layout, weight of pair b = grad_out[b]), then dk/dc * scales back out.
 GradPlan make_grad_inc_plan(int64_t npairs, int64_t ncx, int64_t ncy, int order)
 {
-    GradPlan g = make_grad_plan(kOpPairwise, npairs, npairs, ncx, ncy, 1, order);
-    if (!g.ok) return g;
-    // only the matrix, the per-step records and the boundary rows are used
-    const int64_t m = ncy << order;
-    const size_t dbytes = (size_t)g.nb * grad_band_doubles((int)m, g.R) * sizeof(double);
-    const size_t bbytes = 2 * (size_t)(m + 2) * sizeof(double);
-    const size_t mbytes = (size_t)ncy * g.rows_x * sizeof(double);
-    size_t off = 256;
-    g.mat_off = off;
-    off += align256((size_t)g.chunk * mbytes);
-    g.d_off = off;
-    off += align256((size_t)g.chunk * dbytes);
-    g.bnd_off = off;
-    off += align256((size_t)g.chunk * bbytes);
-    g.ws_bytes = off;
+    GradPlan g;
+    if (!grad_shape(g, npairs, 1, ncx, ncy, order)) return g;
+    g.ws_bytes = grad_wave_layout(g, g.chunk, ncy, 256);
+    g.ok = true;
     return g;
 }
 
@@ -1247,12 +1316,8 @@ int run_backward_inc(const GradPlan &g, const void *inc, int64_t npairs, int64_t
     const bool in64 = dtype == SIGK_F64;
     unsigned char *wsb = reinterpret_cast<unsigned char *>(ws);
     double *mat = reinterpret_cast<double *>(wsb + g.mat_off);
-    GradFns kf = get_grad_kernels(g.R, g.O);
     GradAuxFns aux = get_grad_aux_kernels();
-    if (!kf.fwd || !kf.bwd) return fail(SIGK_EUNSUPPORTED, "no backward kernels for R=%d order=%d", g.R, g.O);
-    int st, nbf = 0, nbb = 0;
-    if ((st = blocks_per_sm((const void *)kf.fwd, 0, &nbf)) || (st = blocks_per_sm((const void *)kf.bwd, 0, &nbb)))
-        return st;
+    int st;
     auto launched = [&](const char *what) -> int {
         count_launch();
         cudaError_t e2 = cudaGetLastError();
@@ -1270,26 +1335,14 @@ int run_backward_inc(const GradPlan &g, const void *inc, int64_t npairs, int64_t
         gp.op = kOpPairwise;
         gp.mat = mat;
         gp.ld = g.rows_x;
-        gp.rows_x = g.rows_x;
         gp.ncx = ncx;
         gp.ncy = ncy;
-        gp.order = order;
         gp.nitems = items;
         gp.ny = npairs;
         gp.w = w;
         gp.in64 = in64;
         gp.x0 = b0;
-        gp.dbuf = reinterpret_cast<double *>(wsb + g.d_off);
-        gp.bnd = reinterpret_cast<double *>(wsb + g.bnd_off);
-        auto grid_for = [&](int nb) -> unsigned {
-            int64_t warps = (int64_t)sm_count() * nb * kWarpsPerBlock;
-            if (warps > items) warps = items;
-            return (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
-        };
-        kf.fwd<<<grid_for(nbf), kWarpsPerBlock * 32, 0, stream>>>(gp);
-        if ((st = launched("backward forward-pass launch"))) return st;
-        kf.bwd<<<grid_for(nbb), kWarpsPerBlock * 32, 0, stream>>>(gp);
-        if ((st = launched("adjoint launch"))) return st;
+        if ((st = launch_grad_wavefronts(g, gp, wsb, stream))) return st;
         aux.inc_blocks<<<(unsigned)blocks, 256, 0, stream>>>(nullptr, in64, g0, g1, g2, items, b0, ncx, ncy, g.rows_x,
                                                              sx, sy, mat, ginc, 1);
         if ((st = launched("increment gradient launch"))) return st;

@@ -127,6 +127,31 @@ def test_chunked_backward_matches(sig, oracle, monkeypatch):
         close(v, u, 1e-13, "chunked")
 
 
+@pytest.mark.parametrize("shape", [
+    # (n_x, n_y, L_x, L_y, d, order)
+    (3, 2, 300, 9, 3, 0),    # three bands, fewer lane steps a band than its period
+    (50, 40, 6, 5, 3, 0),    # several pairs a warp, a lane step beyond the last column
+    (2, 3, 70, 30, 17, 1),   # two bands, three groups of dimensions
+    (3, 2, 12, 90, 9, 1),    # wide lane steps, the last one partly beyond the columns
+    (2, 2, 70, 61, 5, 2),    # wide lane steps, two bands, fewer steps than the period
+    (50, 40, 6, 5, 3, 2),
+    (2, 3, 40, 50, 2, 3),
+    (2, 2, 20, 9, 1, 4),
+    (1, 1, 2, 2, 1, 1),
+])
+def test_gram_gradients_at_block_edges(sig, oracle, shape):
+    """Lane-step, band, tile and run edges of the backward wavefronts and contractions."""
+    nx, ny, lx, ly, d, o = shape
+    x = oracle.brownian(nx, lx, d, 70 + lx)
+    y = oracle.brownian(ny, ly, d, 80 + ly)
+    w = np.random.default_rng(11).standard_normal((nx, ny))
+    X, Y = cuda(x, grad=True), cuda(y, grad=True)
+    (sig.SigPDE(sig.kernels.LinearKernel(), o).gram(X, Y) * cuda(w)).sum().backward()
+    gx, gy = oracle.grad_gram(x, y, o, w)
+    close(host(X.grad), gx, TOL64, "grad x")
+    close(host(Y.grad), gy, TOL64, "grad y")
+
+
 def test_gradcheck_small(sig):
     """torch.autograd.gradcheck: the backward against finite differences of the forward."""
     rng = np.random.default_rng(8)
