@@ -44,10 +44,14 @@ using DeltaFn = void (*)(const void *, int64_t, int64_t, int64_t, int64_t, doubl
 // mode: kPairDelta (path differences), kPairGiven (caller's increments), kPairMat (increment matrix)
 PairFn get_pair_kernel_f64(bool in64, int mode, int R, int O);
 PairFn get_pair_kernel_f32(bool in64, int mode, int R, int O);
-// mode: kNormDelta, kNormGiven or kNormTile (sigk_kernels.cuh)
-NormFn get_norm_kernel(bool in64, int mode, int R, int O);
-// one CTA per path, its bands as a warp pipeline (norm_pipe.cuh)
-NormFn get_norm_pipe_kernel(bool in64, int mode, int R, int O);
+// robust normalisation (norm_wave.cuh): R in {2,4,8,16} rows a lane; fn null where not built
+struct NormKernel {
+    NormFn fn;
+    int cols, rc, ccols; // columns, coarse rows and coarse columns of a lane step
+    int max_warps, regs; // solving warps a CTA, registers a thread (upper estimate)
+};
+// smem_tile, smem_bnd: increments, bottom rows in shared memory (a tile there only with the rows)
+NormKernel get_norm_kernel(int R, int O, bool smem_tile, bool smem_bnd);
 // D: dimension padded to a power of two in {2,...,32}; returns null unless
 // the lane's register tile (coarse rows per lane) * D <= 32.
 StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D);

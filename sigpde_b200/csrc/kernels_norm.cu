@@ -1,43 +1,42 @@
-// Instantiations of normalize_kernel (float64 cells and bracket arithmetic).
+// Instantiations of norm_kernel (float64 cells and bracket arithmetic).
 #include "dispatch.h"
-#include "sigk_kernels.cuh"
+#include "norm_wave.cuh"
 
 namespace sigk {
 namespace {
-template <typename TIN, int R, int M>
-NormFn by_o(int O)
+template <int R, int O>
+NormKernel by_mem(bool smem_tile, bool smem_bnd)
+{
+    using NS = NormShape<R, O>;
+    const int regs = R == 16 ? 255 : 128;
+    return {smem_tile && smem_bnd ? norm_kernel<R, O, true, true>
+            : smem_bnd            ? norm_kernel<R, O, false, true>
+                                  : norm_kernel<R, O, false, false>,
+            NS::C, NS::RC, NS::CC,
+            NS::MAXW, regs};
+}
+template <int R>
+NormKernel by_o(int O, bool smem_tile, bool smem_bnd)
 {
     switch (O) {
-    case 0: return normalize_kernel<TIN, R, 0, M>;
-    case 1: return normalize_kernel<TIN, R, 1, M>;
-    case 2: return normalize_kernel<TIN, R, 2, M>;
-    case 3: return normalize_kernel<TIN, R, 3, M>;
-    default: return normalize_kernel<TIN, R, 4, M>;
-    }
-}
-template <typename TIN, int M>
-NormFn by_r(int R, int O)
-{
-    switch (R) {
-    case 2: return by_o<TIN, 2, M>(O);
-    case 4: return by_o<TIN, 4, M>(O);
-    case 8: return by_o<TIN, 8, M>(O);
-    default: return by_o<TIN, 16, M>(O);
-    }
-}
-template <typename TIN>
-NormFn by_mode(int mode, int R, int O)
-{
-    switch (mode) {
-    case kNormGiven: return by_r<TIN, kNormGiven>(R, O);
-    case kNormTile: return by_r<TIN, kNormTile>(R, O);
-    default: return by_r<TIN, kNormDelta>(R, O);
+    case 0:
+        if constexpr (R <= 4) return by_mem<R, 0>(smem_tile, smem_bnd); // 16 coarse cells a step would spill
+        return NormKernel{};
+    case 1: return by_mem<R, 1>(smem_tile, smem_bnd);
+    case 2: return by_mem<R, 2>(smem_tile, smem_bnd);
+    case 3: return by_mem<R, 3>(smem_tile, smem_bnd);
+    default: return by_mem<R, 4>(smem_tile, smem_bnd);
     }
 }
 } // namespace
 
-NormFn get_norm_kernel(bool in64, int mode, int R, int O)
+NormKernel get_norm_kernel(int R, int O, bool smem_tile, bool smem_bnd)
 {
-    return in64 ? by_mode<double>(mode, R, O) : by_mode<float>(mode, R, O);
+    switch (R) {
+    case 2: return by_o<2>(O, smem_tile, smem_bnd);
+    case 4: return by_o<4>(O, smem_tile, smem_bnd);
+    case 8: return by_o<8>(O, smem_tile, smem_bnd);
+    default: return by_o<16>(O, smem_tile, smem_bnd);
+    }
 }
 } // namespace sigk

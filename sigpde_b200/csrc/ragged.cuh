@@ -124,14 +124,9 @@ __device__ __forceinline__ int wait_progress(const int *prog, int need, long lon
 // One band of one pair.  top_buf / top_prog: the band above (null for band 0);
 // bot_buf / bot_prog: this band's bottom row and progress (bot_buf null for the
 // last band).  Returns K[n][m] in every lane if `last`, else 1.
-// prog_base: progress values of this solve are prog_base + (column blocks
-// done), so one set of counters serves consecutive solves (the pipelined
-// normalisation re-solves a path several times without resetting them);
-// pub_stride: column blocks between publications of the band's progress.
 template <typename T, int R, int O, class Src>
 __device__ T band_solve(const SolveGeom &g, Src &src, int band, bool last, const T *top_buf, const int *top_prog,
-                        T *bot_buf, int *bot_prog, int *error, int prog_base = 0, int pub_stride = kProgressStride,
-                        long long poll_limit = kProgressPollLimit)
+                        T *bot_buf, int *bot_prog, int *error, long long poll_limit)
 {
     using BS = BlockShape<R, O>;
     constexpr int C = BS::C;
@@ -164,8 +159,7 @@ __device__ T band_solve(const SolveGeom &g, Src &src, int band, bool last, const
                 for (int c = 0; c < C; ++c) top[c] = T(1);
             } else if (active) {
                 if (!poisoned && seen <= q) {
-                    const int v0 = wait_progress(top_prog, prog_base + (int)q + 1, poll_limit);
-                    const int v = (v0 < 0 || v0 == 0x7fffffff) ? v0 : v0 - prog_base;
+                    const int v = wait_progress(top_prog, (int)q + 1, poll_limit);
                     if (v < 0 || v == 0x7fffffff) { // ran out, or the band above was refused
                         poisoned = true;
                         if (v < 0) atomicOr(error, kErrWaitTimeout);
@@ -203,9 +197,9 @@ __device__ T band_solve(const SolveGeom &g, Src &src, int band, bool last, const
             if (writer) {
 #pragma unroll
                 for (int c = 0; c < C; ++c) bot_buf[q * C + 1 + c] = bot[c];
-                if ((q + 1) % pub_stride == 0 || q + 1 == g.nsteps) {
+                if ((q + 1) % kProgressStride == 0 || q + 1 == g.nsteps) {
                     __threadfence();
-                    st_release(bot_prog, prog_base + (int)q + 1);
+                    st_release(bot_prog, (int)q + 1);
                 }
             }
         }
@@ -245,8 +239,8 @@ __device__ T ragged_band(const BandSource &bs, int64_t ncx, int64_t ncy, int ord
         src.base = reinterpret_cast<const TM *>(bs.mat);
         src.ld = bs.ld;
         src.ncy = ncy;
-        return band_solve<T, R, O>(g, src, band, last, top_buf, top_prog, bot_buf, bot_prog, error, 0,
-                                   kProgressStride, poll_limit);
+        return band_solve<T, R, O>(g, src, band, last, top_buf, top_prog, bot_buf, bot_prog, error,
+                                   poll_limit);
     } else {
         DeltaIncs<T, BS::RC> src;
         src.dX = reinterpret_cast<const T *>(bs.dX);
@@ -254,8 +248,8 @@ __device__ T ragged_band(const BandSource &bs, int64_t ncx, int64_t ncy, int ord
         src.d = bs.d;
         src.ncy = ncy;
         src.dxs = ((int64_t)BS::RC * bs.d * 32 <= stage_cap) ? stage : nullptr;
-        return band_solve<T, R, O>(g, src, band, last, top_buf, top_prog, bot_buf, bot_prog, error, 0,
-                                   kProgressStride, poll_limit);
+        return band_solve<T, R, O>(g, src, band, last, top_buf, top_prog, bot_buf, bot_prog, error,
+                                   poll_limit);
     }
 }
 

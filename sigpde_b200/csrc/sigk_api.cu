@@ -22,7 +22,7 @@
 #include "ragged.cuh"
 #include "stream.cuh"
 #include "tc.cuh"
-#include "norm_pipe.cuh"
+#include "norm_wave.cuh"
 #include "dgemm_inc.cuh"
 #include "static_inc.cuh"
 #include "grad.cuh"
@@ -191,8 +191,11 @@ PairFn pick_pair(int precision, int dtype, int mode, int R, int O)
 struct OccKey {
     const void *fn;
     size_t smem;
-    int dev;
-    bool operator==(const OccKey &o) const { return fn == o.fn && smem == o.smem && dev == o.dev; }
+    int dev, threads;
+    bool operator==(const OccKey &o) const
+    {
+        return fn == o.fn && smem == o.smem && dev == o.dev && threads == o.threads;
+    }
 };
 struct OccHash {
     size_t operator()(const OccKey &k) const
@@ -203,12 +206,12 @@ struct OccHash {
 std::mutex g_occ_mu;
 std::unordered_map<OccKey, int, OccHash> g_occ;
 
-int blocks_per_sm(const void *fn, size_t smem, int *out)
+int blocks_per_sm(const void *fn, size_t smem, int *out, int threads = kWarpsPerBlock * 32)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
-    OccKey key{fn, smem, dev};
+    OccKey key{fn, smem, dev, threads};
     {
         std::lock_guard<std::mutex> lk(g_occ_mu);
         auto it = g_occ.find(key);
@@ -233,7 +236,7 @@ int blocks_per_sm(const void *fn, size_t smem, int *out)
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
     }
     int nb = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kWarpsPerBlock * 32, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     if (nb <= 0) return fail(SIGK_ELAUNCH, "kernel cannot be resident (smem=%zu bytes)", smem);
     if (nb > kMaxBlocksPerSM) nb = kMaxBlocksPerSM;
@@ -1503,90 +1506,84 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
     }
 }
 
-// Normalisation plan: the increment source (a shared-memory tile of the
-// path's coarse increments when it fits, else precomputed differences, or the
-// caller's increments), the variant, shared memory and workspace layout
-// (boundary rows for multi-band paths, then the float64 differences).
-constexpr size_t kNormTileBytesPerWarp = 48 * 1024;
-
+// Normalisation plan: rows per lane, solving warps, where the path's increment
+// tile and the bands' bottom rows live, and the workspace (float64 differences |
+// tiles | rows).
 struct NormPlan {
-    int mode, R, O, nbands;
-    int64_t tile_pitch, bnd_stride;
-    size_t smem_per_warp, bnd_bytes, dx_off, ws_bytes;
-    // pipelined kernel (one CTA per path, `nw` bands as warps): its shared memory per CTA and the
-    // workspace offsets of the progress counters, the wait flag and the band rows
-    bool pipe;
-    int nw;
-    size_t smem_cta, prog_off, err_off;
+    NormKernel k;
+    int R, O, nbands, nw, nsteps, pitch, col0, threads;
+    int64_t tile; // values
+    bool smem_tile, smem_bnd;
+    int64_t grid;
+    size_t smem, dx_off, tile_off, bnd_off, ws_bytes;
 };
 
-constexpr size_t kNormPipeSmemBytes = 160 * 1024;
+constexpr size_t kNormSmemBytes = 226 * 1024;      // of the 227 KB a CTA may have (its static word)
+constexpr size_t kNormTileCap = size_t(1) << 30;   // of all resident CTAs' tiles in the workspace
 
 NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
 {
-    NormPlan q{};
-    const int64_t tile_pitch = nc | 1; // odd pitch: neighbouring lanes' rows fall in different banks
-    const size_t tile = (size_t)nc * (size_t)tile_pitch * sizeof(double);
-    if (from_inc)
-        q.mode = kNormGiven;
-    else if (tile <= kNormTileBytesPerWarp && !env_flag("SIGK_NO_NORM_TILE"))
-        q.mode = kNormTile;
-    else
-        q.mode = kNormDelta;
-    // only the difference mode stages rows of dx (and may shrink R to fit them)
-    Plan pl = make_plan(SIGK_OP_NORMALIZE, n, n, nc, nc, d, order, 8, q.mode != kNormDelta);
-    q.R = pl.R;
-    q.O = pl.O;
-    q.nbands = pl.nbands;
-    q.bnd_stride = pl.bnd_stride;
-    q.bnd_bytes = align256(pl.ws_bytes);
-    q.tile_pitch = tile_pitch;
-    q.smem_per_warp = q.mode == kNormTile ? tile : q.mode == kNormDelta ? pl.stage_bytes_per_warp : 0;
-    q.dx_off = q.bnd_bytes;
-    q.ws_bytes = from_inc ? q.bnd_bytes : q.dx_off + align256((size_t)n * (size_t)d * (size_t)nc * sizeof(double));
-
-    // Pipelined variant (one CTA per path, R = 2 rows per lane grown until the bands fit one CTA).
-    // Measured on B200 it wins only where it can hold the path's increment tile in shared memory
-    // for the whole CTA while the one-warp-per-path kernel cannot (tile above 48 KB) and the
-    // increments are expensive to re-form (d >= 16): N=32 L=128 d=32 o=1, 1.64 ms vs 6.58 ms.
-    // Elsewhere its band hand-offs cost more than they save (N=512 L=64 d=16 o=1: 0.74 vs 0.29 ms;
-    // N=8 L=256 d=8 o=2: 8.5 vs 5.3 ms), so it is used for that case only (SIGK_NORM_PIPE=1 forces
-    // it when possible, SIGK_NO_NORM_PIPE=1 disables it).
+    const int sms = sm_count();
     const int64_t nref = nc << order;
-    int R = 2;
-    while (R < 16 && (nref + 32 * R - 1) / (32 * R) > kNormPipeMaxWarps) R <<= 1;
-    const int64_t nw = (nref + 32 * R - 1) / (32 * R);
-    const bool wins = !from_inc && d >= 16 && tile > kNormTileBytesPerWarp && tile <= kNormPipeSmemBytes;
-    if (nw >= 2 && nw <= kNormPipeMaxWarps && (wins || env_flag("SIGK_NORM_PIPE")) && !env_flag("SIGK_NO_NORM_PIPE")) {
-        const int rc = rows_per_coarse_lane(R, order);
-        int mode = q.mode;
-        size_t smem = 0;
-        if (mode == kNormTile || mode == kNormDelta) {
-            // one shared tile per CTA when it fits, else per-warp staged differences (or none)
-            mode = (tile <= kNormPipeSmemBytes && !env_flag("SIGK_NO_NORM_TILE")) ? kNormTile : kNormDelta;
-            if (mode == kNormTile) {
-                smem = tile;
-            } else {
-                const size_t st = (size_t)rc * (size_t)d * 32 * sizeof(double) * (size_t)nw;
-                smem = st <= kNormPipeSmemBytes ? st : 0;
+    NormPlan best{};
+    double best_cost = -1.0;
+    for (int smem_tile = 1; smem_tile >= 0; --smem_tile) {
+        if (smem_tile && env_flag("SIGK_NO_NORM_TILE")) continue;
+        for (int R = 2; R <= 16; R *= 2) {
+            NormPlan q{};
+            q.O = order >= 4 ? 4 : order;
+            q.R = R;
+            q.k = get_norm_kernel(R, q.O, smem_tile, true);
+            if (!q.k.fn) continue;
+            q.nbands = (int)((nref + 32 * R - 1) / (32 * R));
+            q.nw = q.nbands < q.k.max_warps ? q.nbands : q.k.max_warps;
+            q.nsteps = (int)((nref + q.k.cols - 1) / q.k.cols);
+            // a step beyond the last coarse column (order 0) is put before the first one, where K = 1
+            q.col0 = q.nsteps * q.k.cols > nref ? 1 : 0;
+            // a column holds its rows, a multiple of RC, and RC zeros for the lanes beyond them; lanes read (column
+            // q - l, row RC l) with 8- or 16-byte loads: the pitch that puts them in different banks
+            const int rc = q.k.rc, low = ((int)nc + rc - 1) / rc * rc + rc;
+            q.pitch = rc == 1 ? (low + 1) / 2 * 2 : rc == 2 ? (low + 3) / 4 * 4 : (low + 1) / 4 * 4 + 2;
+            q.tile = (nc + q.col0) * q.pitch;
+            const size_t tile = (size_t)q.tile * sizeof(double);
+            q.threads = 32 * (q.nw > 4 ? q.nw : 4);
+            const size_t rows = (size_t)(1 + (q.nbands > 1 ? q.nw * q.nsteps : 0)) * q.k.cols * sizeof(double);
+            q.smem_tile = smem_tile;
+            if (smem_tile && tile + rows > kNormSmemBytes) continue;
+            q.smem_bnd = rows <= kNormSmemBytes;
+            if (!q.smem_bnd) q.k = get_norm_kernel(R, q.O, false, false);
+            q.smem = (smem_tile ? tile : 0) + (q.smem_bnd ? rows : 0);
+            // paths an SM works on together, and the time of all of its paths: the steps of a solve, each at the issue
+            // slots of a warp's step (two for each of 3 float64 operations a cell and 5 a coarse cell) times the warps
+            // that share a sub-partition, or a lone warp's slots and latencies (a tile in the L2 costs its loads too).
+            // Rows a lane, us: 24 paths, L = 220, d = 8, order 1: 617 / 565 / 680 with 2 / 4 / 8; 512, L = 64, d = 16,
+            // order 1: 210 / 163 / 205; 512, L = 256, d = 8, order 2: 5984 / 3702 / 2654 (16: 4312)
+            int64_t res = (int64_t)((228 * 1024) / (q.smem + 1024));
+            const int64_t by_regs = 65536 / ((int64_t)q.threads * q.k.regs);
+            if (res > by_regs) res = by_regs;
+            if (res > 2048 / q.threads) res = 2048 / q.threads;
+            if (res < 1) res = 1;
+            const int64_t paths = (n + sms - 1) / sms;
+            const int64_t together = paths < res ? paths : res;
+            const double steps = (double)((q.nbands + q.nw - 1) / q.nw) * (q.nsteps + 31 + (q.nw - 1) * kNormLag);
+            const double slots = 1.15 * (6.0 * R * q.k.cols + (smem_tile ? 10.0 : 22.0) * q.k.rc * q.k.ccols + 50.0);
+            const double shared = slots * (double)((together * q.nw + 3) / 4), alone = slots + (smem_tile ? 130.0 : 230.0);
+            const double cost = (double)((paths + together - 1) / together) * steps * (shared > alone ? shared : alone);
+            if (best_cost >= 0 && cost >= best_cost) continue;
+            q.grid = n < sms * res ? n : sms * res;
+            if (!smem_tile) {
+                const int64_t fit = (int64_t)(kNormTileCap / tile), most = fit > 0 ? fit : 1;
+                if (q.grid > most) q.grid = most;
             }
+            q.dx_off = 0;
+            q.tile_off = from_inc ? 0 : align256((size_t)n * (size_t)d * (size_t)nc * sizeof(double));
+            q.bnd_off = q.tile_off + (smem_tile ? 0 : align256((size_t)q.grid * tile));
+            q.ws_bytes = q.bnd_off + (q.smem_bnd ? 0 : align256((size_t)q.grid * rows));
+            best = q;
+            best_cost = cost;
         }
-        const int64_t m = nc << order;
-        q.pipe = true;
-        q.mode = mode;
-        q.R = R;
-        q.nw = (int)nw;
-        q.smem_cta = smem;
-        q.bnd_stride = ((m + 1 + 31) / 32) * 32;
-        q.prog_off = 0;
-        q.err_off = align256((size_t)n * kNormPipeMaxWarps * sizeof(int));
-        q.bnd_bytes = q.err_off + 256; // counters and flag, zeroed before each launch
-        const size_t rows = align256((size_t)n * (size_t)(nw - 1) * (size_t)q.bnd_stride * sizeof(double));
-        q.dx_off = q.bnd_bytes + rows;
-        q.ws_bytes = from_inc ? q.dx_off
-                              : q.dx_off + align256((size_t)n * (size_t)d * (size_t)nc * sizeof(double));
     }
-    return q;
+    return best;
 }
 
 } // namespace
@@ -1618,7 +1615,13 @@ size_t sigk_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t len_x, int6
         n_y = n_x;
     }
     if (op == SIGK_OP_PAIRWISE) n_y = n_x;
-    if (op == SIGK_OP_NORMALIZE) return norm_plan(n_x, len_x - 1, dim > 0 ? dim : 1, order, dim == 0).ws_bytes;
+    if (op == SIGK_OP_NORMALIZE) {
+        const size_t nb = norm_plan(n_x, len_x - 1, dim > 0 ? dim : 1, order, dim == 0).ws_bytes;
+        if (dim > 0) return nb;
+        // increments given: the caller's k(x,x) come from sigk_pairwise_inc with the same workspace
+        const size_t pb = make_plan(SIGK_OP_NORMALIZE, n_x, n_x, len_x - 1, len_x - 1, 0, order, 8, true).ws_bytes;
+        return nb > pb ? nb : pb;
+    }
     if (is_tc(precision) && dim > 0) {
         const int kop = op == SIGK_OP_PAIRWISE ? kOpPairwise : op == SIGK_OP_GRAM ? kOpGram : kOpGramSym;
         const FtPlan f = make_fused_plan(kop, n_x, n_y, len_x - 1, len_y - 1, dim, order, precision);
@@ -1846,59 +1849,37 @@ static int normalize_impl(const void *x, const void *inc, int64_t n, int64_t nc,
         if (e != cudaSuccess) return cuda_fail(e, "delta kernel launch");
     }
     NormParams p{};
-    p.x = x;
-    p.dx = dx;
-    p.tile_pitch = q.tile_pitch;
     p.n = n;
-    p.nc = nc;
-    p.d = d;
+    p.nc = (int)nc;
     p.order = order;
-    p.fscale = from_inc ? 1.0 : static_scale * std::ldexp(1.0, -2 * order);
+    p.d = d;
+    p.dx = dx;
     p.inc = inc;
     p.is0 = s0;
     p.is1 = s1;
     p.is2 = s2;
+    p.in64 = dtype == SIGK_F64;
+    p.fscale = from_inc ? 1.0 : static_scale * std::ldexp(1.0, -2 * order);
+    p.nbands = q.nbands;
+    p.nw = q.nw;
+    p.nsteps = q.nsteps;
+    p.pitch = q.pitch;
+    p.col0 = q.col0;
+    p.tile = q.tile;
+    p.tiles = q.smem_tile ? nullptr : reinterpret_cast<double *>(wsb + q.tile_off);
+    p.bnd = q.smem_bnd ? nullptr : reinterpret_cast<double *>(wsb + q.bnd_off);
     p.knorm = knorm;
     p.fnorm = fnorm;
     p.tol = tol;
     p.maxit = maxit;
     p.lam = lam;
     p.iters = iters;
-    if (q.pipe) {
-        cudaError_t e = cudaMemsetAsync(wsb, 0, q.bnd_bytes, stream);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(progress)");
-        p.prog = reinterpret_cast<int *>(wsb + q.prog_off);
-        p.err = reinterpret_cast<int *>(wsb + q.err_off);
-        p.bnd = wsb + q.bnd_bytes;
-        p.bnd_stride = q.bnd_stride;
-        p.stage_smem = q.mode == kNormDelta && q.smem_cta > 0;
-        NormFn fn = get_norm_pipe_kernel(dtype == SIGK_F64, q.mode, q.R, q.O);
-        if (q.smem_cta > 48 * 1024) {
-            int dev = 0, optin = 0;
-            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
-            if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
-                return cuda_fail(e, "cudaDeviceGetAttribute");
-            cudaFuncAttributes fa{};
-            if ((e = cudaFuncGetAttributes(&fa, (const void *)fn)) != cudaSuccess)
-                return cuda_fail(e, "cudaFuncGetAttributes");
-            const int dyn_max = optin - (int)fa.sharedSizeBytes; // the kernel's static shared memory counts too
-            if ((size_t)dyn_max < q.smem_cta)
-                return fail(SIGK_ELAUNCH, "normalisation needs %zu bytes of shared memory", q.smem_cta);
-            if ((e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max)) !=
-                cudaSuccess)
-                return cuda_fail(e, "cudaFuncSetAttribute");
-        }
-        const int64_t grid = n < 0x7fffffffLL ? n : 0x7fffffffLL; // one CTA per path (more paths: strided)
-        fn<<<(unsigned)grid, q.nw * 32, q.smem_cta, stream>>>(p);
-        count_launch();
-        e = cudaGetLastError();
-        return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "pipelined normalisation launch");
-    }
-    p.bnd = q.nbands > 1 ? ws : nullptr;
-    p.bnd_stride = q.bnd_stride;
-    p.stage_smem = q.smem_per_warp > 0;
-    NormFn fn = get_norm_kernel(dtype == SIGK_F64, q.mode, q.R, q.O);
-    return launch(fn, p, n, q.smem_per_warp * kWarpsPerBlock, stream);
+    int nb = 0; // opts the kernel in to its shared memory
+    if ((st = blocks_per_sm((const void *)q.k.fn, q.smem, &nb, q.threads))) return st;
+    q.k.fn<<<(unsigned)q.grid, q.threads, q.smem, stream>>>(p);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "normalisation launch");
 }
 
 static int run_normalize(const void *x, const void *inc, int64_t n, int64_t nc, int64_t d, int64_t s0, int64_t s1,

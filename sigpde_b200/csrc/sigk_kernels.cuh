@@ -1,13 +1,11 @@
 // sigk_kernels.cuh -- persistent-warp kernels built on warp_solve (wave.cuh).
 //
 //   pair_kernel       pairwise / Gram / symmetric-Gram signature kernels
-//   normalize_kernel  robust normalisation: per-path Chandrupatla root-find
-//                     whose every iteration re-solves the PDE on-chip
 //
-// Each kernel is a grid of 4-warp blocks sized to the resident capacity of
-// the device; warp w handles work items w, w + W, w + 2W, ... (W = warps in
-// the grid).  Gram items are numbered row-major, so neighbouring warps share
-// x_i and read neighbouring y_j (L1/L2 reuse).
+// A grid of 4-warp blocks sized to the resident capacity of the device; warp w
+// handles work items w, w + W, w + 2W, ... (W = warps in the grid).  Gram items
+// are numbered row-major, so neighbouring warps share x_i and read neighbouring
+// y_j (L1/L2 reuse).
 #pragma once
 
 #include <type_traits>
@@ -141,164 +139,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) pair_kernel(PairParams p)
                 out[xi * p.out_ld + yj] = TIN(val);
                 if (p.op == kOpGramSym && xi != yj) out[yj * p.out_ld + xi] = TIN(val);
             }
-        }
-    }
-}
-
-enum : int { kNormDelta = 0, kNormGiven = 1, kNormTile = 2 };
-
-struct NormParams {
-    const void *x;
-    const double *dx;   // delta / tile modes: path differences (n, d, nc), dimension-major, unscaled
-    int64_t tile_pitch; // tile mode: row pitch (elements) of the shared-memory increment tile
-    int64_t n;
-    int64_t nc;
-    int64_t d;
-    int order;
-    double fscale;      // static_scale * 4^-order (path mode) or 1
-    const void *inc;    // increment mode only
-    int64_t is0, is1, is2;
-    double *knorm;      // builtin: output (may be null); external: input
-    const double *fnorm; // null: builtin f(s) = 2 - 1/(1 + log s)
-    double tol;
-    int maxit;
-    void *lam;
-    int *iters;
-    void *bnd;
-    int64_t bnd_stride;
-    int stage_smem;
-    // pipelined kernel (norm_pipe.cuh): per-CTA band progress counters (16 ints per CTA,
-    // zeroed before the launch) and the flag a band wait that ran out sets
-    int *prog;
-    int *err;
-};
-
-// k(x,x), f(k) and the Chandrupatla iteration for one path, given solve(s) =
-// k at increments scaled by s: sigpde/cuda_pairwise_kernels.py:88-165 with
-// the argument order of sigpde/torch/kernel.py:186-193: g(l) = k(l x) - f(k),
-// g(0) = 1 - f(k), g(1) = k - f(k).  All bracket state is float64 and uniform
-// across the threads that call it (solve returns the same value to all of
-// them); `writer` stores k(x,x).
-template <class Solve>
-__device__ __forceinline__ void normalize_path(const NormParams &p, int64_t b, bool writer, Solve &&solve,
-                                               double &out, int &it)
-{
-    double k, fk;
-    if (p.fnorm == nullptr) {
-        k = solve(1.0);
-        if (isnan(k)) k = __longlong_as_double(0x7ff0000000000000LL); // NaN -> +inf (kernel.py:183)
-        fk = 2.0 - 1.0 / (1.0 + log(k));                              // kernel.py:23-24
-        if (p.knorm && writer) p.knorm[b] = k;
-    } else {
-        k = p.knorm[b];
-        fk = p.fnorm[b];
-    }
-    out = 0.0;
-    it = 0;
-    if (k >= 1.0) { // lambda is forced to 0 for k < 1 (kernel.py:195), so the loop is skipped
-        double a = 0.0, c = 0.0, bb = 1.0;
-        double fa = 1.0 - fk;
-        double fb = k - fk;
-        double fc = fa;
-        double t = 0.5;
-        for (it = 0; it < p.maxit;) {
-            const double xt = a + t * (bb - a);
-            const double sol = solve(xt * xt);
-            const double ft = isnan(sol) ? __longlong_as_double(0x7ff0000000000000LL) : sol - fk;
-            ++it;
-            if (ft * fa >= 0) {
-                c = a;
-                fc = fa;
-            } else {
-                c = bb;
-                bb = a;
-                fc = fb;
-                fb = fa;
-            }
-            a = xt;
-            fa = ft;
-            if (fabs(fa) < fabs(fb)) {
-                out = a;
-                if (fabs(fa) < p.tol) break;
-            } else {
-                out = bb;
-                if (fabs(fb) < p.tol) break;
-            }
-            const double xi = (a - bb) / (c - bb);
-            const double phi = (fa - fb) / (fc - fb);
-            if (phi * phi < xi && (1 - phi) * (1 - phi) < 1 - xi)
-                t = fa / (fb - fa) * fc / (fb - fc) + (c - a) / (bb - a) * fa / (fc - fa) * fb / (fc - fb);
-            else
-                t = 0.5;
-            if (!(0 < t && t < 1)) t = 0.5;
-        }
-    }
-}
-
-// One path per warp: every bracket iteration re-solves the path's PDE on chip.
-template <typename TIN, int R, int O, int MODE>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) normalize_kernel(NormParams p)
-{
-    using T = double;
-    using BS = BlockShape<R, O>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    const SolveGeom g = make_geom<R, O>(p.nc, p.nc, p.order);
-    T *bnd = p.bnd ? reinterpret_cast<T *>(p.bnd) + gwarp * p.bnd_stride : nullptr;
-    TIN *lam_out = reinterpret_cast<TIN *>(p.lam);
-
-    for (int64_t b = gwarp; b < p.n; b += nwarps) {
-        DeltaIncs<T, BS::RC> dsrc;
-        GivenIncs<T, TIN, BS::RC> gsrc;
-        TileIncs<T, BS::RC> tsrc;
-        if constexpr (MODE == kNormGiven) {
-            gsrc.inc = reinterpret_cast<const TIN *>(p.inc) + b * p.is0;
-            gsrc.si = p.is1;
-            gsrc.sj = p.is2;
-        } else if constexpr (MODE == kNormDelta) {
-            dsrc.dX = p.dx + b * p.d * p.nc;
-            dsrc.dY = dsrc.dX;
-            dsrc.d = p.d;
-            dsrc.ncy = p.nc;
-            dsrc.dxs = p.stage_smem ? reinterpret_cast<T *>(smem_raw) + (int64_t)wib * BS::RC * p.d * 32 : nullptr;
-        } else {
-            // build this path's coarse increment tile once: tile[cj][ci] = <dx_ci, dx_cj>
-            T *tile = reinterpret_cast<T *>(smem_raw) + (int64_t)wib * p.nc * p.tile_pitch;
-            const double *dxb = p.dx + b * p.d * p.nc;
-            __syncwarp(); // the previous path's solves are done with the tile
-            for (int64_t e = lane; e < p.nc * p.nc; e += 32) {
-                const int64_t cj = e / p.nc;
-                const int64_t ci = e - cj * p.nc;
-                T acc = T(0);
-                for (int64_t k = 0; k < p.d; ++k) acc = fma(dxb[k * p.nc + ci], dxb[k * p.nc + cj], acc);
-                tile[cj * p.tile_pitch + ci] = acc;
-            }
-            __syncwarp();
-            tsrc.tile = tile;
-            tsrc.pitch = p.tile_pitch;
-        }
-        auto solve = [&](double scale) -> double {
-            if constexpr (MODE == kNormGiven) {
-                gsrc.fscale = p.fscale * scale;
-                return warp_solve<T, R, O>(g, gsrc, bnd);
-            } else if constexpr (MODE == kNormDelta) {
-                dsrc.fscale = p.fscale * scale;
-                return warp_solve<T, R, O>(g, dsrc, bnd);
-            } else {
-                tsrc.fscale = p.fscale * scale;
-                return warp_solve<T, R, O>(g, tsrc, bnd);
-            }
-        };
-
-        double out = 0.0;
-        int it = 0;
-        normalize_path(p, b, lane == 0, solve, out, it);
-        if (lane == 0) {
-            if (lam_out) lam_out[b] = TIN(out);
-            if (p.iters) p.iters[b] = it;
         }
     }
 }

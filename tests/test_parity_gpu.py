@@ -397,6 +397,23 @@ def test_robust_normalization_increment_sources(sig, oracle, L, d, order, monkey
     np.testing.assert_array_equal(host(rk.normalization(X)), lam)
 
 
+@pytest.mark.parametrize("n,L,d,order", [(3, 2, 3, 0), (2, 2, 2, 5), (3, 33, 2, 0), (3, 34, 3, 0), (3, 129, 2, 0),
+                                         (3, 65, 2, 2), (2, 70, 2, 4), (2, 131, 3, 3), (2, 300, 2, 0), (2, 260, 2, 4),
+                                         (1500, 6, 2, 1)])
+def test_robust_normalization_band_edges(sig, oracle, n, L, d, order, monkeypatch):
+    """Paths that end at, just before and just after a band of rows and a lane step, more bands than a
+    CTA has warps, more paths than CTAs, with the increments in shared memory and in the workspace."""
+    x = oracle.brownian(n, L, d, 81 + L, scale=np.linspace(0.7, 4.0, n))
+    X = cuda(x, torch.float64)
+    rk = sig.RobustSigPDE(sig.kernels.LinearKernel(), order)
+    idx = np.unique(np.linspace(0, n - 1, 12).astype(int))
+    want = oracle.normalization(x[idx], order)
+    lam = host(rk.normalization(X))
+    np.testing.assert_allclose(lam[idx], want, rtol=LAM_RTOL, atol=1e-9)
+    monkeypatch.setenv("SIGK_NO_NORM_TILE", "1")
+    np.testing.assert_array_equal(host(rk.normalization(X))[idx], lam[idx])
+
+
 @pytest.mark.parametrize("shape", [(7, 6, 40, 24, 2), (9, 9, 64, 32, 0), (5, 4, 300, 24, 1), (6, 6, 12, 16, 4),
                                    (7, 6, 40, 16, 2)])
 def test_fp64_wide_paths_use_a_float64_increment_matrix(sig, oracle, shape, monkeypatch):
