@@ -452,7 +452,8 @@ __global__ void __launch_bounds__(kFtWarps * 32, 1) fused_tc_kernel(FusedTcParam
     for (int c = 0; c < C; ++c) bot[c] = one;
     Dbl2 corner_next = one;
     int col = 0;
-    int64_t grp = 0, xi = 0, ya = 0;
+    int64_t xi = 0, ya = 0;
+    int64_t nxi = 8 * (g0 / p.hy) + 4 * h + q, nya = 2 * (g0 % p.hy); // of the group that starts next
     for (int64_t b = 0; b < nbound; ++b) {
         boundary(b);
         const int64_t s1 = (b + 1) * RING < S ? (b + 1) * RING : S;
@@ -470,9 +471,13 @@ __global__ void __launch_bounds__(kFtWarps * 32, 1) fused_tc_kernel(FusedTcParam
             const int64_t u = s - lam;
             if (u >= 0 && u < nlocal) {
                 if (col == 0) {
-                    const int64_t g = g0 + grp, a = g / p.hy;
-                    xi = 8 * a + 4 * h + q;
-                    ya = 2 * (g - a * p.hy);
+                    xi = nxi;
+                    ya = nya;
+                    nya += 2;
+                    if (nya == 2 * p.hy) {
+                        nya = 0;
+                        nxi += 8;
+                    }
 #pragma unroll
                     for (int i = 0; i < R; ++i) left[i] = one;
                 }
@@ -493,10 +498,7 @@ __global__ void __launch_bounds__(kFtWarps * 32, 1) fused_tc_kernel(FusedTcParam
                         if (ya + 1 < p.ny) stream_store(sp, 0, xi, ya + 1, v.y);
                     }
                 }
-                if (++col == Tp) {
-                    col = 0;
-                    ++grp;
-                }
+                if (++col == Tp) col = 0;
             }
         }
     }

@@ -94,6 +94,22 @@ __device__ __forceinline__ void stream_decode(const StreamParams &p, int64_t ite
     }
 }
 
+// The item after (xi, yj) in a run.  Every lane moves to its next item at its
+// own step, so this runs once per lane and item, in a divergent branch: decoding
+// the item's number there (a 64-bit division, for the triangle a float64 square
+// root) cost the Gram of 256 x 256 paths, L = 128, order 2, 0.22 of its 5.12 ms
+// and the symmetric Grams of short paths more.
+__device__ __forceinline__ void stream_next(int op, int64_t ny, int64_t &xi, int64_t &yj)
+{
+    ++yj;
+    if (op == kOpPairwise) {
+        ++xi;
+    } else if (yj > (op == kOpGram ? ny - 1 : xi)) {
+        yj = 0;
+        ++xi;
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void stream_store(const StreamParams &p, int64_t item, int64_t xi, int64_t yj, T v)
 {
@@ -214,6 +230,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_reg_paired_kernel(
     float2 corner_next = one;
     int q = 0, k = 0;
     int64_t ia = first, xa = 0, ya = 0, xb = 0, yb = 0;
+    int64_t nxa, nya; // the pair of items that starts next
+    stream_decode(p, first, nxa, nya);
     bool hasb = false;
     const float *dypa = dY, *dypb = dY;
 
@@ -233,13 +251,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_reg_paired_kernel(
             if (q == 0) { // this lane starts items first + 2k, first + 2k + 1
                 ia = first + 2 * k;
                 hasb = 2 * k + 1 < cnt;
-                stream_decode(p, ia, xa, ya);
-                if (hasb) {
-                    stream_decode(p, ia + 1, xb, yb);
-                } else {
-                    xb = xa;
-                    yb = ya;
-                }
+                xa = nxa;
+                ya = nya;
+                stream_next(p.op, p.ny, nxa, nya);
+                xb = hasb ? nxa : xa;
+                yb = hasb ? nya : ya;
+                stream_next(p.op, p.ny, nxa, nya);
                 dypa = dY + ya * (int64_t)D * ncy;
                 dypb = dY + yb * (int64_t)D * ncy;
                 if (xa != cur_xa || xb != cur_xb) {
@@ -322,7 +339,7 @@ __device__ __forceinline__ Dbl2 stencil_cell<Dbl2>(Dbl2 k00, Dbl2 k01, Dbl2 k10,
 // step's cells, where the loads and dot products, which do not depend on the
 // cells, fill the cells' latency gaps (Gram 256 x 256, L = 128, d = 8, order
 // 2: 5.13 ms against 5.31 ms with the increments formed in-step).  The next
-// entry of the run is decoded one entry ahead, when the current one starts;
+// entry of the run is found one entry ahead, when the current one starts;
 // when it has another x path, the dot products formed with the old dx are
 // discarded and redone after the dx reload (rare: a run moves to a new x path
 // at most a few times).
@@ -416,7 +433,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 
                     stream_dot<T, D, RC>(dx, dyp, ncy, cc);
                 }
                 if (k + 1 < cnt) {
-                    stream_decode(p, item + 1, nxi, nyj);
+                    stream_next(p.op, p.ny, nxi, nyj);
                     ndyp = dY + nyj * ystride;
                 }
 #pragma unroll
@@ -467,17 +484,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
     const Dbl2 one{1.0, 1.0};
 
     // entry pair t -> x path t / hy, y paths ya = 2 (t % hy) and ya + 1 (absent when ya + 1 == ny)
-    auto decode = [&](int64_t t, int64_t &x, int64_t &ya, bool &hasb, const double *&pa, const double *&pb) {
-        x = t / hy;
-        ya = 2 * (t - x * hy);
-        hasb = ya + 1 < p.ny;
-        pa = dY + ya * ystride;
-        pb = hasb ? pa + ystride : pa;
-    };
-    int64_t xi = 0, ya = 0, nxi, nya;
+    int64_t xi = 0, ya = 0, nxi = first / hy, nya = 2 * (first - nxi * hy);
     bool hasb = false, nhasb;
     const double *dypa, *dypb, *ndypa, *ndypb;
-    decode(first, nxi, nya, nhasb, ndypa, ndypb);
+    auto paths = [&]() { // of the next entry pair
+        nhasb = nya + 1 < p.ny;
+        ndypa = dY + nya * ystride;
+        ndypb = nhasb ? ndypa + ystride : ndypa;
+    };
+    paths();
     dypa = ndypa;
     dypb = ndypb;
     double dx[RC][D];
@@ -521,7 +536,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
                     stream_dot<double, D, RC>(dx, dypa, ncy, cca);
                     stream_dot<double, D, RC>(dx, dypb, ncy, ccb);
                 }
-                if (k + 1 < cnt) decode(first + k + 1, nxi, nya, nhasb, ndypa, ndypb);
+                if (k + 1 < cnt) {
+                    nya += 2;
+                    if (nya >= p.ny) {
+                        nya = 0;
+                        ++nxi;
+                    }
+                    paths();
+                }
 #pragma unroll
                 for (int r = 0; r < R; ++r) left[r] = one;
             }
@@ -585,14 +607,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
     int64_t item = first, xi = 0, yj = 0;
     const T *dyp = dY;
     const T *dxs = buf0;
+    int64_t sxi, syj;   // the next pair to stage
+    stream_decode(p, first, sxi, syj);
+    int64_t nxi = sxi, nyj = syj; // the lane's next pair
     int staged = 0;     // pairs staged so far (warp-uniform)
     int next_stage = 0; // step at which lane 0 starts pair `staged`
 
     const int total = cnt * nsteps + 31;
     for (int s = 0; s < total; ++s) {
         if (staged < cnt && s == next_stage) { // warp-uniform: lane 0 starts a new pair now
-            int64_t sxi, syj;
-            stream_decode(p, first + staged, sxi, syj);
             T *dst = (staged & 1) ? buf1 : buf0;
             const T *src = dX + sxi * (int64_t)d * ncx;
             __syncwarp();
@@ -602,6 +625,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
                 for (int kk = 0; kk < d; ++kk) dst[(rc * d + kk) * 32 + lane] = ok ? src[kk * ncx + ci] : T(0);
             }
             __syncwarp();
+            stream_next(p.op, p.ny, sxi, syj);
             ++staged;
             next_stage += nsteps;
         }
@@ -615,7 +639,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
         if (s >= lane && k < cnt) {
             if (q == 0) {
                 item = first + k;
-                stream_decode(p, item, xi, yj);
+                xi = nxi;
+                yj = nyj;
+                stream_next(p.op, p.ny, nxi, nyj);
                 dyp = dY + yj * (int64_t)d * ncy;
                 dxs = (k & 1) ? buf1 : buf0;
 #pragma unroll

@@ -779,25 +779,28 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
     unsigned char *ring = ring_mem + ((size_t)wib * Ring::SLOTS * 32 + lane) * Ring::VB;
     constexpr int kSlot = 32 * Ring::VB; // bytes between the slots of one lane
     int rd = 0, wr = 0;                  // slots to read / fill next
-    int tp = 0, kp = 0, qp = 0;          // step, item and column of the next copy
+    int tp = 0, qp = 0;                  // step and column of the next copy
     const TM *bp = inc;
+    // the items that the lane's steps and its copies start next
+    int64_t nxi = 0, nyj = 0, cxi, cyj;
+    if (cnt > 0) stream_decode(sp, p.item0 + first, nxi, nyj);
+    cxi = nxi;
+    cyj = nyj;
+    auto block = [&](int64_t x, int64_t y) { // the pair's increments
+        return p.op == kOpPairwise ? inc + (x - p.item0) * (int64_t)ncy * p.rows_x
+                                   : inc + y * (int64_t)ncy * p.ld + (x - p.x0) * p.rows_x;
+    };
     const int tsteps = cnt * nsteps;
     auto issue = [&]() {
         if (tp < tsteps) {
             if (qp == 0) {
-                int64_t a, b;
-                const int64_t it = p.item0 + first + kp;
-                stream_decode(sp, it, a, b);
-                bp = p.op == kOpPairwise ? inc + (it - p.item0) * (int64_t)ncy * p.rows_x
-                                         : inc + b * (int64_t)ncy * p.ld + (a - p.x0) * p.rows_x;
+                bp = block(cxi, cyj);
+                stream_next(sp.op, sp.ny, cxi, cyj);
             }
             const int cj = (O <= 3) ? qp : ((qp * C) >> p.order);
             ring_fill<TM, RC>((uint32_t)__cvta_generic_to_shared(ring + wr * kSlot), bp + (int64_t)cj * row_ld, ci0,
                               ncx);
-            if (++qp == nsteps) {
-                qp = 0;
-                ++kp;
-            }
+            if (++qp == nsteps) qp = 0;
             ++tp;
         }
         cp_async_commit(); // empty groups past the end keep the count uniform
@@ -811,18 +814,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
     auto fetch = [&]() {
         if (tp < tsteps) {
             if (qp == 0) {
-                int64_t a, b;
-                const int64_t it = p.item0 + first + kp;
-                stream_decode(sp, it, a, b);
-                bp = p.op == kOpPairwise ? inc + (it - p.item0) * (int64_t)ncy * p.rows_x
-                                         : inc + b * (int64_t)ncy * p.ld + (a - p.x0) * p.rows_x;
+                bp = block(cxi, cyj);
+                stream_next(sp.op, sp.ny, cxi, cyj);
             }
             const int cj = (O <= 3) ? qp : ((qp * C) >> p.order);
             load_mat_raw<TM, RC>(bp + (int64_t)cj * row_ld, ci0, ncx, nxt);
-            if (++qp == nsteps) {
-                qp = 0;
-                ++kp;
-            }
+            if (++qp == nsteps) qp = 0;
             ++tp;
         }
     };
@@ -841,10 +838,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
         if (s >= sl && k < cnt) {
             if (q == 0) {
                 item = p.item0 + first + k;
-                stream_decode(sp, item, xi, yj);
-                if constexpr (PF == 0)
-                    base = p.op == kOpPairwise ? inc + (item - p.item0) * (int64_t)ncy * p.rows_x
-                                               : inc + yj * (int64_t)ncy * p.ld + (xi - p.x0) * p.rows_x;
+                xi = nxi;
+                yj = nyj;
+                stream_next(sp.op, sp.ny, nxi, nyj);
+                if constexpr (PF == 0 && !kRegPrefetch) base = block(xi, yj);
 #pragma unroll
                 for (int r = 0; r < R; ++r) left[r] = T(1);
             }
