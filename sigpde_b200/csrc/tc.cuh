@@ -617,83 +617,24 @@ __host__ __forceinline__ size_t tc_gemm_smem(int bn, int kp)
 }
 
 // ------------------------------------------------------------------ wavefront
-// Prefetch ring of stream_inc_kernel: each lane keeps the matrix values of its
-// next PF steps in flight as cp.async copies into its own shared-memory slots
-// (zero-filled where the lane's coarse rows start at or beyond ncx, as
-// load_mat_vals reads them), so a step waits for a copy issued PF steps
-// earlier rather than for a fresh global load.  Only the issuing lane reads a
-// slot, after cp.async.wait_group has made its copy visible to it.
-constexpr int kIncRingLaneBytes = 160; // shared memory per lane for the ring
-
-template <typename TM, int RC, int CELLS>
-struct IncRing {
-    static constexpr int VB = RC * (int)sizeof(TM);   // bytes per lane per step
-    static constexpr int CP = VB < 16 ? VB : 16;      // bytes per copy
-    // steps of lead: two for long steps (32 or more cells a lane); shorter steps measured slower
-    // with a ring (its bookkeeping costs more than the load latency it hides there)
-    static constexpr int STEPS = CELLS >= 32 ? 2 : 0;
-    static constexpr int CAP = kIncRingLaneBytes / VB - 1;
-    static constexpr int PF = STEPS < CAP ? STEPS : (CAP > 0 ? CAP : 0); // 0: plain loads (load_mat_vals)
-    static constexpr int SLOTS = PF + 1;
+// Lane step of stream_inc_kernel: R rows by C columns.  At orders 0 and 1 a step
+// takes several coarse columns: the shuffles, loads and control of a step cost
+// about as many issue slots as 16 cells do, and with one coarse column a step
+// they outweighed the cells (order 1, 8 rows: 110 other instructions to 60
+// float64 ones; RBF Gram 200 x 170, L = 128 / 111: 1.16 -> 0.87 ms of
+// wavefront).  A step that reaches beyond the last column is put before the
+// first one instead, with increments 0: K = 1 there exactly, so values do not
+// depend on the step's width.
+template <int R, int O, typename TM>
+struct IncShape {
+    static constexpr int RC = BlockShape<R, O>::RC;
+    // held in registers one step ahead: two columns up to 64 bytes a column, four up to 16 (order 0, 4 rows,
+    // float64, 51200 pairs: 1.06 ms with two, 1.58 with four; order 0, 8 rows, float64, 40000 pairs, L = 136: the
+    // Gram in 4.02 ms with two, 4.31 with one)
+    static constexpr int most = RC * (int)sizeof(TM) > 64 ? 1 : RC * (int)sizeof(TM) > 16 ? 2 : 4;
+    static constexpr int CC = O == 0 ? most : O == 1 ? (most < 2 ? most : 2) : 1; // coarse columns a step
+    static constexpr int C = CC * BlockShape<R, O>::C;
 };
-
-template <int SZ>
-__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void *src, int src_bytes)
-{
-    if constexpr (SZ == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(SZ), "r"(src_bytes)
-                     : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Copy the lane's RC values of one matrix row (chunks starting at or beyond
-// ncx are zero-filled without a read) into a ring slot.
-template <typename TM, int RC>
-__device__ __forceinline__ void ring_fill(uint32_t dst, const TM *row, int ci0, int ncx)
-{
-    constexpr int VB = RC * (int)sizeof(TM);
-    constexpr int CP = VB < 16 ? VB : 16;
-    constexpr int EPC = CP / (int)sizeof(TM);
-#pragma unroll
-    for (int q = 0; q < VB / CP; ++q) {
-        const bool ok = ci0 + q * EPC < ncx;
-        cp_async_zfill<CP>(dst + q * CP, ok ? row + ci0 + q * EPC : row, ok ? CP : 0);
-    }
-}
-
-template <typename T, typename TM, int RC>
-__device__ __forceinline__ void ring_read(const unsigned char *src, T (&c)[RC])
-{
-    if constexpr (RC == 1) {
-        c[0] = T(*reinterpret_cast<const TM *>(src));
-    } else if constexpr (sizeof(TM) == 8) {
-#pragma unroll
-        for (int q = 0; q < RC / 2; ++q) {
-            const double2 v = reinterpret_cast<const double2 *>(src)[q];
-            c[2 * q + 0] = T(v.x);
-            c[2 * q + 1] = T(v.y);
-        }
-    } else if constexpr (RC == 2) {
-        const float2 v = *reinterpret_cast<const float2 *>(src);
-        c[0] = T(v.x);
-        c[1] = T(v.y);
-    } else {
-#pragma unroll
-        for (int q = 0; q < RC / 4; ++q) {
-            const float4 v = reinterpret_cast<const float4 *>(src)[q];
-            c[4 * q + 0] = T(v.x);
-            c[4 * q + 1] = T(v.y);
-            c[4 * q + 2] = T(v.z);
-            c[4 * q + 3] = T(v.w);
-        }
-    }
-}
 
 struct StreamIncParams {
     int op;           // kOpPairwise / kOpGram / kOpGramSym
@@ -721,8 +662,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
 {
     static_assert(W == 32 || W == 16, "a pipeline is a warp or a half-warp");
     using BS = BlockShape<R, O>;
-    constexpr int C = BS::C;
-    constexpr int RC = BS::RC;
+    using IS = IncShape<R, O, TM>;
+    constexpr int C = IS::C, CC = IS::CC, RC = IS::RC, BC = BS::C;
     const int lane = threadIdx.x & 31;
     const int sl = lane & (W - 1); // lane within the pipeline
     const int wib = threadIdx.x >> 5;
@@ -736,7 +677,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
     const int cnt_max = (int)((p.nitems - wfirst) < p.per_warp ? (p.nitems - wfirst) : p.per_warp);
     const int ncx = (int)p.ncx, ncy = (int)p.ncy;
     const int n = ncx << p.order;
-    const int nsteps = (ncy << p.order) / C;
+    const int nsteps = ((ncy << p.order) + C - 1) / C;
+    const int off = CC > 1 ? nsteps * CC - ncy : 0; // columns before the first one
     const int ci0 = (sl * R) >> p.order;
     const int lstar = (n - 1) / R, rstar = (n - 1) % R;
     const int64_t row_ld = p.op == kOpPairwise ? p.rows_x : p.ld;
@@ -756,76 +698,51 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
         return;
     }
 
+    const TM *inc = reinterpret_cast<const TM *>(p.inc);
+    // the lane's current item, and the one whose increments are loaded
+    int64_t xi = 0, yj = 0, cxi, cyj;
+    if (cnt > 0) stream_decode(sp, p.item0 + first, xi, yj);
+    cxi = xi;
+    cyj = yj;
+    auto rows_of = [&](int64_t x, int64_t y) { // the lane's rows at column -off of the pair's increments
+        const TM *b = p.op == kOpPairwise ? inc + (x - p.item0) * (int64_t)ncy * p.rows_x
+                                          : inc + y * (int64_t)ncy * p.ld + (x - p.x0) * p.rows_x;
+        return b + ci0 - (int64_t)off * row_ld;
+    };
+    const TM *src = rows_of(cxi, cyj);
+    int tp = cnt * nsteps, qp = 0; // steps left to load, step of the item
+    // The next step's increments, loaded one step ahead, as stored: a conversion would wait for the load.
+    // (A ring of cp.async copies three steps ahead measured slower at most shapes: its shared-memory reads
+    // and copies are more instructions than it hides in latency.)
+    TM nxt[CC][RC];
+    auto fetch = [&]() {
+        if (tp > 0) {
+            --tp;
+#pragma unroll
+            for (int cc = 0; cc < CC; ++cc) {
+                const bool in = CC == 1 || qp > 0 || cc >= off;
+                const TM *col = O <= 3 ? src + cc * row_ld : src + (int64_t)((qp * C) >> p.order) * row_ld;
+                load_mat_raw<TM, RC>(col, in ? ci0 : ncx, ncx, nxt[cc]);
+            }
+            if constexpr (O <= 3) src += CC * row_ld;
+            if (++qp == nsteps) {
+                qp = 0;
+                stream_next(sp.op, sp.ny, cxi, cyj);
+                src = rows_of(cxi, cyj);
+            }
+        }
+    };
+
     T left[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) left[r] = T(1);
     T bot[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) bot[c] = T(1);
-    T corner_next = T(1);
-    int q = 0, k = 0;
-    int64_t item = 0, xi = 0, yj = 0;
-    const TM *inc = reinterpret_cast<const TM *>(p.inc);
-    const TM *base = inc;
-    const int total = cnt_max * nsteps + (W - 1);
-
-    // prefetch ring: the copy for the lane's step t + PF is issued at step t
-    using Ring = IncRing<TM, RC, R * C>;
-    // without a ring, float64 matrices load each step's values one step ahead into registers
-    // (config 3 fp64: 3.70 -> 3.27 ms); float32 matrices measured no gain (2.22 vs 2.25 ms)
-    constexpr bool kRegPrefetch = sizeof(TM) == 8;
-    constexpr int PF = Ring::PF;
-    __shared__ __align__(16) unsigned char ring_mem[PF > 0 ? kWarpsPerBlock * Ring::SLOTS * 32 * Ring::VB : 16];
-    unsigned char *ring = ring_mem + ((size_t)wib * Ring::SLOTS * 32 + lane) * Ring::VB;
-    constexpr int kSlot = 32 * Ring::VB; // bytes between the slots of one lane
-    int rd = 0, wr = 0;                  // slots to read / fill next
-    int tp = 0, qp = 0;                  // step and column of the next copy
-    const TM *bp = inc;
-    // the items that the lane's steps and its copies start next
-    int64_t nxi = 0, nyj = 0, cxi, cyj;
-    if (cnt > 0) stream_decode(sp, p.item0 + first, nxi, nyj);
-    cxi = nxi;
-    cyj = nyj;
-    auto block = [&](int64_t x, int64_t y) { // the pair's increments
-        return p.op == kOpPairwise ? inc + (x - p.item0) * (int64_t)ncy * p.rows_x
-                                   : inc + y * (int64_t)ncy * p.ld + (x - p.x0) * p.rows_x;
-    };
-    const int tsteps = cnt * nsteps;
-    auto issue = [&]() {
-        if (tp < tsteps) {
-            if (qp == 0) {
-                bp = block(cxi, cyj);
-                stream_next(sp.op, sp.ny, cxi, cyj);
-            }
-            const int cj = (O <= 3) ? qp : ((qp * C) >> p.order);
-            ring_fill<TM, RC>((uint32_t)__cvta_generic_to_shared(ring + wr * kSlot), bp + (int64_t)cj * row_ld, ci0,
-                              ncx);
-            if (++qp == nsteps) qp = 0;
-            ++tp;
-        }
-        cp_async_commit(); // empty groups past the end keep the count uniform
-        if (++wr == Ring::SLOTS) wr = 0;
-    };
-    if constexpr (PF > 0) {
-#pragma unroll 1
-        for (int i = 0; i < PF; ++i) issue();
-    }
-    TM nxt[RC]; // the lane's next step's values (kRegPrefetch)
-    auto fetch = [&]() {
-        if (tp < tsteps) {
-            if (qp == 0) {
-                bp = block(cxi, cyj);
-                stream_next(sp.op, sp.ny, cxi, cyj);
-            }
-            const int cj = (O <= 3) ? qp : ((qp * C) >> p.order);
-            load_mat_raw<TM, RC>(bp + (int64_t)cj * row_ld, ci0, ncx, nxt);
-            if (++qp == nsteps) qp = 0;
-            ++tp;
-        }
-    };
-    if constexpr (PF == 0) {
-        if (kRegPrefetch) fetch();
-    }
+    T corner = T(1);
+    int q = 0;
+    const int run = cnt * nsteps, total = cnt_max * nsteps + (W - 1);
+    fetch();
 
     for (int s = 0; s < total; ++s) {
         T top[C];
@@ -835,44 +752,36 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_inc_kernel(StreamI
 #pragma unroll
             for (int c = 0; c < C; ++c) top[c] = T(1);
         }
-        if (s >= sl && k < cnt) {
-            if (q == 0) {
-                item = p.item0 + first + k;
-                xi = nxi;
-                yj = nyj;
-                stream_next(sp.op, sp.ny, nxi, nyj);
-                if constexpr (PF == 0 && !kRegPrefetch) base = block(xi, yj);
+        if ((unsigned)(s - sl) < (unsigned)run) {
+            T cur[CC][RC];
+#pragma unroll
+            for (int cc = 0; cc < CC; ++cc)
+#pragma unroll
+                for (int rc = 0; rc < RC; ++rc) cur[cc][rc] = T(nxt[cc][rc]);
+            fetch();
+#pragma unroll
+            for (int cc = 0; cc < CC; ++cc) {
+                T A[RC], B[RC], t[BC], bt[BC];
+#pragma unroll
+                for (int rc = 0; rc < RC; ++rc) stencil_coefs(cur[cc][rc], A[rc], B[rc]);
+#pragma unroll
+                for (int c = 0; c < BC; ++c) t[c] = top[cc * BC + c];
+                stream_block<T, R, O>(left, t, corner, A, B, bt);
+                corner = t[BC - 1];
+#pragma unroll
+                for (int c = 0; c < BC; ++c) bot[cc * BC + c] = bt[c];
+            }
+            if (++q == nsteps) { // the lane's next item starts
+                q = 0;
+                if (sl == lstar)
+                    stream_store(sp, p.op == kOpPairwise ? xi : 0, xi, yj, pick_row(left, rstar));
+                stream_next(sp.op, sp.ny, xi, yj);
 #pragma unroll
                 for (int r = 0; r < R; ++r) left[r] = T(1);
-            }
-            const T corner = (q == 0) ? T(1) : corner_next;
-            corner_next = top[C - 1];
-            T cur[RC];
-            if constexpr (PF > 0) {
-                cp_async_wait<PF - 1>(); // this step's copy has landed
-                ring_read<T, TM, RC>(ring + rd * kSlot, cur);
-                if (++rd == Ring::SLOTS) rd = 0;
-                issue();
-            } else if (kRegPrefetch) {
-#pragma unroll
-                for (int rc = 0; rc < RC; ++rc) cur[rc] = T(nxt[rc]);
-                fetch();
-            } else {
-                const int cj = (O <= 3) ? q : ((q * C) >> p.order);
-                load_mat_vals<T, TM, RC>(base + (int64_t)cj * row_ld, ci0, ncx, cur);
-            }
-            T A[RC], B[RC];
-#pragma unroll
-            for (int rc = 0; rc < RC; ++rc) stencil_coefs(cur[rc], A[rc], B[rc]);
-            stream_block<T, R, O>(left, top, corner, A, B, bot);
-            if (q == nsteps - 1 && sl == lstar) stream_store(sp, item, xi, yj, pick_row(left, rstar));
-            if (++q == nsteps) {
-                q = 0;
-                ++k;
+                corner = T(1);
             }
         }
     }
-    if constexpr (PF > 0) cp_async_wait<0>();
 }
 
 } // namespace sigk

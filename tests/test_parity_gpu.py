@@ -437,6 +437,23 @@ def test_fp64_wide_paths_use_a_float64_increment_matrix(sig, oracle, shape, monk
     assert_rel(got[1], oracle.gram(x, None, o), RTOL64, "sym")
 
 
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("L", [20, 70, 200, 300])
+def test_increment_matrix_step_remainders(sig, oracle, L, order, monkeypatch):
+    """Matrix wavefronts that take several coarse columns a step: every remainder of the columns, at each
+    number of rows a lane, bitwise the one-column fused path."""
+    k = sig.SigPDE(sig.kernels.LinearKernel(), order)
+    X = cuda(oracle.brownian(3, L, 16, 91 + L), torch.float64)
+    for ly in (34, 35, 36, 37):
+        Y = cuda(oracle.brownian(4, ly, 16, 92 + ly), torch.float64)
+        monkeypatch.delenv("SIGK_NO_DGEMM_INC", raising=False)
+        got = [host(k.gram(X, Y)), host(k.gram(Y))]
+        monkeypatch.setenv("SIGK_NO_DGEMM_INC", "1")
+        for a, b in zip(got, [host(k.gram(X, Y)), host(k.gram(Y))]):
+            np.testing.assert_array_equal(a, b)
+        assert_rel(got[0], oracle.gram(host(X), host(Y), order), RTOL64, "gram")
+
+
 def test_robust_normalization_alternating_shared_memory_sizes(sig, oracle):
     """One kernel instance launched with large, then smaller, then large
     shared-memory tiles (the per-function opt-in must cover all of them)."""
