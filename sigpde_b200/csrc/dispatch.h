@@ -9,6 +9,7 @@ namespace sigk {
 
 struct PairParams;
 struct NormParams;
+struct PairWaveParams;
 struct StreamParams;
 struct RaggedParams;
 struct StreamIncParams;
@@ -27,6 +28,7 @@ namespace sigk {
 
 using PairFn = void (*)(PairParams);
 using NormFn = void (*)(NormParams);
+using PairWaveFn = void (*)(PairWaveParams);
 using StreamFn = void (*)(StreamParams);
 using RaggedFn = void (*)(RaggedParams);
 using RaggedDeltaFn = void (*)(const void *, const int64_t *, const int64_t *, const int *, double, const void *,
@@ -52,6 +54,12 @@ struct NormKernel {
 };
 // smem_tile, smem_bnd: increments, bottom rows in shared memory (a tile there only with the rows)
 NormKernel get_norm_kernel(int R, int O, bool smem_tile, bool smem_bnd);
+// few pairs, one CTA each (pair_wave.cuh): R in {2,4,8} rows a lane; fn null where not built
+struct PairWaveKernel {
+    PairWaveFn fn;
+    int cols, rc, ccols, max_warps;
+};
+PairWaveKernel get_pair_wave_kernel(int R, int O);
 // D: dimension padded to a power of two in {2,...,32}; returns null unless
 // the lane's register tile (coarse rows per lane) * D <= 32.
 StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D);

@@ -248,8 +248,11 @@ __device__ __forceinline__ void norm_build_tile(const NormParams &p, int64_t b, 
 // which gives 1 exactly; after its last one it runs on, and the run ends with
 // the step that finishes row n.  A step's coefficients are formed during the
 // step before, from increments loaded PF steps earlier.
-template <int R, int O, bool SMEM, bool BSMEM>
-__device__ __forceinline__ double norm_solve(const NormParams &p, const double *tile, double *bnd, double f,
+// P: NormParams, or another kernel's parameters with the same geometry (nc: rows
+// of the pair).  CHAIN: one dependent operation a cell down a column instead of
+// two; without it the cells are those of stencil_cell, bit for bit.
+template <int R, int O, bool SMEM, bool BSMEM, bool CHAIN, class P>
+__device__ __forceinline__ double norm_solve(const P &p, const double *tile, double *bnd, double f,
                                              double *s_val)
 {
     using NS = NormShape<R, O>;
@@ -309,9 +312,8 @@ __device__ __forceinline__ double norm_solve(const NormParams &p, const double *
                         double up = top[c], dg = c == 0 ? corner : top[c > 0 ? c - 1 : 0];
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
-                            // one dependent operation a cell down the column, not two
-                            const double l = left[r], a = A[cc][NS::rc_of(r)];
-                            up = fma(up, a, fma(l, a, -(dg * B[cc][NS::rc_of(r)])));
+                            const double l = left[r], a = A[cc][NS::rc_of(r)], bb = B[cc][NS::rc_of(r)];
+                            up = CHAIN ? fma(up, a, fma(l, a, -(dg * bb))) : stencil_cell(dg, up, l, a, bb);
                             dg = l;
                             left[r] = up;
                         }
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(NormShape<R, O>::MAXW * 32, 1) norm_kernel(Nor
         __syncthreads();
         if ((threadIdx.x >> 5) < p.nw) {
             auto solve = [&](double scale) -> double {
-                return norm_solve<R, O, SMEM, BSMEM>(p, tile, bnd, p.fscale * scale, &s_val);
+                return norm_solve<R, O, SMEM, BSMEM, true>(p, tile, bnd, p.fscale * scale, &s_val);
             };
             double out = 0.0;
             int it = 0;

@@ -22,7 +22,7 @@
 #include "ragged.cuh"
 #include "stream.cuh"
 #include "tc.cuh"
-#include "norm_wave.cuh"
+#include "pair_wave.cuh"
 #include "dgemm_inc.cuh"
 #include "static_inc.cuh"
 #include "grad.cuh"
@@ -1353,6 +1353,107 @@ int run_backward_inc(const GradPlan &g, const void *inc, int64_t npairs, int64_t
     return SIGK_OK;
 }
 
+// ------------------------------------------------------------------ few pairs
+// Plan of a call with few pairs (pair_wave.cuh): float64 cells of linear-kernel pairs whose increment tile
+// fits shared memory.
+struct PairWavePlan {
+    bool ok = false;
+    PairWaveKernel k{};
+    int nbands = 0, nw = 0, nsteps = 0, pitch = 0, col0 = 0, tile = 0, threads = 0;
+    int64_t items = 0;
+    size_t smem = 0;
+};
+
+constexpr size_t kPairWaveSmemBytes = 220 * 1024;
+
+PairWavePlan make_pair_wave_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order)
+{
+    PairWavePlan best;
+    const int64_t items = op == kOpPairwise ? nx : (op == kOpGram ? nx * ny : nx * (nx + 1) / 2);
+    const int sms = sm_count();
+    const int64_t per_sm = (items + sms - 1) / sms;
+    // a switch that asks for another float64 route asks for that one
+    if (per_sm > 64 || env_flag("SIGK_NO_PAIR_WAVE") || env_flag("SIGK_NO_STREAM") || env_flag("SIGK_NO_DGEMM_INC") ||
+        env_flag("SIGK_NO_DGEMM_PIPE") || env_flag("SIGK_NO_REG_DX"))
+        return best;
+    if (ncx > 4096 || ncy > 4096 || d > 4096 || (ncx << order) > (1 << 20) || (ncy << order) > (1 << 20)) return best;
+    const int64_t n = ncx << order, m = ncy << order;
+    double best_cost = 0.0;
+    for (int R = 2; R <= 8; R *= 2) {
+        PairWavePlan q;
+        q.k = get_pair_wave_kernel(R, order >= 4 ? 4 : order);
+        if (!q.k.fn) continue;
+        q.nbands = (int)((n + 32 * R - 1) / (32 * R));
+        q.nw = q.nbands < q.k.max_warps ? q.nbands : q.k.max_warps;
+        q.nsteps = (int)((m + q.k.cols - 1) / q.k.cols);
+        q.col0 = q.nsteps * q.k.cols > m ? 1 : 0;
+        const int rc = q.k.rc, low = ((int)ncx + rc - 1) / rc * rc + rc;
+        q.pitch = rc == 1 ? (low + 1) / 2 * 2 : rc == 2 ? (low + 3) / 4 * 4 : (low + 1) / 4 * 4 + 2;
+        const int64_t tile = (ncy + q.col0) * q.pitch;
+        const int64_t rows = (int64_t)(1 + (q.nbands > 1 ? q.nw * q.nsteps : 0)) * q.k.cols;
+        q.smem = (size_t)(tile + rows + (ncx + ncy) * d) * sizeof(double);
+        if (q.smem > kPairWaveSmemBytes) continue;
+        q.tile = (int)tile;
+        q.threads = 32 * (q.nw > 4 ? q.nw : 4);
+        q.items = items;
+        int64_t res = (int64_t)((228 * 1024) / (q.smem + 1024));
+        if (res > 65536 / (q.threads * 128)) res = 65536 / (q.threads * 128);
+        const int64_t together = per_sm < res ? per_sm : res;
+        const double steps = (double)((q.nbands + q.nw - 1) / q.nw) * (q.nsteps + 31 + (q.nw - 1) * kNormLag);
+        const double slots = 1.15 * (6.0 * R * q.k.cols + 10.0 * rc * q.k.ccols + 50.0);
+        const double shared = slots * (double)((together * q.nw + 3) / 4), alone = slots + 130.0;
+        const double cost = (double)((per_sm + together - 1) / together) * steps * (shared > alone ? shared : alone);
+        if (best.ok && cost >= best_cost) continue;
+        q.ok = true;
+        best = q;
+        best_cost = cost;
+    }
+    if (!best.ok) return best;
+    // The streaming wavefront's time in the same unit (cycles): its longest warp's steps at a lone warp's cost, and
+    // two more launches.  Measured, us a call, here / there: 256 pairs, L = 128, d = 8, order 2: 128 / 182 (576 pairs
+    // 223 / 184); 300 pairs, L = 65, d = 3, order 1: 43 / 65; 1024 pairs, L = 64, d = 16, order 1: 71 / 84 (2025 pairs
+    // 111 / 96); 100 pairs, L = 100 / 90, d = 32, order 3: 109 / 275; 600 pairs, L = 101 / 77, d = 4, order 0: 71 / 72.
+    const int Rs = pick_rows(n), C = order >= 4 ? 8 : 1 << order;
+    const int64_t bands = (n + 32 * Rs - 1) / (32 * Rs), run = (items + 12 * sms - 1) / (12 * sms);
+    const double steps = bands > 1 ? (double)run * bands * (m / C + 31) : (double)run * (m / C) + 31;
+    if (best_cost > steps * (300.0 + 15.0 * Rs * C) + 12000.0) best.ok = false;
+    return best;
+}
+
+int run_pairs_wave(const PairWavePlan &q, int op, const void *x, const void *y, int64_t ny, int64_t lx, int64_t ly,
+                   int64_t d, int dtype, int order, double static_scale, const void *sx, const void *sy, void *out,
+                   int64_t out_ld, cudaStream_t stream)
+{
+    PairWaveParams p{};
+    p.op = op;
+    p.in64 = dtype == SIGK_F64;
+    p.x = x;
+    p.y = op == kOpGramSym ? x : y;
+    p.sx = sx;
+    p.sy = op == kOpGramSym ? sx : sy;
+    p.f = static_scale * std::ldexp(1.0, -2 * order);
+    p.ny = ny;
+    p.nc = (int)(lx - 1);
+    p.ncy = (int)(ly - 1);
+    p.d = d;
+    p.order = order;
+    p.out = out;
+    p.out_ld = out_ld;
+    p.nitems = q.items;
+    p.nbands = q.nbands;
+    p.nw = q.nw;
+    p.nsteps = q.nsteps;
+    p.pitch = q.pitch;
+    p.col0 = q.col0;
+    p.tile = q.tile;
+    int nb = 0; // opts the kernel in to its shared memory
+    if (int st = blocks_per_sm((const void *)q.k.fn, q.smem, &nb, q.threads)) return st;
+    q.k.fn<<<(unsigned)q.items, q.threads, q.smem, stream>>>(p);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "pair kernel launch");
+}
+
 int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int64_t lx, int64_t ly, int64_t d,
               int dtype, int order, double static_scale, const void *sx, const void *sy, void *out, int64_t out_ld,
               int precision, void *ws, size_t ws_bytes, cudaStream_t stream)
@@ -1387,6 +1488,9 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
         precision = cell_prec(precision); // shapes outside the TC plan: CUDA-core increments, same cells
     }
     if (precision == SIGK_PREC_FP64) {
+        const PairWavePlan q = make_pair_wave_plan(op, nx, ny, lx - 1, ly - 1, d, order);
+        if (q.ok)
+            return run_pairs_wave(q, op, x, y, ny, lx, ly, d, dtype, order, static_scale, sx, sy, out, out_ld, stream);
         TcPlan t = make_mat64_plan(op, nx, ny, lx - 1, ly - 1, d, order);
         if (t.ok) {
             if (!ws || ws_bytes < t.ws_bytes)
@@ -1632,6 +1736,8 @@ size_t sigk_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t len_x, int6
     }
     if (precision == SIGK_PREC_FP64 && dim > 0) {
         const int kop = op == SIGK_OP_PAIRWISE ? kOpPairwise : op == SIGK_OP_GRAM ? kOpGram : kOpGramSym;
+        // nothing is used; callers that size a buffer by this keep one
+        if (make_pair_wave_plan(kop, n_x, n_y, len_x - 1, len_y - 1, dim, order).ok) return 256;
         TcPlan t = make_mat64_plan(kop, n_x, n_y, len_x - 1, len_y - 1, dim, order);
         if (t.ok) return t.ws_bytes;
     }

@@ -437,6 +437,31 @@ def test_fp64_wide_paths_use_a_float64_increment_matrix(sig, oracle, shape, monk
     assert_rel(got[1], oracle.gram(x, None, o), RTOL64, "sym")
 
 
+@pytest.mark.parametrize("lx,ly,d,order", [(2, 2, 1, 0), (3, 40, 2, 0), (33, 34, 3, 0), (66, 35, 2, 0), (130, 20, 2, 0),
+                                           (17, 18, 5, 1), (34, 33, 3, 1), (66, 70, 4, 1), (9, 12, 3, 2), (40, 20, 33, 2),
+                                           (70, 15, 2, 2), (18, 20, 2, 3), (3, 9, 2, 4), (12, 5, 2, 6)])
+def test_few_pairs_bit_identical(sig, oracle, lx, ly, d, order, monkeypatch):
+    """Calls with few pairs (one CTA a pair): band, step and lane edges, scales, both input types, bitwise
+    the streaming and per-pair kernels (SIGK_NO_PAIR_WAVE=1) and within the fp64 bound of the oracle."""
+    k = sig.SigPDE(sig.kernels.LinearKernel(1.3), order)
+    x, y = oracle.brownian(3, lx, d, 17 + lx), oracle.brownian(3, ly, d, 18 + ly)
+
+    def values():
+        out = []
+        for dtype in (torch.float64, torch.float32):
+            X, Y = cuda(x, dtype), cuda(y, dtype)
+            sx, sy = cuda(np.linspace(0.6, 1.4, 3), dtype), cuda(np.linspace(1.2, 0.7, 3), dtype)
+            out += [host(v) for v in (k.gram(X, Y), k.gram(X, Y, sx, sy), k.gram(X), k.gram(X, None, sx),
+                                      k.pairwise(X, Y), k.pairwise(X, Y, sx, sy))]
+        return out
+
+    got = values()
+    assert_rel(got[0], oracle.gram(x * np.sqrt(1.3), y * np.sqrt(1.3), order), RTOL64, "gram")
+    monkeypatch.setenv("SIGK_NO_PAIR_WAVE", "1")
+    for a, b in zip(got, values()):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("order", [0, 1])
 @pytest.mark.parametrize("L", [20, 70, 200, 300])
 def test_increment_matrix_step_remainders(sig, oracle, L, order, monkeypatch):
@@ -444,6 +469,7 @@ def test_increment_matrix_step_remainders(sig, oracle, L, order, monkeypatch):
     number of rows a lane, bitwise the one-column fused path."""
     k = sig.SigPDE(sig.kernels.LinearKernel(), order)
     X = cuda(oracle.brownian(3, L, 16, 91 + L), torch.float64)
+    monkeypatch.setenv("SIGK_NO_PAIR_WAVE", "1")
     for ly in (34, 35, 36, 37):
         Y = cuda(oracle.brownian(4, ly, 16, 92 + ly), torch.float64)
         monkeypatch.delenv("SIGK_NO_DGEMM_INC", raising=False)
