@@ -847,7 +847,19 @@ TcPlan mat64_layout(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, in
 
 TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order)
 {
-    if (op == kOpPairwise || d < kDgMinDim || env_flag("SIGK_NO_DGEMM_INC")) return TcPlan{};
+    if (op == kOpPairwise || env_flag("SIGK_NO_DGEMM_INC")) return TcPlan{};
+    if (d < kDgMinDim) {
+        // Below that, where the fused kernels would read each lane's dx from shared memory: a streaming shape whose
+        // dx tile does not fit registers (ms, fused / matrix: 80 x 80, L = 200, order 0, d = 8: 2.04 / 0.90, with the
+        // tile in registers at d = 4: 0.41 / 0.83; 128 x 128, L = 120, order 1, d = 12: 2.51 / 0.97), and several
+        // bands from d = 8 on (80 x 80, L = 300, order 1: 4.55 / 3.32 at d = 8, 2.91 / 3.18 at d = 4).
+        const int64_t n = ncx << order, m = ncy << order;
+        const int Rs = pick_rows(n), C = order >= 4 ? 8 : 1 << order;
+        int Dp = 2;
+        while (Dp < d) Dp <<= 1;
+        const bool band = n <= 32 * Rs, regs = rows_per_coarse_lane(Rs, order) * Dp <= 32;
+        if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 : d < 8)) return TcPlan{};
+    }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,
     // which forms the dot products a step ahead of the cells (256 x 256, L = 64, d = 16, order 2: 1.97 vs
     // 2.19 ms; the same values).  Orders 0-1 (few cells a coarse column) and wider dx tiles keep the matrix.
@@ -1736,8 +1748,7 @@ size_t sigk_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t len_x, int6
     }
     if (precision == SIGK_PREC_FP64 && dim > 0) {
         const int kop = op == SIGK_OP_PAIRWISE ? kOpPairwise : op == SIGK_OP_GRAM ? kOpGram : kOpGramSym;
-        // nothing is used; callers that size a buffer by this keep one
-        if (make_pair_wave_plan(kop, n_x, n_y, len_x - 1, len_y - 1, dim, order).ok) return 256;
+        // calls with few pairs (pair_wave.cuh) use none of this: the size is that of the route they would take else
         TcPlan t = make_mat64_plan(kop, n_x, n_y, len_x - 1, len_y - 1, dim, order);
         if (t.ok) return t.ws_bytes;
     }
