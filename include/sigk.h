@@ -231,6 +231,19 @@ SIGK_API int sigk_backward_inc(const void *inc, int64_t npairs, int64_t nc_x, in
                                void *workspace, size_t workspace_bytes, sigk_stream_t stream);
 
 /*
+ * Coarse increments of static-kernel values: for G (n_a, n_b, rows, cols) with
+ * element strides (s0, s1, s2, s3) in dtype_src,
+ *   inc(a, b, i, j) = (G(i+1, j+1) + G(i, j) - G(i+1, j) - G(i, j+1)) / 4^order,
+ * contiguous (n_a, n_b, rows - 1, cols - 1) in dtype_dst; the sum is rounded in
+ * dtype_src (the increments of sigpde/torch/kernel.py:13-21).  adjoint != 0: src
+ * is dL/dinc, contiguous, and dst receives dL/dG with the strides; rows and cols
+ * are those of G in both directions.  No workspace.
+ */
+SIGK_API int sigk_second_diff(int adjoint, const void *src, int64_t n_a, int64_t n_b, int64_t rows, int64_t cols,
+                              int64_t s0, int64_t s1, int64_t s2, int64_t s3, int dtype_src, int order, void *dst,
+                              int dtype_dst, sigk_stream_t stream);
+
+/*
  * Self norms k(x_b, x_b) in float64, NaN mapped to +inf.
  * First half of RobustSigPDE._norm_factors (sigpde/torch/kernel.py:181-183);
  * used when the normaliser is a user callable that the host applies.

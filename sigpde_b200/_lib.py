@@ -72,6 +72,7 @@ SIGNATURES = {
     "sigk_backward_inc_workspace_size": (_sz, [_i64, _i64, _i64, _int]),
     "sigk_backward_inc": (_int, [_vp, _i64, _i64, _i64, _i64, _i64, _i64, _int, _int, _vp, _vp, _vp, _vp, _i64, _i64,
                                  _i64, _vp, _sz, _vp]),
+    "sigk_second_diff": (_int, [_int, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _int, _int, _vp, _int, _vp]),
     "sigk_self_norms": (_int, [_vp, _i64, _i64, _i64, _int, _int, _dbl, _vp, _vp, _sz, _vp]),
     "sigk_normalize": (_int, [_vp, _i64, _i64, _i64, _int, _int, _dbl, _vp, _vp, _dbl, _int, _vp, _vp, _vp, _sz,
                               _vp]),

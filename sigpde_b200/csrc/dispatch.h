@@ -21,6 +21,7 @@ struct StaticIncParams;
 struct GradParams;
 struct RaggedDgemmParams;
 struct GradContractParams;
+struct SecondDiffParams;
 struct FusedTcParams;
 }
 struct CUtensorMap_st; // cuda.h
@@ -122,6 +123,9 @@ struct GradAuxFns {
                        const void *, const void *, double *, void *, int);
 };
 GradAuxFns get_grad_aux_kernels();
+// Second differences of static-kernel values and their adjoint (second_diff.cuh); wide: 64-bit element numbers
+using SecondDiffFn = void (*)(SecondDiffParams);
+SecondDiffFn get_second_diff_kernel(bool adjoint, bool src64, bool dst64, bool wide);
 // mat64: the increment matrix holds float64 (dgemm_inc_kernel) instead of float32 (tensor cores)
 // W: lanes a pair pipeline (32, or 16 for pairs of at most 16 R rows with R <= 8)
 StreamIncFn get_stream_inc_kernel(bool f64cells, int R, int O, bool mat64, int W = 32);

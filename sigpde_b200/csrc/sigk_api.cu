@@ -23,6 +23,7 @@
 #include "stream.cuh"
 #include "tc.cuh"
 #include "pair_wave.cuh"
+#include "second_diff.cuh"
 #include "dgemm_inc.cuh"
 #include "static_inc.cuh"
 #include "grad.cuh"
@@ -1919,6 +1920,29 @@ int sigk_backward_inc(const void *inc, int64_t npairs, int64_t nc_x, int64_t nc_
     if (((uintptr_t)workspace & 255) != 0) return fail(SIGK_EINVAL, "workspace must be 256-byte aligned");
     return run_backward_inc(g, inc, npairs, nc_x, nc_y, s0, s1, s2, dtype, order, scale_x, scale_y, grad_out,
                             grad_inc, g0, g1, g2, workspace, (cudaStream_t)stream);
+}
+
+int sigk_second_diff(int adjoint, const void *src, int64_t n_a, int64_t n_b, int64_t rows, int64_t cols, int64_t s0,
+                     int64_t s1, int64_t s2, int64_t s3, int dtype_src, int order, void *dst, int dtype_dst,
+                     sigk_stream_t stream)
+{
+    int st = check_common(dtype_src, SIGK_PREC_FP64, order);
+    if (st || (st = check_common(dtype_dst, SIGK_PREC_FP64, order))) return st;
+    if (n_a < 1 || n_b < 1 || rows < 2 || cols < 2)
+        return fail(SIGK_EINVAL, "need n_a, n_b >= 1 and rows, cols >= 2 (got %lld, %lld, %lld, %lld)", (long long)n_a,
+                    (long long)n_b, (long long)rows, (long long)cols);
+    if ((st = check_dev(src, "src", false)) || (st = check_dev(dst, "dst", false))) return st;
+    const int64_t total = adjoint ? n_a * n_b * rows * cols : n_a * n_b * (rows - 1) * (cols - 1);
+    int64_t blocks = (total + 255) / 256;
+    if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+    // 32-bit element numbers also step past the end by one grid
+    const bool wide = total + blocks * 256 > (int64_t)UINT32_MAX;
+    SecondDiffParams p{src, dst, n_a, n_b, rows, cols, s0, s1, s2, s3, std::ldexp(1.0, -2 * order)};
+    get_second_diff_kernel(adjoint != 0, dtype_src == SIGK_F64, dtype_dst == SIGK_F64, wide)
+        <<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(p);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "second-difference launch");
 }
 
 // Shared body of sigk_normalize, sigk_normalize_inc and sigk_self_norms

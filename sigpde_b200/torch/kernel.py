@@ -119,6 +119,76 @@ def gram_inner_product(x, y, static_kernel, dyadic_order):
     return ip / float(4 ** dyadic_order)
 
 
+def _takes_second_diff(G, dim):
+    """Whether sigk_second_diff reads G: a plain CUDA tensor of the engine's types
+    (a static kernel of the protocol may return any tensor; the rest goes through torch)."""
+    return (type(G) is torch.Tensor and G.is_cuda and G.layout is torch.strided and not G.is_neg() and
+            G.dtype in (torch.float32, torch.float64) and G.dim() == dim and G.numel() > 0 and
+            G.shape[-1] >= 2 and G.shape[-2] >= 2)
+
+
+def _dense(shape, strides) -> bool:
+    """Strides that number the elements of a dense tensor, in any order of its axes."""
+    n = 1
+    for st, sz in sorted((st, sz) for sz, st in zip(shape, strides) if sz > 1):
+        if st != n:
+            return False
+        n *= sz
+    return True
+
+
+def _second_diff(adjoint, src, shape, strides, order, dst):
+    """One sigk_second_diff launch; shape and strides are those of the static Gram."""
+    (na, nb), (s0, s1) = ((1, shape[0]), (0, strides[0])) if len(shape) == 3 else (shape[:2], strides[:2])
+    with torch.cuda.device(src.device):
+        _lib.call("sigk_second_diff", adjoint, _ptr(src), na, nb, shape[-2], shape[-1], s0, s1, strides[-2],
+                  strides[-1], _dtype_code(src), order, _ptr(dst), _dtype_code(dst), _stream())
+    return dst
+
+
+def _second_diff_forward(G, order, dtype):
+    inc = torch.empty((*G.shape[:-2], G.shape[-2] - 1, G.shape[-1] - 1), dtype=dtype, device=G.device)
+    return _second_diff(0, G, G.shape, G.stride(), order, inc)
+
+
+class _SecondDiff(torch.autograd.Function):
+    """Coarse increments from the static Gram G in one launch, and dL/dG in one
+    (linear in G, so nothing is saved)."""
+
+    @staticmethod
+    def forward(ctx, G, order, dtype):
+        ctx.meta = (tuple(G.shape), G.stride(), G.dtype, order)
+        return _second_diff_forward(G, order, dtype)
+
+    @staticmethod
+    def backward(ctx, grad_inc):
+        shape, strides, dtype, order = ctx.meta
+        grad_inc = grad_inc.detach().contiguous()
+        # laid out as G (a Gram's axes are permuted), so that the static kernel's own backward reads both alike
+        gG = (torch.empty_strided(shape, strides, dtype=dtype, device=grad_inc.device) if _dense(shape, strides)
+              else torch.empty(shape, dtype=dtype, device=grad_inc.device))
+        return _second_diff(1, grad_inc, shape, gG.stride(), order, gG), None, None
+
+
+def _increments(x, y, static_kernel, dyadic_order, pairwise, dtype):
+    """pairwise_inner_product / gram_inner_product in `dtype`, for the solver's own calls."""
+    G = static_kernel.pairwise(x, y) if pairwise else static_kernel.gram(x, y)
+    if _takes_second_diff(G, 3 if pairwise else 4):
+        if torch.is_grad_enabled() and G.requires_grad:
+            return _SecondDiff.apply(G, dyadic_order, dtype)
+        return _second_diff_forward(G, dyadic_order, dtype)
+    if pairwise:
+        G = G[:, 1:, 1:] + G[:, :-1, :-1] - G[:, 1:, :-1] - G[:, :-1, 1:]
+    else:
+        G = G[:, :, 1:, 1:] + G[:, :, :-1, :-1] - G[:, :, 1:, :-1] - G[:, :, :-1, 1:]
+    return (G / float(4 ** dyadic_order)).to(dtype)
+
+
+def _part(t, s0, s1):
+    """Rows [s0, s1) of t; t itself where that is all of it (no view, and no scatter in its backward)."""
+    return t if s0 == 0 and s1 == t.shape[0] else t[s0:s1]
+
+
 def log_normalizer(x):
     """Default robust normaliser f(s) = 2 - 1/(1 + log s) (sigpde/torch/kernel.py:23-24)."""
     return 2 - 1 / (1 + x.log())
@@ -230,11 +300,12 @@ def _generic_differentiable(solver, op, x, y, x_scale, y_scale, max_batch):
         sy = _broadcast_scale(ys, B, yv) if scaled else None
         parts = []
         for s0, s1 in _batches(B, max_batch):
-            inc = pairwise_inner_product(x[s0:s1], yv[s0:s1], solver.static_kernel, solver.dyadic_order).to(x.dtype)
+            inc = _increments(_part(x, s0, s1), _part(yv, s0, s1), solver.static_kernel, solver.dyadic_order, True,
+                              x.dtype)
             if scaled:  # in torch, so that autograd reaches the scales (sigpde/cuda_pairwise_kernels.py:61,69)
                 inc = inc * (sx[s0:s1] * sy[s0:s1])[:, None, None]
             parts.append(_IncSolve.apply(inc, None, None, solver))
-        return torch.cat(parts)
+        return parts[0] if len(parts) == 1 else torch.cat(parts)
     sym = y is None
     yv = x if sym else y
     _check_paths(yv, "y")
@@ -252,7 +323,8 @@ def _generic_differentiable(solver, op, x, y, x_scale, y_scale, max_batch):
             if sym and y0 > x0:  # upper tiles are the transposed lower ones
                 row.append(None)
                 continue
-            inc = gram_inner_product(x[x0:x1], yv[y0:y1], solver.static_kernel, solver.dyadic_order).to(x.dtype)
+            inc = _increments(_part(x, x0, x1), _part(yv, y0, y1), solver.static_kernel, solver.dyadic_order, False,
+                              x.dtype)
             if scaled:  # in torch, so that autograd reaches the scales (sigpde/cuda_gram_kernels.py:52,60)
                 inc = inc * (sx[x0:x1][:, None] * sy[y0:y1][None, :])[:, :, None, None]
             tx, ty, ncx, ncy = inc.shape
@@ -361,7 +433,7 @@ class SigPDE:
                           prec, _ptr(ws), nws, _stream())
                 return result
             for s0, s1 in _batches(B, max_batch):
-                inc = pairwise_inner_product(x[s0:s1], y[s0:s1], self.static_kernel, self.dyadic_order)
+                inc = _increments(x[s0:s1], y[s0:s1], self.static_kernel, self.dyadic_order, True, x.dtype)
                 self._solve_pairwise_inc(inc, None if sx is None else sx[s0:s1],
                                          None if sy is None else sy[s0:s1], result[s0:s1])
         return result
@@ -418,7 +490,7 @@ class SigPDE:
             tile = math.ceil(math.sqrt(max_batch))  # sigpde/torch/kernel.py:68
             for y0, y1 in _batches(Ny, tile):
                 for x0, x1 in _batches(Nx, tile):
-                    inc = gram_inner_product(x[x0:x1], y[y0:y1], self.static_kernel, self.dyadic_order)
+                    inc = _increments(x[x0:x1], y[y0:y1], self.static_kernel, self.dyadic_order, False, x.dtype)
                     self._solve_gram_inc(inc, None if sx is None else sx[x0:x1], None if sy is None else sy[y0:y1],
                                          result, x0, y0, False)
         return result
@@ -448,7 +520,7 @@ class SigPDE:
                 for x0, x1 in _batches(N, tile):
                     if x0 < y0:
                         continue  # upper tiles are mirrored from the lower ones
-                    inc = gram_inner_product(x[x0:x1], x[y0:y1], self.static_kernel, self.dyadic_order)
+                    inc = _increments(x[x0:x1], x[y0:y1], self.static_kernel, self.dyadic_order, False, x.dtype)
                     self._solve_gram_inc(inc, None if sx is None else sx[x0:x1], None if sx is None else sx[y0:y1],
                                          result, x0, y0, x0 == y0)
                     if x0 != y0:
@@ -516,7 +588,7 @@ class _RobustLambda(torch.autograd.Function):
         solver = SigPDE(rk.static_kernel, rk.dyadic_order, "fp64")
         with torch.enable_grad():
             xg = x.detach().requires_grad_()
-            inc = pairwise_inner_product(xg, xg, rk.static_kernel, rk.dyadic_order).to(torch.float64)
+            inc = _increments(xg, xg, rk.static_kernel, rk.dyadic_order, True, torch.float64)
             lv = lam.detach().to(torch.float64).requires_grad_()
             k_lam = _IncSolve.apply(inc * (lv * lv)[:, None, None], None, None, solver)
             k_0 = _IncSolve.apply(inc, None, None, solver)
@@ -577,7 +649,7 @@ class RobustSigPDE:
                 return lam, iters
             # generic static kernel: torch builds the self-increments, in float64
             for s0, s1 in _batches(N, max_batch):
-                inc = pairwise_inner_product(x[s0:s1], x[s0:s1], self.static_kernel, order).to(torch.float64)
+                inc = _increments(x[s0:s1], x[s0:s1], self.static_kernel, order, True, torch.float64)
                 nb, nc, _ = inc.shape
                 knorm = torch.empty(nb, device=x.device, dtype=torch.float64)
                 ws, nws = _workspace(_lib.SIGK_OP_NORMALIZE, nb, nb, nc + 1, nc + 1, 0, order, _lib.SIGK_F64,

@@ -287,3 +287,33 @@ def test_backward_refusals(sig):
     g = sig.RobustSigPDE(sig.kernels.LinearKernel(), 1).gram(x, None, cuda([0.5, 0.9]))
     g.sum().backward()
     assert x.grad is not None
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 2), (3, 2, 9), (5, 33, 17), (2, 3, 2, 5), (4, 3, 18, 11)])
+@pytest.mark.parametrize("types", [(torch.float32, torch.float32), (torch.float32, torch.float64),
+                                   (torch.float64, torch.float32), (torch.float64, torch.float64)])
+def test_second_difference_kernel(sig, shape, types):
+    """Increments from static-kernel values and their adjoint against the torch expressions.  The
+    values are small integers over a power of two, so every order of summation is exact: no tolerance."""
+    import sigpde_b200.torch.kernel as kmod
+    pairwise, order = len(shape) == 3, 2
+    g = torch.Generator().manual_seed(sum(shape))
+    base = torch.randint(-64, 65, shape, generator=g).to(types[0]).cuda()
+    layouts = [base, base.transpose(-1, -2).contiguous().transpose(-1, -2), base[:, :1].expand(shape)]
+    if not pairwise:  # a Gram: (A, M, B, N) permuted
+        layouts.append(base.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3))
+
+    for G in layouts:
+        class Given:
+            def pairwise(self, X, Y):
+                return X
+            gram = pairwise
+        fn = kmod.pairwise_inner_product if pairwise else kmod.gram_inner_product
+        Ga, Gb = G.detach().requires_grad_(), G.detach().requires_grad_()
+        want = fn(Ga, None, Given(), order).to(types[1])
+        got = kmod._increments(Gb, None, Given(), order, pairwise, types[1])
+        assert got.grad_fn.name().startswith("_SecondDiff") and got.dtype == types[1] and torch.equal(got, want)
+        assert torch.equal(kmod._increments(G, None, Given(), order, pairwise, types[1]), want)
+        w = torch.randint(-16, 17, tuple(want.shape), generator=g).to(types[1]).cuda()
+        (wa,), (wb,) = torch.autograd.grad(want, Ga, w), torch.autograd.grad(got, Gb, w)
+        assert wb.dtype == types[0] and torch.equal(wa, wb)
