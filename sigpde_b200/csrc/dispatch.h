@@ -21,6 +21,7 @@ struct StaticIncParams;
 struct GradParams;
 struct RaggedDgemmParams;
 struct GradContractParams;
+struct GradStageParams;
 struct SecondDiffParams;
 struct FusedTcParams;
 }
@@ -113,12 +114,14 @@ struct GradAuxFns {
     void (*pair_inc)(const double *, const double *, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, double *);
     void (*gx)(GradContractParams);
     void (*gy)(GradContractParams);
-    void (*reduce)(const double *, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, double *);
-    void (*points)(const double *, int64_t, int64_t, int64_t, double, const void *, int, void *);
+    void (*points)(const double *, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, double, const void *,
+                   int, void *);
+    void (*stage32)(GradStageParams); // float32 points
+    void (*stage64)(GradStageParams);
     void (*rows)(const double *, int64_t, int64_t, int64_t, int64_t, int, double *);
     void (*gx_gram)(GradContractParams);
     void (*gy_gram)(GradContractParams);
-    void (*gy_reduce)(const double *, int64_t, int64_t, double *);
+    void (*gy_reduce)(const double *, int64_t, int64_t, int, double *);
     void (*inc_blocks)(const void *, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t,
                        const void *, const void *, double *, void *, int);
 };

@@ -652,7 +652,7 @@ struct GradContractParams {
     double *part;          // gx: [slice][nrows_m][d], gy of a Gram: [range of m][ncols_n][d] partial sums
     int64_t slice;         // gx: columns per slice
     int64_t mslice;        // gy of a Gram: m per range (a multiple of kGyTile)
-    double *gdy;           // gy: (ny, ncy, d) accumulated (+=) over chunks
+    double *gdy;           // gy of pairs: (ny, ncy, d)
     int64_t x0;
 };
 
@@ -802,7 +802,7 @@ __global__ void grad_gy_kernel(GradContractParams p)
             double v = acc[k];
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFullMask, v, off);
-            if (lane == 0 && k0 + k < p.d) p.gdy[yrow * p.d + k0 + k] += v;
+            if (lane == 0 && k0 + k < p.d) p.gdy[yrow * p.d + k0 + k] = v;
         }
     }
 }
@@ -889,52 +889,101 @@ __global__ void __launch_bounds__(kGyWarps * 32, 2) grad_gy_gram_kernel(GradCont
     }
 }
 
-// gdy[e] += sum over the ranges of m of part[range][e], in order.
+// gdy[e] (first: =, else +=) the sum over the ranges of m of part[range][e], in order: Grams of several chunks.
 template <int V = 0> // instantiated once, in kernels_grad.cu
-__global__ void grad_gy_reduce_kernel(const double *part, int64_t nranges, int64_t total, double *gdy)
+__global__ void grad_gy_reduce_kernel(const double *part, int64_t nranges, int64_t total, int first, double *gdy)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
     double s = 0.0;
     for (int64_t i = 0; i < nranges; ++i) s += part[i * total + e];
-    gdy[e] += s;
+    gdy[e] = first ? s : gdy[e] + s;
 }
 
-// gdx[(x0 + il) * ncx + ci][k] = sum over slices of part (rows ci < ncx).
+// Gradient at the points of paths path0, ..: g[path][t][k] = scale(path) * (gd[t-1][k] - gd[t][k]), gd of the
+// path's coarse differences, each the sum over nparts partial sums in order, in the output dtype.  A path has
+// `pitch` rows of d values in a partial sum, which is `stride` values long.  The sums are formed here, twice a
+// cell, rather than by a launch before this one: on a small batch the launch costs more.
 template <int V = 0> // instantiated once, in kernels_grad.cu
-__global__ void grad_reduce_kernel(const double *part, int64_t nslices, int64_t nrows_m, int64_t rows_x, int64_t ncx,
-                                   int64_t d, int64_t x0, double *gdx)
-{
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nrows_m * d) return;
-    const int64_t mm = e / d, k = e - mm * d;
-    const int64_t il = mm / rows_x, ci = mm - il * rows_x;
-    if (ci >= ncx) return;
-    double s = 0.0;
-    for (int64_t sl = 0; sl < nslices; ++sl) s += part[(sl * nrows_m + mm) * d + k];
-    gdx[((x0 + il) * ncx + ci) * d + k] = s;
-}
-
-// grad at the points: g[path][t][k] = scale(path) * (gd[t-1][k] - gd[t][k]),
-// gd of the path's coarse differences (ncells = len - 1), in the output dtype.
-template <int V = 0> // instantiated once, in kernels_grad.cu
-__global__ void grad_points_kernel(const double *gd, int64_t npaths, int64_t len, int64_t d, double f,
-                                   const void *sc, int in64, void *out)
+__global__ void grad_points_kernel(const double *part, int64_t nparts, int64_t stride, int64_t pitch, int64_t path0,
+                                   int64_t npaths, int64_t len, int64_t d, double f, const void *sc, int in64,
+                                   void *out)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= npaths * len * d) return;
     const int64_t pth = e / (len * d), r = e - pth * len * d, t = r / d, k = r - t * d;
     const int64_t nc = len - 1;
-    const double *g = gd + pth * nc * d;
-    const double a = t >= 1 ? g[(t - 1) * d + k] : 0.0;
-    const double b = t < nc ? g[t * d + k] : 0.0;
-    const double s = sc ? (in64 ? reinterpret_cast<const double *>(sc)[pth]
-                                : (double)reinterpret_cast<const float *>(sc)[pth]) : 1.0;
+    const double *g = part + (pth * pitch + t) * d + k;
+    double a = 0.0, b = 0.0;
+    for (int64_t i = 0; i < nparts; ++i) {
+        if (t >= 1) a += g[i * stride - d];
+        if (t < nc) b += g[i * stride];
+    }
+    const double s = sc ? (in64 ? reinterpret_cast<const double *>(sc)[path0 + pth]
+                                : (double)reinterpret_cast<const float *>(sc)[path0 + pth]) : 1.0;
     const double v = (a - b) * f * s;
     if (in64)
-        reinterpret_cast<double *>(out)[e] = v;
+        reinterpret_cast<double *>(out)[path0 * len * d + e] = v;
     else
-        reinterpret_cast<float *>(out)[e] = (float)v;
+        reinterpret_cast<float *>(out)[path0 * len * d + e] = (float)v;
+}
+
+// All layouts of the scaled differences that a backward pass reads, straight from the points in one launch: x and y
+// dimension-major per path (as delta_kernel), y by cells, and, where the pairs are one chunk, x as grad_rows_kernel.
+struct GradStageParams {
+    const void *x, *y, *sx, *sy;
+    double fx;                    // static scale * 4^-order, on the x side
+    int64_t nx, ny, ncx, ncy, d;
+    double *dx, *dy, *dyt, *dxt;  // dxt may be null
+    int64_t rows_x;
+    int dim_major;                // dxt: [k][path * rows_x + r], else [path * rows_x + r][k]
+};
+
+template <typename TIN>
+__device__ __forceinline__ double grad_diff(const void *x_, const void *s_, double f, int64_t nc, int64_t d,
+                                            int64_t path, int64_t c, int64_t k)
+{
+    const TIN *x = reinterpret_cast<const TIN *>(x_) + (path * (nc + 1) + c) * d + k;
+    const double g = s_ ? f * (double)reinterpret_cast<const TIN *>(s_)[path] : f;
+    return ((double)x[d] - (double)x[0]) * g;
+}
+
+template <typename TIN>
+__global__ void grad_stage_kernel(GradStageParams p)
+{
+    const int64_t tx = p.nx * p.ncx * p.d, ty = p.ny * p.ncy * p.d, txt = p.dxt ? p.nx * p.rows_x * p.d : 0;
+    const int64_t total = tx + 2 * ty + txt;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        int64_t e = i;
+        if (e < tx) {
+            const int64_t row = e / p.ncx, c = e - row * p.ncx, path = row / p.d, k = row - path * p.d;
+            p.dx[e] = grad_diff<TIN>(p.x, p.sx, p.fx, p.ncx, p.d, path, c, k);
+            continue;
+        }
+        e -= tx;
+        if (e < ty) {
+            const int64_t row = e / p.ncy, c = e - row * p.ncy, path = row / p.d, k = row - path * p.d;
+            p.dy[e] = grad_diff<TIN>(p.y, p.sy, 1.0, p.ncy, p.d, path, c, k);
+            continue;
+        }
+        e -= ty;
+        if (e < ty) {
+            const int64_t row = e / p.d, k = e - row * p.d, path = row / p.ncy, c = row - path * p.ncy;
+            p.dyt[e] = grad_diff<TIN>(p.y, p.sy, 1.0, p.ncy, p.d, path, c, k);
+            continue;
+        }
+        e -= ty;
+        int64_t row, k;
+        if (p.dim_major) {
+            k = e / (p.nx * p.rows_x);
+            row = e - k * p.nx * p.rows_x;
+        } else {
+            row = e / p.d;
+            k = e - row * p.d;
+        }
+        const int64_t path = row / p.rows_x, c = row - path * p.rows_x;
+        p.dxt[e] = c < p.ncx ? grad_diff<TIN>(p.x, p.sx, p.fx, p.ncx, p.d, path, c, k) : 0.0;
+    }
 }
 
 } // namespace sigk

@@ -50,8 +50,9 @@ GradFns get_grad_kernels(int R, int O, bool wide) { return wide ? grad_by_r<2>(R
 
 GradAuxFns get_grad_aux_kernels()
 {
-    return {grad_pair_inc_kernel<>, grad_gx_kernel<>, grad_gy_kernel<>, grad_reduce_kernel<>, grad_points_kernel<>,
-            grad_rows_kernel<>, grad_gx_gram_kernel<>, grad_gy_gram_kernel<>, grad_gy_reduce_kernel<>, grad_inc_blocks_kernel<>};
+    return {grad_pair_inc_kernel<>, grad_gx_kernel<>, grad_gy_kernel<>, grad_points_kernel<>,
+            grad_stage_kernel<float>, grad_stage_kernel<double>, grad_rows_kernel<>, grad_gx_gram_kernel<>,
+            grad_gy_gram_kernel<>, grad_gy_reduce_kernel<>, grad_inc_blocks_kernel<>};
 }
 
 } // namespace sigk

@@ -1017,7 +1017,7 @@ struct GradPlan {
     int R = 0, O = 0, nb = 0, nsteps = 0, period = 0;
     bool wide = false;
     int64_t rows_x = 0, chunk = 0, nchunks = 0, per_warp = 0, slice = 0, nslices = 0, mslice = 0, bnd_stride = 0;
-    size_t dx_off = 0, dy_off = 0, gdx_off = 0, gdy_off = 0, part_off = 0, mat_off = 0, rec_off = 0, bnd_off = 0,
+    size_t dx_off = 0, dy_off = 0, gdy_off = 0, part_off = 0, mat_off = 0, rec_off = 0, bnd_off = 0,
            xt_off = 0, yt_off = 0, ws_bytes = 0;
 };
 
@@ -1110,8 +1110,6 @@ GradPlan make_grad_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy
     off += align256((size_t)nx * d * ncx * sizeof(double));
     g.dy_off = off;
     off += align256((size_t)ny_paths * d * ncy * sizeof(double));
-    g.gdx_off = off;
-    off += align256((size_t)nx * ncx * d * sizeof(double));
     g.gdy_off = off;
     off += align256((size_t)ny_paths * ncy * d * sizeof(double));
     // y contraction of a Gram: ranges of m, enough of them for several waves of CTAs, at least 4 tiles each
@@ -1174,27 +1172,12 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
     unsigned char *wsb = reinterpret_cast<unsigned char *>(ws);
     double *dx = reinterpret_cast<double *>(wsb + g.dx_off);
     double *dy = reinterpret_cast<double *>(wsb + g.dy_off);
-    double *gdx = reinterpret_cast<double *>(wsb + g.gdx_off);
     double *gdy = reinterpret_cast<double *>(wsb + g.gdy_off);
     double *part = reinterpret_cast<double *>(wsb + g.part_off);
     double *mat = reinterpret_cast<double *>(wsb + g.mat_off);
     const int64_t ny_paths = op == kOpPairwise ? nx : ny;
-    cudaError_t e = cudaMemsetAsync(gdy, 0, (size_t)ny_paths * ncy * d * sizeof(double), stream);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
-    DeltaFn delta = get_delta_kernel(true, in64);
-    auto run_delta = [&](const void *src, int64_t npaths, int64_t len, double f, const void *sc, double *dst) -> int {
-        const int64_t total = npaths * (len - 1) * d;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-        delta<<<(unsigned)blocks, 256, 0, stream>>>(src, npaths, len, d, d, f, sc, dst);
-        count_launch();
-        cudaError_t e2 = cudaGetLastError();
-        return e2 == cudaSuccess ? SIGK_OK : cuda_fail(e2, "delta kernel launch");
-    };
     const double fs = static_scale * std::ldexp(1.0, -2 * order);
     int st;
-    if ((st = run_delta(x, nx, lx, fs, sx, dx))) return st;
-    if ((st = run_delta(y, ny_paths, ly, 1.0, sy, dy))) return st;
     double *dxt = reinterpret_cast<double *>(wsb + g.xt_off);
     double *dyt = reinterpret_cast<double *>(wsb + g.yt_off);
     auto run_rows = [&](const double *src, int64_t npaths, int64_t nc, int64_t rows, bool dim_major, double *dst) -> int {
@@ -1206,12 +1189,43 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
         cudaError_t e2 = cudaGetLastError();
         return e2 == cudaSuccess ? SIGK_OK : cuda_fail(e2, "row-layout launch");
     };
-    if ((st = run_rows(dy, ny_paths, ncy, ncy, false, dyt))) return st;
     GradAuxFns aux = get_grad_aux_kernels();
     auto launched = [&](const char *what) -> int {
         count_launch();
         cudaError_t e2 = cudaGetLastError();
         return e2 == cudaSuccess ? SIGK_OK : cuda_fail(e2, what);
+    };
+    const bool whole = g.nchunks == 1;
+    {
+        GradStageParams q{};
+        q.x = x;
+        q.y = y;
+        q.sx = sx;
+        q.sy = sy;
+        q.fx = fs;
+        q.nx = nx;
+        q.ny = ny_paths;
+        q.ncx = ncx;
+        q.ncy = ncy;
+        q.d = d;
+        q.dx = dx;
+        q.dy = dy;
+        q.dyt = dyt;
+        q.dxt = whole ? dxt : nullptr;
+        q.rows_x = g.rows_x;
+        q.dim_major = op != kOpPairwise;
+        const int64_t total = d * (nx * ncx + 2 * ny_paths * ncy + (whole ? nx * g.rows_x : 0));
+        int64_t blocks = (total + 255) / 256;
+        if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+        (in64 ? aux.stage64 : aux.stage32)<<<(unsigned)blocks, 256, 0, stream>>>(q);
+        if ((st = launched("difference launch"))) return st;
+    }
+    auto points = [&](const double *src, int64_t nparts, int64_t stride, int64_t pitch, int64_t p0, int64_t np,
+                      int64_t len, double f, const void *sc, void *out, const char *what) -> int {
+        const int64_t tot = np * len * d;
+        aux.points<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(src, nparts, stride, pitch, p0, np, len, d, f, sc,
+                                                                     in64, out);
+        return launched(what);
     };
     for (int64_t c = 0; c < g.nchunks; ++c) {
         const int64_t i0 = c * g.chunk, i1 = (i0 + g.chunk < nx) ? i0 + g.chunk : nx, nxc = i1 - i0;
@@ -1240,7 +1254,7 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
             gp.ld = ld;
             if ((st = launch_dgemm_inc(gp, stream))) return st;
         }
-        if ((st = run_rows(dx + i0 * d * ncx, nxc, ncx, g.rows_x, op != kOpPairwise, dxt))) return st;
+        if (!whole && (st = run_rows(dx + i0 * d * ncx, nxc, ncx, g.rows_x, op != kOpPairwise, dxt))) return st;
         GradParams gp{};
         gp.op = op;
         gp.mat = mat;
@@ -1253,7 +1267,7 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
         gp.in64 = in64;
         gp.x0 = i0;
         if ((st = launch_grad_wavefronts(g, gp, wsb, stream))) return st;
-        // contractions: x side (partial slices, then their ordered sum) and y side
+        // contractions: partial sums of the x side, then of the y side
         GradContractParams cp{};
         cp.op = op;
         cp.mat = mat;
@@ -1280,10 +1294,8 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
                 aux.gx_gram<<<dim3((unsigned)((cp.nrows_m + 2 * kGxThreads - 1) / (2 * kGxThreads)), (unsigned)nsl),
                               kGxThreads, 0, stream>>>(cp);
             if ((st = launched("x contraction launch"))) return st;
-            const int64_t tot = cp.nrows_m * d;
-            aux.reduce<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(part, nsl, cp.nrows_m, g.rows_x, ncx, d, i0,
-                                                                        gdx);
-            if ((st = launched("x reduction launch"))) return st;
+            if ((st = points(part, nsl, cp.nrows_m * d, g.rows_x, i0, nxc, lx, fs, sx, gx, "x point-gradient launch")))
+                return st;
         }
         if (gy) {
             if (op == kOpPairwise) {
@@ -1295,21 +1307,18 @@ int run_backward(const GradPlan &g, int op, const void *x, const void *y, int64_
                               stream>>>(cp);
                 if ((st = launched("y contraction launch"))) return st;
                 const int64_t tot = ny * ncy * d;
-                aux.gy_reduce<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(part, ranges, tot, gdy);
+                if (whole) {
+                    if ((st = points(part, ranges, tot, ncy, 0, ny, ly, 1.0, sy, gy, "y point-gradient launch")))
+                        return st;
+                    continue;
+                }
+                aux.gy_reduce<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(part, ranges, tot, c == 0, gdy);
             }
             if ((st = launched("y contraction launch"))) return st;
         }
     }
-    if (gx) {
-        const int64_t tot = nx * lx * d;
-        aux.points<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(gdx, nx, lx, d, fs, sx, in64, gx);
-        if ((st = launched("x point-gradient launch"))) return st;
-    }
-    if (gy) {
-        const int64_t tot = ny_paths * ly * d;
-        aux.points<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(gdy, ny_paths, ly, d, 1.0, sy, in64, gy);
-        if ((st = launched("y point-gradient launch"))) return st;
-    }
+    if (gy && (op == kOpPairwise || !whole))
+        return points(gdy, 1, 0, ncy, 0, ny_paths, ly, 1.0, sy, gy, "y point-gradient launch");
     return SIGK_OK;
 }
 
