@@ -11,6 +11,7 @@ struct PairParams;
 struct NormParams;
 struct PairWaveParams;
 struct StreamParams;
+struct DeltaParams;
 struct RaggedParams;
 struct StreamIncParams;
 struct TcImageParams;
@@ -41,7 +42,7 @@ using TcRaggedImageFn = void (*)(TcRaggedImageParams);
 using DgemmIncFn = void (*)(DgemmIncParams);
 using StaticIncFn = void (*)(StaticIncParams);
 using TcGemmFn = void (*)(TcGemmParams, CUtensorMap_st);
-using DeltaFn = void (*)(const void *, int64_t, int64_t, int64_t, int64_t, double, const void *, void *);
+using DeltaFn = void (*)(DeltaParams);
 
 // f64cells: float64 cells (SIGK_PREC_FP64) vs float32; in64: float64 inputs;
 // R in {2,4,8,16} rows per lane; O = min(order, 4).
@@ -72,7 +73,7 @@ StreamFn get_stream_reg_kernel_f32x2(int R, int O, int D);
 // float64 cells, two Gram entries of one x path per lane (kOpGram only)
 StreamFn get_stream_reg_kernel_f64x2(int R, int O, int D);
 StreamFn get_stream_smem_kernel(bool f64cells, int R, int O);
-DeltaFn get_delta_kernel(bool f64cells, bool in64);
+DeltaFn get_delta_kernel(bool grouped, bool f64cells, bool in64); // grouped: float64 dimensions in groups of 2
 // mat: increments from a precomputed matrix (tensor-core modes) instead of differences
 // mat64: the increment matrix holds float64 (fp64 cells with a plan) instead of float32
 RaggedFn get_ragged_kernel(bool f64cells, bool in64, bool mat, bool mat64 = false);

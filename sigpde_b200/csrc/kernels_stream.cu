@@ -37,9 +37,10 @@ StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D)
     return f64cells ? get_stream_reg_kernel_f64(R, O, D) : get_stream_reg_kernel_f32(R, O, D);
 }
 
-DeltaFn get_delta_kernel(bool f64cells, bool in64)
+DeltaFn get_delta_kernel(bool grouped, bool f64cells, bool in64)
 {
-    if (f64cells) return in64 ? delta_kernel<double, double> : delta_kernel<double, float>;
-    return in64 ? delta_kernel<float, double> : delta_kernel<float, float>;
+    if (f64cells && grouped) return in64 ? delta_kernel<double, double, 2> : delta_kernel<double, float, 2>;
+    if (f64cells) return in64 ? delta_kernel<double, double, 1> : delta_kernel<double, float, 1>;
+    return in64 ? delta_kernel<float, double, 1> : delta_kernel<float, float, 1>;
 }
 } // namespace sigk

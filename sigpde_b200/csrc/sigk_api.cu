@@ -886,6 +886,43 @@ TcPlan make_static_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy
     return mat64_layout(op, nx, ny, ncx, ncy, d, order, false, es);
 }
 
+// Scaled differences of one or both sides of a call (delta_kernel).
+int launch_delta(DeltaParams &p, bool grouped, bool f64cells, bool in64, cudaStream_t stream)
+{
+    const int64_t paths = p.side[0].npaths + p.side[1].npaths, most = (int64_t)sm_count() * 64;
+    const int64_t blocks = paths < most ? paths : most;
+    int64_t longest = 0;
+    for (const DeltaSide &q : p.side)
+        if (q.npaths > 0 && q.len - 1 > longest) longest = q.len - 1;
+    int64_t tiles = (longest + kDeltaCols - 1) / kDeltaCols;
+    if (tiles > 64) tiles = 64;
+    p.pitch = (p.dp < kDeltaDims ? (int)p.dp : kDeltaDims) | 1;
+    const int64_t cols = longest < kDeltaCols ? longest : kDeltaCols;
+    const size_t smem = (size_t)(cols + 1) * p.pitch * (f64cells ? sizeof(double) : sizeof(float));
+    get_delta_kernel(grouped, f64cells, in64)<<<dim3((unsigned)blocks, (unsigned)tiles), kDeltaThreads, smem, stream>>>(p);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "delta kernel launch");
+}
+
+// Both sides of run_pairs: static scale * 4^-order (f) and scale_x on x, scale_y on y.  A symmetric Gram takes both
+// from x, scale_x on each side: f goes on the row side only, so a second buffer is needed unless f == 1 (dy == dx).
+int launch_deltas(int op, const void *x, const void *y, int64_t nx, int64_t ny, int64_t lx, int64_t ly, int64_t d,
+                  int64_t dp, double f, const void *sx, const void *sy, bool grouped, bool f64cells, bool in64, void *dx,
+                  void *&dy, cudaStream_t stream)
+{
+    DeltaParams p{};
+    p.d = d;
+    p.dp = dp;
+    p.side[0] = DeltaSide{x, sx, dx, nx, lx, f};
+    p.side[1] = op == kOpGramSym ? DeltaSide{x, sx, dy, nx, lx, 1.0} : DeltaSide{y, sy, dy, ny, ly, 1.0};
+    if (op == kOpGramSym && f == 1.0) {
+        p.side[1].npaths = 0;
+        dy = dx;
+    }
+    return launch_delta(p, grouped, f64cells, in64, stream);
+}
+
 int run_pairs_mat64(const TcPlan &t, int op, const void *x, const void *y, int64_t nx, int64_t ny, int64_t lx,
                     int64_t ly, int64_t d, int dtype, int order, double static_scale, const void *sx, const void *sy,
                     void *out, int64_t out_ld, int precision, void *ws, cudaStream_t stream)
@@ -900,29 +937,12 @@ int run_pairs_mat64(const TcPlan &t, int op, const void *x, const void *y, int64
     double *mat = reinterpret_cast<double *>(wsb + t.ct_off);
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(unsigned), stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
-    // scaled differences, as the fused path: static scale * 4^-order * scale_x on x, scale_y on y
-    // (the symmetric Gram: both from x, scale_x on each side)
-    DeltaFn delta = get_delta_kernel(true, in64);
-    auto run_delta = [&](const void *src, int64_t npaths, int64_t len, double f, const void *sc, double *dst) -> int {
-        const int64_t total = npaths * (len - 1) * d;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-        delta<<<(unsigned)blocks, 256, 0, stream>>>(src, npaths, len, d, d, f, sc, dst);
-        count_launch();
-        cudaError_t e2 = cudaGetLastError();
-        return e2 == cudaSuccess ? SIGK_OK : cuda_fail(e2, "delta kernel launch");
-    };
-    const double fs = static_scale * std::ldexp(1.0, -2 * order);
     const bool sym = op == kOpGramSym;
-    if ((st = run_delta(x, nx, lx, fs, sx, dx))) return st;
-    if (sym) {
-        if (fs == 1.0)
-            dy = dx;
-        else if ((st = run_delta(x, nx, lx, 1.0, sx, dy)))
-            return st;
-    } else if ((st = run_delta(y, ny, ly, 1.0, sy, dy))) {
+    void *dyv = dy;
+    if ((st = launch_deltas(op, x, y, nx, ny, lx, ly, d, d, static_scale * std::ldexp(1.0, -2 * order), sx, sy, false,
+                            true, in64, dx, dyv, stream)))
         return st;
-    }
+    dy = reinterpret_cast<double *>(dyv);
     for (int64_t c = 0; c < t.nchunks; ++c) {
         const int64_t i0 = c * t.chunk, i1 = (i0 + t.chunk < nx) ? i0 + t.chunk : nx, nxc = i1 - i0;
         DgemmIncParams gp{};
@@ -1533,35 +1553,11 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
         unsigned char *wsb = reinterpret_cast<unsigned char *>(ws);
         void *dx = wsb + pl.dx_off;
         void *dy = wsb + pl.dy_off;
-        DeltaFn delta = get_delta_kernel(f64, in64);
         const int nsm = sm_count();
         const int64_t dp = pl.stream && pl.D ? pl.D : d;
-        auto run_delta = [&](const void *src, int64_t npaths, int64_t len, double f, const void *sc,
-                             void *dst) -> int {
-            const int64_t total = npaths * (len - 1) * dp;
-            int64_t blocks = (total + 255) / 256;
-            if (blocks > (int64_t)nsm * 8) blocks = (int64_t)nsm * 8;
-            delta<<<(unsigned)blocks, 256, 0, stream>>>(src, npaths, len, d, dp, f, sc, dst);
-            count_launch();
-            cudaError_t e = cudaGetLastError();
-            return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "delta kernel launch");
-        };
-        // static scale * 4^-order and scale_x go into dX, scale_y into dY; the
-        // symmetric Gram reads one buffer for both sides, scaled by scale_x
-        const double fs = static_scale * std::ldexp(1.0, -2 * order);
-        if (op == kOpGramSym) {
-            // f goes on the row side only, so a second buffer is needed unless f == 1
-            if (fs == 1.0) {
-                if ((st = run_delta(x, nx, lx, 1.0, sx, dx))) return st;
-                dy = dx;
-            } else {
-                if ((st = run_delta(x, nx, lx, fs, sx, dx))) return st;
-                if ((st = run_delta(x, nx, lx, 1.0, sx, dy))) return st;
-            }
-        } else {
-            if ((st = run_delta(x, nx, lx, fs, sx, dx))) return st;
-            if ((st = run_delta(y, ny, ly, 1.0, sy, dy))) return st;
-        }
+        if ((st = launch_deltas(op, x, y, nx, ny, lx, ly, d, dp, static_scale * std::ldexp(1.0, -2 * order), sx, sy,
+                                pl.stream && pl.D, f64, in64, dx, dy, stream)))
+            return st;
 
         if (!pl.stream) { // one pair per warp, any number of bands
             PairParams p{};
@@ -1604,10 +1600,9 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
         sp.nitems = nitems;
         // float32 cells with register dx: two pairs per lane on paired instructions
         const bool paired = !f64 && pl.D && nitems >= 2 && !env_flag("SIGK_NO_PAIRED_F32");
+        const bool dual_ok = f64 && pl.D && op == kOpGram && ny >= 2 && !env_flag("SIGK_NO_DUAL_F64");
         // float64 cells of a Gram with register dx: two entries of one x path per lane
-        StreamFn dual_fn = (f64 && pl.D && op == kOpGram && ny >= 2 && !env_flag("SIGK_NO_DUAL_F64"))
-                               ? get_stream_reg_kernel_f64x2(pl.R, pl.O, pl.D)
-                               : nullptr;
+        StreamFn dual_fn = dual_ok ? get_stream_reg_kernel_f64x2(pl.R, pl.O, pl.D) : nullptr;
         const bool dual = dual_fn != nullptr;
         StreamFn fn = paired  ? get_stream_reg_kernel_f32x2(pl.R, pl.O, pl.D)
                       : dual  ? dual_fn
@@ -1989,14 +1984,10 @@ static int normalize_impl(const void *x, const void *inc, int64_t n, int64_t nc,
     double *dx = nullptr;
     if (!from_inc) { // unscaled float64 differences, dimension-major (the kernel applies the scale)
         dx = reinterpret_cast<double *>(wsb + q.dx_off);
-        DeltaFn delta = get_delta_kernel(true, dtype == SIGK_F64);
-        const int64_t total = n * nc * d;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-        delta<<<(unsigned)blocks, 256, 0, stream>>>(x, n, nc + 1, d, d, 1.0, nullptr, dx);
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(e, "delta kernel launch");
+        DeltaParams dq{};
+        dq.d = dq.dp = d;
+        dq.side[0] = DeltaSide{x, nullptr, dx, n, nc + 1, 1.0};
+        if (int e = launch_delta(dq, false, true, dtype == SIGK_F64, stream)) return e;
     }
     NormParams p{};
     p.n = n;

@@ -30,38 +30,78 @@
 
 namespace sigk {
 
-// dx[p][k][c] = T(x[p][c+1][k]) - T(x[p][c][k]) for all paths p, stored
-// dimension-major: the lanes of a warp read neighbouring coarse columns c of
-// one dimension k in the same instruction (lane l is one column behind lane
-// l-1), so a load touches 2 cache lines instead of 16.  Dimensions d <= k < dp
-// are written as zeros (dp = padded dimension of the register variant), so the
-// inner loop needs no bound checks.
-// Every row is multiplied by f * s[p] (s may be null): folding the static
-// scale, 4^-order and the per-path scales into the differences leaves the
-// stream kernels nothing to scale, since <f s_i dx_i, s_j dy_j> is the scaled
+// Differences of both sides of a call in one launch, dimension-major in groups of
+// G: dx[p][k / G][c][k % G].  The lanes of a warp read neighbouring coarse columns
+// c in the same instruction (lane l is one column behind lane l-1), so a load
+// touches few cache lines.  G = 2 for the float64 register variants: 16 bytes a
+// lane, half the loads.  (All D values of a column together, dx[p][c][k], is as
+// few instructions, but spreads a load over up to 32 lines: 128 x 128 paths,
+// L = 33 / 128, d = 16, order 2: 1273 us against 524 with G = 1.)  Dimensions
+// d <= k < dp are zeros (dp: the register variants' padded dimension), so that
+// the inner loop needs no bound checks.
+// dx = T(x[p][c+1][k]) - T(x[p][c][k]), times f * s[p] (s may be null): folding
+// the static scale, 4^-order and the per-path scales into the differences leaves
+// the wavefronts nothing to scale, since <f s_i dx_i, s_j dy_j> is the scaled
 // increment f * s_i * s_j * <dx_i, dy_j> of sigpde/cuda_gram_kernels.py:52,60.
-template <typename T, typename TIN>
-__global__ void delta_kernel(const void *x_, int64_t npaths, int64_t len, int64_t d, int64_t dp, double f,
-                             const void *s_, void *dx_)
+struct DeltaSide {
+    const void *x;
+    const void *s;      // per-path scales or null
+    void *dx;
+    int64_t npaths, len;
+    double f;
+};
+struct DeltaParams {
+    DeltaSide side[2];  // the second may have no paths
+    int64_t d, dp;      // dp >= d: dimensions written
+    int pitch;          // values between two points in shared memory (odd: no bank conflicts)
+};
+
+constexpr int kDeltaThreads = 128, kDeltaCols = 128, kDeltaDims = 32;
+
+// Points come in and differences leave in different orders, so a tile of columns
+// by dimensions goes through shared memory and both sides of the copy are
+// contiguous.  A CTA takes whole paths (or a path's column tiles), so that
+// indexes need no 64-bit divisions: an element a thread, with three of them on
+// the chain before its first load, cost the Gram of 512 paths, L = 64, d = 16
+// 10.4 us, this kernel 5.0.
+template <typename T, typename TIN, int G>
+__global__ void __launch_bounds__(kDeltaThreads) delta_kernel(DeltaParams p)
 {
-    const TIN *__restrict__ x = reinterpret_cast<const TIN *>(x_);
-    const TIN *__restrict__ sc = reinterpret_cast<const TIN *>(s_);
-    T *__restrict__ dx = reinterpret_cast<T *>(dx_);
-    const int64_t nc = len - 1;
-    const int64_t per_path = nc * dp;
-    const int64_t total = npaths * per_path;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t p = e / per_path;
-        const int64_t r = e - p * per_path; // k * nc + c
-        const int64_t k = r / nc;
-        const int64_t c = r - k * nc;
-        if (k < d) {
-            const TIN *xp = x + p * len * d + c * d + k;
-            const T g = sc ? T(f * (double)sc[p]) : T(f);
-            dx[e] = (T(xp[d]) - T(xp[0])) * g;
-        } else {
-            dx[e] = T(0);
+    extern __shared__ __align__(16) unsigned char delta_smem[];
+    T *pts = reinterpret_cast<T *>(delta_smem);
+    const int64_t paths = p.side[0].npaths + p.side[1].npaths, d = p.d;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t i = blockIdx.x; i < paths; i += gridDim.x) {
+        const bool first = i < p.side[0].npaths;
+        const DeltaSide q = first ? p.side[0] : p.side[1];
+        const int64_t path = first ? i : i - p.side[0].npaths, nc = q.len - 1;
+        const T g = q.s ? T(q.f * (double)reinterpret_cast<const TIN *>(q.s)[path]) : T(q.f);
+        for (int64_t c0 = (int64_t)blockIdx.y * kDeltaCols; c0 < nc; c0 += (int64_t)gridDim.y * kDeltaCols) {
+            const int ncols = (int)(nc - c0 < kDeltaCols ? nc - c0 : kDeltaCols);
+            for (int64_t k0 = 0; k0 < p.dp; k0 += kDeltaDims) {
+                const int nw = (int)(p.dp - k0 < kDeltaDims ? p.dp - k0 : kDeltaDims); // written, a multiple of G
+                const int nk = (int)(d - k0 < nw ? (d > k0 ? d - k0 : 0) : nw);        // read
+                const TIN *x = reinterpret_cast<const TIN *>(q.x) + (path * q.len + c0) * d + k0;
+                const float inv = 1.0f / (float)nk; // e / nk below: e < 2^13, so the half keeps the floor exact
+                for (int e = threadIdx.x; e < (ncols + 1) * nk; e += kDeltaThreads) {
+                    const int r = (int)(((float)e + 0.5f) * inv), k = e - r * nk;
+                    pts[r * p.pitch + k] = T(x[r * d + k]);
+                }
+                __syncthreads();
+                T *dx = reinterpret_cast<T *>(q.dx) + (path * p.dp + k0) * nc + c0 * G;
+                for (int k = warp * G; k < nw; k += kDeltaThreads / 32 * G)
+                    for (int c = lane; c < ncols; c += 32) {
+                        const T *a = pts + c * p.pitch + k;
+                        T v[G];
+#pragma unroll
+                        for (int h = 0; h < G; ++h) v[h] = k + h < nk ? (a[p.pitch + h] - a[h]) * g : T(0);
+                        if constexpr (G == 2)
+                            *reinterpret_cast<double2 *>(dx + k * nc + c * G) = make_double2(v[0], v[1]);
+                        else
+                            dx[k * nc + c] = v[0];
+                    }
+                __syncthreads(); // the tile is free
+            }
         }
     }
 }
@@ -69,8 +109,8 @@ __global__ void delta_kernel(const void *x_, int64_t npaths, int64_t len, int64_
 struct StreamParams {
     int op;             // kOpPairwise / kOpGram / kOpGramSym
     int in64;           // 1: scales and output are float64, 0: float32
-    const void *dx;     // (nx, dp, ncx) in T, scaled (see delta_kernel)
-    const void *dy;     // (ny, dp, ncy) in T, scaled
+    const void *dx;     // differences in T, scaled (see delta_kernel; float64 register variants: groups of 2)
+    const void *dy;
     int64_t nx, ny;
     int64_t ncx, ncy, d;
     int64_t dp;         // padded dimension of dx / dy (d for the shared-memory variant)
@@ -164,6 +204,23 @@ __device__ __forceinline__ T pick_row(const T (&left)[R], int rstar)
     for (int r = 1; r < R; ++r)
         if (r == rstar) v = left[r];
     return v;
+}
+
+// The D differences of column c (`at`: the path's values + G c) of a path of nc columns.
+template <typename T, int D>
+__device__ __forceinline__ void stream_load_row(const T *at, int64_t nc, T (&v)[D])
+{
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int h = 0; h < D / 2; ++h) {
+            const double2 t = reinterpret_cast<const double2 *>(at)[h * nc];
+            v[2 * h] = t.x;
+            v[2 * h + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < D; ++k) v[k] = at[k * nc];
+    }
 }
 
 // Paired float32 cells.  A float32 lane of stream_reg_kernel is issue-bound
@@ -346,25 +403,30 @@ __device__ __forceinline__ Dbl2 stencil_cell<Dbl2>(Dbl2 k00, Dbl2 k01, Dbl2 k10,
 template <typename T, int D, int RC>
 __device__ __forceinline__ void stream_dot(const T (&dx)[RC][D], const T *dyr, int64_t ncy, T (&cc)[RC])
 {
+    T dy[D];
+    stream_load_row<T, D>(dyr, ncy, dy);
 #pragma unroll
     for (int rc = 0; rc < RC; ++rc) cc[rc] = T(0);
 #pragma unroll
-    for (int kk = 0; kk < D; ++kk) {
-        const T dy = dyr[kk * ncy];
+    for (int kk = 0; kk < D; ++kk)
 #pragma unroll
-        for (int rc = 0; rc < RC; ++rc) cc[rc] = fma(dx[rc][kk], dy, cc[rc]);
-    }
+        for (int rc = 0; rc < RC; ++rc) cc[rc] = fma(dx[rc][kk], dy[kk], cc[rc]);
 }
 
 template <typename T, int D, int RC>
 __device__ __forceinline__ void stream_load_dx(const T *dX, int64_t xi, int ncx, int ci0, T (&dx)[RC][D])
 {
+    constexpr int G = sizeof(T) == 8 ? 2 : 1;
     const T *src = dX + xi * (int64_t)D * ncx;
 #pragma unroll
     for (int rc = 0; rc < RC; ++rc) {
         const int ci = ci0 + (RC > 1 ? rc : 0);
+        if (ci < ncx) {
+            stream_load_row<T, D>(src + ci * G, ncx, dx[rc]);
+        } else {
 #pragma unroll
-        for (int kk = 0; kk < D; ++kk) dx[rc][kk] = (ci < ncx) ? src[kk * ncx + ci] : T(0);
+            for (int kk = 0; kk < D; ++kk) dx[rc][kk] = T(0);
+        }
     }
 }
 
@@ -377,6 +439,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 
     using BS = BlockShape<R, O>;
     constexpr int C = BS::C;
     constexpr int RC = BS::RC;
+    constexpr int G = sizeof(T) == 8 ? 2 : 1; // of the differences' layout
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
@@ -447,7 +510,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 
             // the next step: q + 1 of this entry, or step 0 of the next one
             const int qn = (q + 1 == nsteps) ? 0 : q + 1;
             const int cjn = (O <= 3) ? qn : ((qn * C) >> p.order);
-            stream_dot<T, D, RC>(dx, ((qn == 0) ? ndyp : dyp) + cjn, ncy, cc);
+            stream_dot<T, D, RC>(dx, ((qn == 0) ? ndyp : dyp) + (int64_t)cjn * G, ncy, cc);
             stream_block<T, R, O>(left, top, corner, A, B, bot);
             if (q == nsteps - 1 && lane == lstar) stream_store(p, item, xi, yj, pick_row(left, rstar));
             if (++q == nsteps) {
@@ -554,8 +617,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
             for (int rc = 0; rc < RC; ++rc) stencil_coefs(Dbl2{cca[rc], ccb[rc]}, A[rc], B[rc]);
             const int qn = (q + 1 == nsteps) ? 0 : q + 1;
             const int cjn = (O <= 3) ? qn : ((qn * C) >> p.order);
-            stream_dot<double, D, RC>(dx, ((qn == 0) ? ndypa : dypa) + cjn, ncy, cca);
-            stream_dot<double, D, RC>(dx, ((qn == 0) ? ndypb : dypb) + cjn, ncy, ccb);
+            stream_dot<double, D, RC>(dx, ((qn == 0) ? ndypa : dypa) + (int64_t)cjn * 2, ncy, cca);
+            stream_dot<double, D, RC>(dx, ((qn == 0) ? ndypb : dypb) + (int64_t)cjn * 2, ncy, ccb);
             stream_block<Dbl2, R, O>(left, top, corner, A, B, bot);
             if (q == nsteps - 1 && lane == lstar) {
                 const Dbl2 v = pick_row(left, rstar);

@@ -618,3 +618,17 @@ def test_c_abi_errors_are_reported(sig):
     st = _lib.lib().sigk_pairwise(host_buf.ctypes.data, X.data_ptr(), 2, 5, 5, 3, 0, 0, 1.0, None, None,
                                   out.data_ptr(), 0, None, 0, None)
     assert st == _lib.SIGK_EINVAL and "device pointer" in _lib.last_error()
+
+
+@pytest.mark.parametrize("L,d", [(2, 1), (128, 3), (129, 31), (130, 32), (257, 33), (258, 65), (40, 100)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_difference_tiles(sig, oracle, L, d, dtype, monkeypatch):
+    """delta_kernel at the edges of its tiles (128 columns, 32 dimensions), padded dimensions, both sides of a call."""
+    monkeypatch.setenv("SIGK_NO_PAIR_WAVE", "1")
+    k = sig.SigPDE(sig.kernels.LinearKernel(1.3), 0)
+    x, y = oracle.brownian(3, L, d, 51 + L), oracle.brownian(2, 35, d, 52 + L)
+    X, Y = cuda(x, dtype), cuda(y, dtype)
+    x, y = host(X).astype(np.float64) * np.sqrt(1.3), host(Y).astype(np.float64) * np.sqrt(1.3)
+    tol = RTOL64 if dtype == torch.float64 else 2e-7  # a float32 result is rounded once: 2^-24
+    assert_rel(host(k.gram(X, Y)), oracle.gram(x, y, 0), tol, "gram")
+    assert_rel(host(k.gram(X)), oracle.gram(x, None, 0), tol, "symmetric")
