@@ -65,13 +65,14 @@ struct PairWaveKernel {
 PairWaveKernel get_pair_wave_kernel(int R, int O);
 // D: dimension padded to a power of two in {2,...,32}; returns null unless
 // the lane's register tile (coarse rows per lane) * D <= 32.
-StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D);
-StreamFn get_stream_reg_kernel_f64(int R, int O, int D);
+// W: lanes a pipeline (float64 cells; 16 with R <= 8)
+StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D, int W = 32);
+StreamFn get_stream_reg_kernel_f64(int R, int O, int D, int W);
 StreamFn get_stream_reg_kernel_f32(int R, int O, int D);
 // float32 cells, two pairs per lane on paired float32 instructions (same shapes)
 StreamFn get_stream_reg_kernel_f32x2(int R, int O, int D);
 // float64 cells, two Gram entries of one x path per lane (kOpGram only)
-StreamFn get_stream_reg_kernel_f64x2(int R, int O, int D);
+StreamFn get_stream_reg_kernel_f64x2(int R, int O, int D, int W = 32);
 StreamFn get_stream_smem_kernel(bool f64cells, int R, int O);
 DeltaFn get_delta_kernel(bool grouped, bool f64cells, bool in64); // grouped: float64 dimensions in groups of 2
 // mat: increments from a precomputed matrix (tensor-core modes) instead of differences

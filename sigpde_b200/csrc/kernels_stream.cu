@@ -32,9 +32,9 @@ StreamFn get_stream_smem_kernel(bool f64cells, int R, int O)
     return f64cells ? by_r<double>(R, O) : by_r<float>(R, O);
 }
 
-StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D)
+StreamFn get_stream_reg_kernel(bool f64cells, int R, int O, int D, int W)
 {
-    return f64cells ? get_stream_reg_kernel_f64(R, O, D) : get_stream_reg_kernel_f32(R, O, D);
+    return f64cells ? get_stream_reg_kernel_f64(R, O, D, W) : get_stream_reg_kernel_f32(R, O, D);
 }
 
 DeltaFn get_delta_kernel(bool grouped, bool f64cells, bool in64)

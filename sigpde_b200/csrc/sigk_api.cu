@@ -1600,26 +1600,43 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
         sp.nitems = nitems;
         // float32 cells with register dx: two pairs per lane on paired instructions
         const bool paired = !f64 && pl.D && nitems >= 2 && !env_flag("SIGK_NO_PAIRED_F32");
+        // Float64 cells of pairs of at most 128 rows: half-warp pipelines of twice the rows a lane (half the pipeline
+        // fill, and a step's shuffles, loads and control for twice the cells), where the pairs are more than the
+        // resident warps.  us, half-warp / warp: 128 x 128 paths, L = 65, d = 8, order 1: 207 / 264; L = 50 / 47, d = 4,
+        // order 0: 114 / 139; L = 128, d = 4, order 0: 328 / 370; L = 17 / 66, d = 16, order 2: 221 / 356; symmetric,
+        // 180 paths, L = 50, d = 8, order 0: 157 / 252; 3000 pairs, L = 65 / 128, d = 8, order 1: 138 / 189.  1000 pairs
+        // are alike or slower (L = 33 / 128, d = 16, order 2: 155 / 134): a run of one pair has no fill to save.
         const bool dual_ok = f64 && pl.D && op == kOpGram && ny >= 2 && !env_flag("SIGK_NO_DUAL_F64");
+        int W = 32;
+        if (f64 && pl.D && pl.n <= 128 && !env_flag("SIGK_NO_HALF_WARP")) {
+            int Rh = 2;
+            while (16 * Rh < pl.n) Rh *= 2;
+            const int64_t runs = dual_ok ? nx * ((ny + 1) / 2) : nitems;
+            if (rows_per_coarse_lane(Rh, order) * pl.D <= 32 && runs > (int64_t)nsm * (dual_ok ? 8 : 12)) {
+                W = 16;
+                pl.R = Rh;
+            }
+        }
         // float64 cells of a Gram with register dx: two entries of one x path per lane
-        StreamFn dual_fn = dual_ok ? get_stream_reg_kernel_f64x2(pl.R, pl.O, pl.D) : nullptr;
+        StreamFn dual_fn = dual_ok ? get_stream_reg_kernel_f64x2(pl.R, pl.O, pl.D, W) : nullptr;
         const bool dual = dual_fn != nullptr;
         StreamFn fn = paired  ? get_stream_reg_kernel_f32x2(pl.R, pl.O, pl.D)
                       : dual  ? dual_fn
-                      : pl.D ? get_stream_reg_kernel(f64, pl.R, pl.O, pl.D)
+                      : pl.D ? get_stream_reg_kernel(f64, pl.R, pl.O, pl.D, W)
                              : get_stream_smem_kernel(f64, pl.R, pl.O);
         if (!fn) return fail(SIGK_EUNSUPPORTED, "no stream kernel for R=%d O=%d D=%d", pl.R, pl.O, pl.D);
         const size_t smem = pl.stage_bytes_per_warp * kWarpsPerBlock;
         int nb = 0;
         if ((st = blocks_per_sm((const void *)fn, smem, &nb))) return st;
-        int64_t nwarps = (int64_t)nsm * nb * kWarpsPerBlock;
+        const int pipes = kWarpsPerBlock * 32 / W; // of a CTA
+        int64_t nwarps = (int64_t)nsm * nb * pipes;
         const int64_t units = paired ? (nitems + 1) / 2 : dual ? nx * ((ny + 1) / 2) : nitems; // pipeline slots
         if (nwarps > units) nwarps = units;
         sp.per_warp = (units + nwarps - 1) / nwarps;
         if (paired) sp.per_warp *= 2; // an even run per warp: no half-empty slot but the last warp's
         if (dual) sp.nitems = units;  // the dual kernel walks entry pairs
         const int64_t used = (sp.nitems + sp.per_warp - 1) / sp.per_warp;
-        const int64_t blocks = (used + kWarpsPerBlock - 1) / kWarpsPerBlock;
+        const int64_t blocks = (used + pipes - 1) / pipes;
         fn<<<(unsigned)blocks, kWarpsPerBlock * 32, smem, stream>>>(sp);
         count_launch();
         cudaError_t e = cudaGetLastError();

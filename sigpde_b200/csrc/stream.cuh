@@ -430,9 +430,12 @@ __device__ __forceinline__ void stream_load_dx(const T *dX, int64_t xi, int ncx,
     }
 }
 
+// W lanes a pair pipeline: 32, or 16 for short pairs (n <= 16 R), where each half-warp streams its own run of pairs
+// (per_warp counts pairs a pipeline): twice the rows a lane for the same pairs and half the pipeline fill.
+//
 // Three CTAs (12 warps) per SM, except for blocks of 8 or more coarse rows a lane,
 // whose coefficient arrays need more than 168 registers.
-template <typename T, int R, int O, int D>
+template <typename T, int R, int O, int D, int W = 32>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 8 ? 2 : 3))
     stream_reg_kernel(StreamParams p)
 {
@@ -440,12 +443,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 
     constexpr int C = BS::C;
     constexpr int RC = BS::RC;
     constexpr int G = sizeof(T) == 8 ? 2 : 1; // of the differences' layout
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    const int64_t first = gwarp * p.per_warp;
-    if (first >= p.nitems) return; // warp-uniform
-    const int cnt = (int)((p.nitems - first) < p.per_warp ? (p.nitems - first) : p.per_warp);
+    const int lane = threadIdx.x & (W - 1); // within the pipeline
+    const int64_t pipe = ((int64_t)blockIdx.x * (kWarpsPerBlock * 32) + threadIdx.x) / W;
+    const int64_t wfirst = pipe / (32 / W) * (32 / W) * p.per_warp; // of the warp's first pipeline
+    if (wfirst >= p.nitems) return; // warp-uniform
+    // a second pipeline without items takes part in the shuffles only
+    const bool idle = W < 32 && pipe * p.per_warp >= p.nitems;
+    const int64_t first = idle ? p.nitems - 1 : pipe * p.per_warp;
+    const int cnt = idle ? 0 : (int)((p.nitems - first) < p.per_warp ? (p.nitems - first) : p.per_warp);
+    const int cnt_max = (int)((p.nitems - wfirst) < p.per_warp ? (p.nitems - wfirst) : p.per_warp);
     const T *dX = reinterpret_cast<const T *>(p.dx);
     const T *dY = reinterpret_cast<const T *>(p.dy);
     const int ncx = (int)p.ncx, ncy = (int)p.ncy;
@@ -475,11 +481,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 
     T corner_next = T(1);
     int q = 0, k = 0;
 
-    const int total = cnt * nsteps + 31;
+    const int total = cnt_max * nsteps + W - 1;
     for (int s = 0; s < total; ++s) {
         T top[C];
 #pragma unroll
-        for (int c = 0; c < C; ++c) top[c] = __shfl_up_sync(kFullMask, bot[c], 1);
+        for (int c = 0; c < C; ++c) top[c] = __shfl_up_sync(kFullMask, bot[c], 1, W);
         if (lane == 0) {
 #pragma unroll
             for (int c = 0; c < C; ++c) top[c] = T(1);
@@ -523,18 +529,21 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (BlockShape<R, O>::RC >= 
 
 // Two entries of one x path per lane, increments one step ahead as in
 // stream_reg_kernel.
-template <int R, int O, int D>
+template <int R, int O, int D, int W = 32>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel(StreamParams p)
 {
     using BS = BlockShape<R, O>;
     constexpr int C = BS::C;
     constexpr int RC = BS::RC;
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    const int64_t first = gwarp * p.per_warp;
-    if (first >= p.nitems) return; // warp-uniform
-    const int cnt = (int)((p.nitems - first) < p.per_warp ? (p.nitems - first) : p.per_warp);
+    const int lane = threadIdx.x & (W - 1); // within the pipeline
+    const int64_t pipe = ((int64_t)blockIdx.x * (kWarpsPerBlock * 32) + threadIdx.x) / W;
+    const int64_t wfirst = pipe / (32 / W) * (32 / W) * p.per_warp; // of the warp's first pipeline
+    if (wfirst >= p.nitems) return; // warp-uniform
+    // a second pipeline without items takes part in the shuffles only
+    const bool idle = W < 32 && pipe * p.per_warp >= p.nitems;
+    const int64_t first = idle ? p.nitems - 1 : pipe * p.per_warp;
+    const int cnt = idle ? 0 : (int)((p.nitems - first) < p.per_warp ? (p.nitems - first) : p.per_warp);
+    const int cnt_max = (int)((p.nitems - wfirst) < p.per_warp ? (p.nitems - wfirst) : p.per_warp);
     const double *dX = reinterpret_cast<const double *>(p.dx);
     const double *dY = reinterpret_cast<const double *>(p.dy);
     const int ncx = (int)p.ncx, ncy = (int)p.ncy;
@@ -574,13 +583,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
     Dbl2 corner_next = one;
     int q = 0, k = 0;
 
-    const int total = cnt * nsteps + 31;
+    const int total = cnt_max * nsteps + W - 1;
     for (int s = 0; s < total; ++s) {
         Dbl2 top[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            top[c].x = __shfl_up_sync(kFullMask, bot[c].x, 1);
-            top[c].y = __shfl_up_sync(kFullMask, bot[c].y, 1);
+            top[c].x = __shfl_up_sync(kFullMask, bot[c].x, 1, W);
+            top[c].y = __shfl_up_sync(kFullMask, bot[c].y, 1, W);
         }
         if (lane == 0) {
 #pragma unroll

@@ -620,6 +620,30 @@ def test_c_abi_errors_are_reported(sig):
     assert st == _lib.SIGK_EINVAL and "device pointer" in _lib.last_error()
 
 
+@pytest.mark.parametrize("L,order,d", [(17, 0, 3), (18, 0, 5), (33, 0, 8), (34, 0, 3), (65, 0, 2), (66, 0, 2), (129, 0, 4),
+                                       (33, 1, 7), (34, 1, 2), (65, 1, 8), (17, 2, 16), (33, 2, 3), (5, 3, 20), (17, 3, 4),
+                                       (9, 4, 6)])
+def test_half_warp_pipelines(sig, oracle, L, order, d, monkeypatch):
+    """Short pairs as half-warp pipelines, at the edges of the rows a lane and with runs that leave the last
+    warp's second pipeline short or empty: bitwise the whole-warp pipelines, within the fp64 bound of the oracle."""
+    k = sig.SigPDE(sig.kernels.LinearKernel(), order)
+    ly = max(36, L - 1) if order < 3 else 36
+    x, y = oracle.brownian(61, L, d, 41 + L), oracle.brownian(53, ly, d, 42 + L)
+    X, Y = cuda(x, torch.float64), cuda(y, torch.float64)
+    B = 1790
+    at = torch.arange(B, device="cuda")
+    Xp, Yp = X[at % 61].contiguous(), Y[at % 53].contiguous()
+
+    def values():
+        return [host(v) for v in (k.gram(X, Y), k.gram(X), k.gram(Y), k.pairwise(Xp, Yp))]
+
+    got = values()
+    assert_rel(got[0][:4, :5], oracle.gram(x[:4], y[:5], order), RTOL64, "gram")
+    monkeypatch.setenv("SIGK_NO_HALF_WARP", "1")
+    for a, b in zip(got, values()):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("L,d", [(2, 1), (128, 3), (129, 31), (130, 32), (257, 33), (258, 65), (40, 100)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 def test_difference_tiles(sig, oracle, L, d, dtype, monkeypatch):
