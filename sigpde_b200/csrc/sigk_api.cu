@@ -1529,15 +1529,19 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
         }
         precision = cell_prec(precision); // shapes outside the TC plan: CUDA-core increments, same cells
     }
+    // Few pairs: needs no workspace, but takes the one of the general route (sigk_workspace_size), so that a call is
+    // refused for its workspace whichever kernel its sizes choose.
+    PairWavePlan q;
     if (precision == SIGK_PREC_FP64) {
-        const PairWavePlan q = make_pair_wave_plan(op, nx, ny, lx - 1, ly - 1, d, order);
-        if (q.ok)
-            return run_pairs_wave(q, op, x, y, ny, lx, ly, d, dtype, order, static_scale, sx, sy, out, out_ld, stream);
+        q = make_pair_wave_plan(op, nx, ny, lx - 1, ly - 1, d, order);
         TcPlan t = make_mat64_plan(op, nx, ny, lx - 1, ly - 1, d, order);
         if (t.ok) {
             if (!ws || ws_bytes < t.ws_bytes)
                 return fail(SIGK_ENOMEM, "workspace of %zu bytes needed (got %zu)", t.ws_bytes, ws ? ws_bytes : 0);
             if (((uintptr_t)ws & 255) != 0) return fail(SIGK_EINVAL, "workspace must be 256-byte aligned");
+            if (q.ok)
+                return run_pairs_wave(q, op, x, y, ny, lx, ly, d, dtype, order, static_scale, sx, sy, out, out_ld,
+                                      stream);
             return run_pairs_mat64(t, op, x, y, nx, ny, lx, ly, d, dtype, order, static_scale, sx, sy, out, out_ld,
                                    precision, ws, stream);
         }
@@ -1546,6 +1550,8 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
     const int64_t nitems = op == kOpPairwise ? nx : (op == kOpGram ? nx * ny : nx * (nx + 1) / 2);
     Plan pl = make_plan(op, nx, ny, lx - 1, ly - 1, d, order, ts, false);
     if ((st = check_ws(pl, ws, ws_bytes))) return st;
+    if (q.ok)
+        return run_pairs_wave(q, op, x, y, ny, lx, ly, d, dtype, order, static_scale, sx, sy, out, out_ld, stream);
     const bool in64 = dtype == SIGK_F64;
     const bool f64 = precision == SIGK_PREC_FP64;
 
