@@ -28,7 +28,8 @@
 //   grad_gx_kernel / grad_gy_kernel   contractions of dk/dc with the scaled
 //                    differences of the other side: the gradients with
 //                    respect to the coarse differences;
-//   grad_points_kernel   differences of those: gradients at the points.
+//   grad_points_kernel   their partial sums, and the differences of those: gradients at the points;
+//   grad_stage_kernel    the scaled differences in every layout that these read.
 #pragma once
 
 #include "dgemm_inc.cuh"
@@ -635,7 +636,7 @@ __global__ void grad_inc_blocks_kernel(const void *inc, int in64, int64_t s0, in
 // Gradients with respect to the x side's scaled-difference rows: for each
 // matrix row m (x path il, cell ci), part[slice][m][k] = sum over the slice's
 // y cells n paired with it (Gram: all of them; pairwise: its own pair's) of
-// G[n][m] * dyt[n][k].  grad_reduce_kernel adds the slices in order.
+// G[n][m] * dyt[n][k].  grad_points_kernel adds the slices in order.
 // dxt / dyt are the scaled differences in row layout (one row of d values per
 // cell; x rows padded to rows_x per path with zeros), so that the inner loops
 // index them directly.

@@ -853,13 +853,18 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         // Below that, where the fused kernels would read each lane's dx from shared memory: a streaming shape whose
         // dx tile does not fit registers (ms, fused / matrix: 80 x 80, L = 200, order 0, d = 8: 2.04 / 0.90, with the
         // tile in registers at d = 4: 0.41 / 0.83; 128 x 128, L = 120, order 1, d = 12: 2.51 / 0.97), and several
-        // bands from d = 8 on (80 x 80, L = 300, order 1: 4.55 / 3.32 at d = 8, 2.91 / 3.18 at d = 4).
+        // bands from d = 8 on (80 x 80, L = 300, order 1: 4.55 / 3.32 at d = 8, 2.91 / 3.18 at d = 4).  From order 2 on
+        // the increments are few beside the cells, and a warp with one pair has latencies to hide them in: with fewer
+        // than 6 pairs an SM the matrix only adds its own time (L = 239 / 154, d = 10, order 2: 588 pairs 389 / 437 us,
+        // 960 pairs 505 / 478).
         const int64_t n = ncx << order, m = ncy << order;
         const int Rs = pick_rows(n), C = order >= 4 ? 8 : 1 << order;
         int Dp = 2;
         while (Dp < d) Dp <<= 1;
         const bool band = n <= 32 * Rs, regs = rows_per_coarse_lane(Rs, order) * Dp <= 32;
-        if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 : d < 8)) return TcPlan{};
+        const int64_t pairs = op == kOpGram ? nx * ny : nx * (nx + 1) / 2;
+        const bool few = order >= 2 && pairs < (int64_t)sm_count() * 6;
+        if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 : d < 8 || few)) return TcPlan{};
     }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,
     // which forms the dot products a step ahead of the cells (256 x 256, L = 64, d = 16, order 2: 1.97 vs
@@ -1443,8 +1448,11 @@ PairWavePlan make_pair_wave_plan(int op, int64_t nx, int64_t ny, int64_t ncx, in
         const int64_t together = per_sm < res ? per_sm : res;
         const double steps = (double)((q.nbands + q.nw - 1) / q.nw) * (q.nsteps + 31 + (q.nw - 1) * kNormLag);
         const double slots = 1.15 * (6.0 * R * q.k.cols + 10.0 * rc * q.k.ccols + 50.0);
-        const double shared = slots * (double)((together * q.nw + 3) / 4), alone = slots + 130.0;
-        const double cost = (double)((per_sm + together - 1) / together) * steps * (shared > alone ? shared : alone);
+        const double shared = slots * (double)((together * q.nw + 3) / 4), alone = slots + 200.0;
+        // and the increments before it (224 pairs, L = 128, order 2, one CTA an SM: 144 us at d = 10, 167 at d = 24)
+        const double incs = (together == 1 ? 106.0 : 50.0) * (double)(per_sm * ((ncx + 31) / 32) * ((ncy + 31) / 32) * d);
+        const double cost =
+            (double)((per_sm + together - 1) / together) * steps * (shared > alone ? shared : alone) + incs;
         if (best.ok && cost >= best_cost) continue;
         q.ok = true;
         best = q;

@@ -25,8 +25,8 @@
 //                       cp.async.bulk.tensor, to HBM);
 //   stream_inc_kernel   the streaming wavefront of stream.cuh reading its
 //                       increments from that matrix (vector loads of the
-//                       lane's coarse rows, or for long steps a cp.async ring
-//                       two steps ahead) instead of forming dot products.
+//                       lane's coarse rows, one step ahead) instead of forming
+//                       dot products.
 #pragma once
 
 #include <cuda.h> // CUtensorMap
