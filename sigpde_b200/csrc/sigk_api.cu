@@ -865,6 +865,9 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         const int64_t pairs = op == kOpGram ? nx * ny : nx * (nx + 1) / 2;
         const bool few = order >= 2 && pairs < (int64_t)sm_count() * 6;
         if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 : d < 8 || few)) return TcPlan{};
+        // not where one x path's increments alone exceed a chunk: the fused kernels need no matrix at all
+        if ((size_t)((ncx + 3) / 4 * 4) * (size_t)((op == kOpGram ? ny : nx) * ncy) * sizeof(double) > tc_chunk_cap())
+            return TcPlan{};
     }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,
     // which forms the dot products a step ahead of the cells (256 x 256, L = 64, d = 16, order 2: 1.97 vs
@@ -1543,6 +1546,10 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
     if (precision == SIGK_PREC_FP64) {
         q = make_pair_wave_plan(op, nx, ny, lx - 1, ly - 1, d, order);
         TcPlan t = make_mat64_plan(op, nx, ny, lx - 1, ly - 1, d, order);
+        // the narrow paths' matrix is a choice: a smaller workspace that holds the fused route's differences takes that
+        if (t.ok && d < kDgMinDim && ws && ws_bytes < t.ws_bytes &&
+            ws_bytes >= make_plan(op, nx, ny, lx - 1, ly - 1, d, order, sizeof(double), false).ws_bytes)
+            t.ok = false;
         if (t.ok) {
             if (!ws || ws_bytes < t.ws_bytes)
                 return fail(SIGK_ENOMEM, "workspace of %zu bytes needed (got %zu)", t.ws_bytes, ws ? ws_bytes : 0);
@@ -2202,8 +2209,15 @@ extern "C" int sigk_gram_noalloc(const void *x, const void *y, int64_t n_x, int6
                                  const void *scale_x, const void *scale_y, void *out, int precision,
                                  sigk_stream_t stream)
 {
-    const size_t need =
-        sigk_workspace_size(SIGK_OP_GRAM, n_x, n_y, len_x, len_y, dim, order, dtype, precision);
+    size_t need = sigk_workspace_size(SIGK_OP_GRAM, n_x, n_y, len_x, len_y, dim, order, dtype, precision);
+    if (need > kNoAllocScratchBytes && dim < kDgMinDim) { // a narrow Gram's matrix, which run_pairs does without
+        const int64_t ncx = len_x - 1, ncy = len_y - 1;
+        const bool tc = is_tc(precision) &&
+                        (make_fused_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order, precision).ok ||
+                         make_tc_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order, tsize_of(precision)).ok);
+        if (!tc && cell_prec(precision) == SIGK_PREC_FP64 && make_mat64_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order).ok)
+            need = make_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order, sizeof(double), false).ws_bytes;
+    }
     if (need > kNoAllocScratchBytes)
         return fail(SIGK_EINVAL,
                     "sigk_gram_noalloc: this Gram needs %zu bytes of scratch; the no-allocation entry point has "

@@ -112,3 +112,22 @@ def test_noalloc_gram_refuses_more_than_its_scratch():
     assert st == _lib.SIGK_EINVAL
     msg = _lib.last_error()
     assert "8 MiB" in msg and "sigk_gram_noalloc" in msg
+
+
+@pytest.mark.parametrize("nx,ny,length,dim,order", [(60, 50, 200, 8, 0), (40, 50, 120, 12, 1)])
+def test_noalloc_takes_narrow_grams_without_their_matrix(nx, ny, length, dim, order):
+    """Grams below d = 16 whose increment matrix exceeds the scratch: the no-allocation entry point, and sigk_gram
+    with a workspace of the differences alone, take the fused kernels; the same values."""
+    from sigpde_b200 import _lib
+    lib = _lib.lib()
+    X, Y = _paths(nx, length, dim, 5), _paths(ny, length, dim, 6)
+    want, nws = _gram_with_workspace(lib, X, Y, order, None, None)
+    assert nws > NOALLOC_BYTES
+    assert torch.equal(_gram_noalloc(lib, X, Y, order, None, None), want)
+    out = torch.full_like(want, float("nan"))
+    small = 2 * (nx + ny) * length * dim * 8
+    ws = torch.empty(small, dtype=torch.uint8, device="cuda")
+    st = lib.sigk_gram(X.data_ptr(), Y.data_ptr(), nx, ny, length, length, dim, _lib.SIGK_F32, order, 1.0, None, None,
+                       out.data_ptr(), 0, ws.data_ptr(), small, torch.cuda.current_stream().cuda_stream)
+    assert st == 0, _lib.last_error()
+    assert torch.equal(out, want)
