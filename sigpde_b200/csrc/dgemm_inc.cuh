@@ -2,7 +2,8 @@
 //
 // The fused kernels form each coarse increment <dx_ci, dy_cj> inside the
 // wavefront: d FMAs per coarse cell, re-done by every pair, on the critical
-// path of each step.  For d >= 16 that dominates, so the Gram ops first write
+// path of each step.  For d >= 16 (and below, where a lane's dx does not fit its
+// registers) that dominates, so the Gram ops first write
 // the increments of all pairs with one register-blocked FP64 GEMM over the
 // scaled, dimension-major differences (delta_kernel) and the wavefront then
 // reads them (stream_inc_kernel / pair_kernel in matrix mode, float64
