@@ -138,7 +138,7 @@ __device__ __forceinline__ void stream_decode(const StreamParams &p, int64_t ite
 // own step, so this runs once per lane and item, in a divergent branch: decoding
 // the item's number there (a 64-bit division, for the triangle a float64 square
 // root) cost the Gram of 256 x 256 paths, L = 128, order 2, 0.22 of its 5.12 ms
-// and the symmetric Grams of short paths more.
+// and the symmetric Grams of short paths more (not in stream_smem_kernel).
 __device__ __forceinline__ void stream_next(int op, int64_t ny, int64_t &xi, int64_t &yj)
 {
     ++yj;
@@ -679,9 +679,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
     int64_t item = first, xi = 0, yj = 0;
     const T *dyp = dY;
     const T *dxs = buf0;
-    int64_t sxi, syj;   // the next pair to stage
-    stream_decode(p, first, sxi, syj);
-    int64_t nxi = sxi, nyj = syj; // the lane's next pair
     int staged = 0;     // pairs staged so far (warp-uniform)
     int next_stage = 0; // step at which lane 0 starts pair `staged`
 
@@ -689,6 +686,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
     for (int s = 0; s < total; ++s) {
         if (staged < cnt && s == next_stage) { // warp-uniform: lane 0 starts a new pair now
             T *dst = (staged & 1) ? buf1 : buf0;
+            int64_t sxi, syj;
+            stream_decode(p, first + staged, sxi, syj);
             const T *src = dX + sxi * (int64_t)d * ncx;
             __syncwarp();
             for (int rc = 0; rc < RC; ++rc) {
@@ -697,7 +696,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
                 for (int kk = 0; kk < d; ++kk) dst[(rc * d + kk) * 32 + lane] = ok ? src[kk * ncx + ci] : T(0);
             }
             __syncwarp();
-            stream_next(p.op, p.ny, sxi, syj);
             ++staged;
             next_stage += nsteps;
         }
@@ -711,9 +709,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) stream_smem_kernel(Stream
         if (s >= lane && k < cnt) {
             if (q == 0) {
                 item = first + k;
-                xi = nxi;
-                yj = nyj;
-                stream_next(p.op, p.ny, nxi, nyj);
+                // decoded here, not kept by stream_next: two more pairs of indexes across the loop over the
+                // dimensions cost 100 x 110 paths, L = 200 / 180, d = 9, order 1, float32 1.92 -> 2.28 ms
+                stream_decode(p, item, xi, yj);
                 dyp = dY + yj * (int64_t)d * ncy;
                 dxs = (k & 1) ? buf1 : buf0;
 #pragma unroll
