@@ -185,6 +185,14 @@ __device__ __forceinline__ void normalize_path(const NormParams &p, int64_t b, b
     }
 }
 
+// Values that lane 0's pointer to the row above moves on after step q (nsteps blocks of `cols` values).  The loads go on
+// until the warp's window of steps closes, so the pointer stays on the last block: behind the last row of a CTA lies
+// its neighbour's region, or the end of the workspace.
+__host__ __device__ constexpr int norm_row_move(int q, int nsteps, int cols)
+{
+    return (unsigned)q < (unsigned)(nsteps - 1) ? cols : 0;
+}
+
 // of the solving warps
 __device__ __forceinline__ void norm_barrier(int warps)
 {
@@ -333,7 +341,7 @@ __device__ __forceinline__ double norm_solve(const P &p, const double *tile, dou
                         tn[c] = in ? v.x : 1.0;
                         tn[c + 1] = in ? v.y : 1.0;
                     }
-                    above.move(in && b > 0 ? C : 0);
+                    above.move(b > 0 ? norm_row_move(q, nsteps, C) : 0);
                     const double fq = in ? f : 0.0;
 #pragma unroll
                     for (int cc = 0; cc < CC; ++cc)
