@@ -94,7 +94,7 @@ template <>
 struct NormMem<false> {
     const double *a;
     __device__ __forceinline__ explicit NormMem(const double *p) : a(p) {}
-    __device__ __forceinline__ void move(int values) { a += values; }
+    __device__ __forceinline__ void move(int64_t values) { a += values; }
     __device__ __forceinline__ double get(int i) const
     {
         double v;
@@ -191,6 +191,14 @@ __device__ __forceinline__ void normalize_path(const NormParams &p, int64_t b, b
 __host__ __device__ constexpr int norm_row_move(int q, int nsteps, int cols)
 {
     return (unsigned)q < (unsigned)(nsteps - 1) ? cols : 0;
+}
+
+// Values from a lane's rows of the first coarse column to those of step q, where a coarse column takes several steps
+// (steps outside the run stay on the first one).  A tile in the workspace has nc * pitch values: past 2^31 from about
+// 46000 coarse columns on.
+__host__ __device__ constexpr int64_t norm_col_offset(int q, int nsteps, int cols, int order, int pitch)
+{
+    return (int64_t)((((unsigned)q < (unsigned)nsteps ? q : 0) * cols) >> order) * pitch;
 }
 
 // of the solving warps
@@ -351,7 +359,7 @@ __device__ __forceinline__ double norm_solve(const P &p, const double *tile, dou
                     const int qn = q + PF;
                     NormMem<SMEM> src = rows;
                     if constexpr (!NS::WHOLE)
-                        src.move(((((unsigned)qn < (unsigned)nsteps ? qn : 0) * C) >> p.order) * p.pitch);
+                        src.move(norm_col_offset(qn, nsteps, C, p.order, p.pitch));
 #pragma unroll
                     for (int cc = 0; cc < CC; ++cc) {
                         if constexpr (RC == 1) {
