@@ -350,11 +350,16 @@ __device__ __forceinline__ double norm_solve(const P &p, const double *tile, dou
                         tn[c + 1] = in ? v.y : 1.0;
                     }
                     above.move(b > 0 ? norm_row_move(q, nsteps, C) : 0);
+                    // An infinite increment times 0 is NaN: a root-find takes the NaN of its path for an overflow either
+                    // way, and a selection a coefficient cost it 3%; a pair's own value may be infinite.
                     const double fq = in ? f : 0.0;
 #pragma unroll
                     for (int cc = 0; cc < CC; ++cc)
 #pragma unroll
-                        for (int rc = 0; rc < RC; ++rc) stencil_coefs(cn[j % PF][cc][rc] * fq, A[cc][rc], B[cc][rc]);
+                        for (int rc = 0; rc < RC; ++rc) {
+                            const double v = cn[j % PF][cc][rc];
+                            stencil_coefs(CHAIN ? v * fq : in ? v * f : 0.0, A[cc][rc], B[cc][rc]);
+                        }
                     // increments of step q + PF; `rows` stays inside the columns
                     const int qn = q + PF;
                     NormMem<SMEM> src = rows;
