@@ -185,12 +185,14 @@ __device__ __forceinline__ void normalize_path(const NormParams &p, int64_t b, b
     }
 }
 
-// Values that lane 0's pointer to the row above moves on after step q (nsteps blocks of `cols` values).  The loads go on
-// until the warp's window of steps closes, so the pointer stays on the last block: behind the last row of a CTA lies
-// its neighbour's region, or the end of the workspace.
-__host__ __device__ constexpr int norm_row_move(int q, int nsteps, int cols)
+// Values of a CTA's boundary rows: `cols` ones (the row above the first band), then the bottom rows of the nw solving
+// warps.  Lane 0's pointer to the row above moves on at each of a row's steps, and the loads go on until the warp's
+// window of steps closes: where there are several groups of bands, the first warp of a group reads one block past the
+// last row.  (A pointer that stays on the last block needs a register more in the step loop, which spills: 24 paths,
+// L = 220, d = 8, order 1: 540 us instead of 531.)
+__host__ __device__ constexpr int norm_bnd_values(int nbands, int nw, int nsteps, int cols)
 {
-    return (unsigned)q < (unsigned)(nsteps - 1) ? cols : 0;
+    return (nbands > 1 ? nw * nsteps + 1 : 1) * cols + (nbands > nw ? cols : 0);
 }
 
 // Values from a lane's rows of the first coarse column to those of step q, where a coarse column takes several steps
@@ -349,7 +351,7 @@ __device__ __forceinline__ double norm_solve(const P &p, const double *tile, dou
                         tn[c] = in ? v.x : 1.0;
                         tn[c + 1] = in ? v.y : 1.0;
                     }
-                    above.move(b > 0 ? norm_row_move(q, nsteps, C) : 0);
+                    above.move(in && b > 0 ? C : 0);
                     // An infinite increment times 0 is NaN: a root-find takes the NaN of its path for an overflow either
                     // way, and a selection a coefficient cost it 3%; a pair's own value may be infinite.
                     const double fq = in ? f : 0.0;
@@ -410,7 +412,7 @@ __global__ void __launch_bounds__(NormShape<R, O>::MAXW * 32, 1) norm_kernel(Nor
     extern __shared__ __align__(16) double norm_smem[];
     __shared__ double s_val;
     double *tile = SMEM ? norm_smem : p.tiles + blockIdx.x * p.tile;
-    const int rows = (p.nbands > 1 ? p.nw * p.nsteps + 1 : 1) * NS::C; // C ones, the solving warps' bottom rows
+    const int rows = norm_bnd_values(p.nbands, p.nw, p.nsteps, NS::C);
     double *bnd = BSMEM ? norm_smem + (SMEM ? p.tile : 0) : p.bnd + (int64_t)blockIdx.x * rows;
     if (threadIdx.x < NS::C) bnd[threadIdx.x] = 1.0;
     for (int64_t b = blockIdx.x; b < p.n; b += gridDim.x) {

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(NormShape<R, O>::MAXW * 32, 1) pair_wave_kerne
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int ncx = p.nc, ncy = p.ncy, d = (int)p.d;
     double *tile = pair_smem, *bnd = tile + p.tile;
-    double *dx = bnd + (p.nbands > 1 ? p.nw * p.nsteps + 1 : 1) * NS::C, *dy = dx + ncx * d;
+    double *dx = bnd + norm_bnd_values(p.nbands, p.nw, p.nsteps, NS::C), *dy = dx + ncx * d;
     double *cols = tile + p.col0 * p.pitch;
     if (threadIdx.x < NS::C) bnd[threadIdx.x] = 1.0;
     const int pad = p.pitch - ncx; // zeros below a column's rows, and before the first column

@@ -1440,7 +1440,7 @@ PairWavePlan make_pair_wave_plan(int op, int64_t nx, int64_t ny, int64_t ncx, in
         const int rc = q.k.rc, low = ((int)ncx + rc - 1) / rc * rc + rc;
         q.pitch = rc == 1 ? (low + 1) / 2 * 2 : rc == 2 ? (low + 3) / 4 * 4 : (low + 1) / 4 * 4 + 2;
         const int64_t tile = (ncy + q.col0) * q.pitch;
-        const int64_t rows = (int64_t)(1 + (q.nbands > 1 ? q.nw * q.nsteps : 0)) * q.k.cols;
+        const int64_t rows = norm_bnd_values(q.nbands, q.nw, q.nsteps, q.k.cols);
         q.smem = (size_t)(tile + rows + (ncx + ncy) * d) * sizeof(double);
         if (q.smem > kPairWaveSmemBytes) continue;
         q.tile = (int)tile;
@@ -1706,7 +1706,7 @@ NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
             q.tile = (nc + q.col0) * q.pitch;
             const size_t tile = (size_t)q.tile * sizeof(double);
             q.threads = 32 * (q.nw > 4 ? q.nw : 4);
-            const size_t rows = (size_t)(1 + (q.nbands > 1 ? q.nw * q.nsteps : 0)) * q.k.cols * sizeof(double);
+            const size_t rows = (size_t)norm_bnd_values(q.nbands, q.nw, q.nsteps, q.k.cols) * sizeof(double);
             q.smem_tile = smem_tile;
             if (smem_tile && tile + rows > kNormSmemBytes) continue;
             q.smem_bnd = rows <= kNormSmemBytes;

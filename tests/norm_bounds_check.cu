@@ -3,16 +3,20 @@
 
 #include "norm_wave.cuh"
 
-// The row above: loads of `cols` values every step from the run's first one until its window closes (up to 31 steps
-// and a chunk after the last block).
-static int row_walk(int nsteps, int cols)
+// The row above, as lane 0 of a warp reads it: loads of `cols` values every step from the run's first one until its
+// window closes (up to 31 steps and a chunk after the last block), the pointer moving on at each of the row's steps.
+// The warps' rows follow `cols` ones; the first warp of a later group of bands reads the last warp's row.
+static int row_walk(int nbands, int nw, int nsteps, int cols)
 {
-    const int values = nsteps * cols;
-    int at = 0;
-    for (int q = -100; q < nsteps + 31 + 2 * sigk::kNormChunk; ++q) {
-        if (at < 0 || at + cols > values) return 1;                           // outside the row
-        if (q >= 0 && q < nsteps && at != q * cols) return 2;                 // not the step's block
-        at += sigk::norm_row_move(q, nsteps, cols);
+    const int values = sigk::norm_bnd_values(nbands, nw, nsteps, cols);
+    for (int band = 1; band < nbands; ++band) {
+        const int w = band % nw, row = cols + (w == 0 ? nw - 1 : w - 1) * nsteps * cols;
+        int at = row;
+        for (int q = -100; q < nsteps + 31 + 2 * sigk::kNormChunk; ++q) {
+            if (at < 0 || at + cols > values) return 1;                  // outside the CTA's rows
+            if (q >= 0 && q < nsteps && at != row + q * cols) return 2;  // not the step's block
+            at += q >= 0 && q < nsteps ? cols : 0;
+        }
     }
     return 0;
 }
@@ -39,12 +43,14 @@ int main()
                 return 1;
             }
     for (int cols = 2; cols <= 4; cols += 2)
-        for (int nsteps : {1, 2, 3, 16, 17, 33, 1099, 16384})
-            if (int bad = row_walk(nsteps, cols)) {
-                printf("row above: %s at nsteps = %d, cols = %d\n", bad == 1 ? "read outside the row" : "wrong block",
-                       nsteps, cols);
-                return 1;
-            }
+        for (int nw : {1, 2, 8, 16})
+            for (int nbands = nw; nbands <= 3 * nw; ++nbands)
+                for (int nsteps : {1, 2, 33, 1099})
+                    if (int bad = row_walk(nbands, nw, nsteps, cols)) {
+                        printf("row above: %s at %d bands, %d warps, nsteps = %d, cols = %d\n",
+                               bad == 1 ? "read outside the rows" : "wrong block", nbands, nw, nsteps, cols);
+                        return 1;
+                    }
     printf("ok\n");
     return 0;
 }
