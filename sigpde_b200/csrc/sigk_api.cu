@@ -868,6 +868,13 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         // not where one x path's increments alone exceed a chunk: the fused kernels need no matrix at all
         if ((size_t)((ncx + 3) / 4 * 4) * (size_t)((op == kOpGram ? ny : nx) * ncy) * sizeof(double) > tc_chunk_cap())
             return TcPlan{};
+        // nor where the matrix comes in chunks of too few pairs: each chunk's wavefront waits for its slowest warp, and
+        // several bands want more of them (ms, fused / matrix.  One band: 128 x 128, L = 120, d = 12, order 1, chunks
+        // of 384 pairs 2.75 / 2.75, 512 2.75 / 2.19; 200 x 170, L = 250, d = 14, order 1, 510 15.2 / 14.1, 1170 15.2 /
+        // 9.8.  Several: 80 x 80, L = 300, d = 8, order 1, 725 4.5 / 7.1, 1450 4.5 / 4.4, 2900 4.5 / 3.6; 40 x 40,
+        // L = 400, d = 8, order 3, 1600 5.7 / 5.9; symmetric, 47 paths, L = 1786, d = 11, order 1, 113 22.8 / 145).
+        const TcPlan t = mat64_layout(op, nx, ny, ncx, ncy, d, order, true);
+        if (t.nchunks > 1 && pairs < t.nchunks * sm_count() * (band ? 6 : 12)) return TcPlan{};
     }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,
     // which forms the dot products a step ahead of the cells (256 x 256, L = 64, d = 16, order 2: 1.97 vs
