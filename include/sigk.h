@@ -129,6 +129,14 @@ SIGK_API size_t sigk_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t le
                            int order, int dtype, int precision);
 
 /*
+ * The least scratch with which the same call runs.  It is sigk_workspace_size but for float64-cell Grams of narrow
+ * paths (dim < 16): with all of sigk_workspace_size (up to 1.5 GiB) they read a matrix of all increments, with less they
+ * take kernels that need the path differences alone and give the same values.
+ */
+SIGK_API size_t sigk_workspace_min_size(int op, int64_t n_x, int64_t n_y, int64_t len_x, int64_t len_y, int64_t dim,
+                                        int order, int dtype, int precision);
+
+/*
  * Pairwise signature kernel with the linear static kernel.
  * Replaces SigPDE.pairwise's increment build + PairwisePDESolver.solve /
  * solve_scaled (sigpde/torch/kernel.py:31-65, sigpde/torch/kernel.py:13-16,
@@ -417,8 +425,8 @@ SIGK_API int sigk_ragged_status(const void *workspace, sigk_stream_t stream);
  * Same arguments and result as sigk_gram, minus the workspace: the scratch
  * sigk_gram takes from the caller comes from an 8 MiB array that is part of
  * this library's device image (each GPU that loads the library holds it until
- * the process exits).  Nothing is allocated.  A Gram whose scratch
- * (sigk_workspace_size(SIGK_OP_GRAM, ...)) exceeds 8 MiB is rejected with
+ * the process exits).  Nothing is allocated.  A Gram whose least scratch
+ * (sigk_workspace_min_size(SIGK_OP_GRAM, ...)) exceeds 8 MiB is rejected with
  * SIGK_EINVAL and a message naming the limit; 256 x 256 paths of length 128
  * in 8 dimensions at order 2 with float64 cells need about 4.2 MB.
  *

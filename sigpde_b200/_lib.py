@@ -58,6 +58,7 @@ SIGNATURES = {
     "sigk_launch_count": (ctypes.c_uint64, []),
     "sigk_set_wait_limit": (_i64, [_i64]),
     "sigk_workspace_size": (_sz, [_int, _i64, _i64, _i64, _i64, _i64, _int, _int, _int]),
+    "sigk_workspace_min_size": (_sz, [_int, _i64, _i64, _i64, _i64, _i64, _int, _int, _int]),
     "sigk_pairwise": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _int, _int, _dbl, _vp, _vp, _vp, _int, _vp, _sz,
                              _vp]),
     "sigk_gram": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _int, _dbl, _vp, _vp, _vp, _int, _vp, _sz,

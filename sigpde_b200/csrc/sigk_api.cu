@@ -332,6 +332,7 @@ struct TcPlan {
     int kp;
     int64_t rows_x, rows_y;   // matrix rows per x path (ncx rounded up to 4) and per y path
     int64_t chunk, nchunks;   // x paths per chunk
+    int64_t cap_pairs;        // > 0: chunks of a symmetric Gram by their x paths times y paths instead
     int64_t a_tiles, b_tiles; // operand tiles per image
     size_t a_bytes, b_bytes;  // bytes of one (hi or lo) image
     size_t err_off, a_off, b_off, ct_off, ws_bytes;
@@ -343,14 +344,14 @@ struct TcPlan {
 // matrices measured slower with small chunks, so they keep kTcChunkBytes.
 constexpr size_t kTcChunkBytesHalfWarpO1 = size_t(1) << 30;
 
-size_t tc_chunk_cap(bool half_warp_order1 = false)
+size_t tc_chunk_cap(size_t by_default = kTcChunkBytes)
 {
     const char *v = getenv("SIGK_TC_CHUNK_MB");
     if (v && v[0]) {
         long long mb = atoll(v);
         if (mb > 0) return (size_t)mb << 20;
     }
-    return half_warp_order1 ? kTcChunkBytesHalfWarpO1 : kTcChunkBytes;
+    return by_default;
 }
 
 TcPlan make_tc_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order, size_t tsize)
@@ -375,7 +376,7 @@ TcPlan make_tc_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, in
     t.rows_y = ncy;
     const int64_t width = op == kOpPairwise ? ncy : (op == kOpGram ? ny : nx) * ncy; // matrix rows per x path
     const size_t per_x = (size_t)t.rows_x * (size_t)width * sizeof(float);
-    int64_t chunk = (int64_t)(tc_chunk_cap(order == 1 && n <= 128) / per_x);
+    int64_t chunk = (int64_t)(tc_chunk_cap(order == 1 && n <= 128 ? kTcChunkBytesHalfWarpO1 : kTcChunkBytes) / per_x);
     if (chunk < 1) chunk = 1;
     if (chunk > nx) chunk = nx;
     t.chunk = chunk;
@@ -809,10 +810,19 @@ int launch_dgemm_inc(const DgemmIncParams &gp, cudaStream_t stream)
     return e == cudaSuccess ? SIGK_OK : cuda_fail(e, "float64 increment GEMM launch");
 }
 
+// End of the chunk of x paths that starts at i0.
+int64_t chunk_end(const TcPlan &t, int64_t i0, int64_t nx)
+{
+    int64_t i1 = i0 + t.chunk;
+    if (t.cap_pairs) // x paths i0 .. i1 - 1 take i1 y paths' columns
+        for (i1 = i0 + 1; i1 < nx && (i1 + 1 - i0) * (i1 + 1) <= t.cap_pairs;) ++i1;
+    return i1 < nx ? i1 : nx;
+}
+
 // es: bytes per element of the increment matrix (8 for float64 cells, 4 for float32 cells); the chunk of x
 // paths per launch and the matrix's share of the workspace follow it.
 TcPlan mat64_layout(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order, bool diffs,
-                    size_t es = sizeof(double))
+                    size_t es = sizeof(double), size_t cap = tc_chunk_cap(), bool narrow = false)
 {
     TcPlan t{};
     const int64_t n = ncx << order, m = ncy << order;
@@ -832,19 +842,39 @@ TcPlan mat64_layout(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, in
     t.rows_y = ncy;
     const int64_t ny_paths = op == kOpGram ? ny : nx;
     const size_t per_x = (size_t)t.rows_x * (size_t)(ny_paths * ncy) * es;
-    int64_t chunk = (int64_t)(tc_chunk_cap() / per_x);
+    int64_t chunk = (int64_t)(cap / per_x);
     if (chunk < 1) chunk = 1;
     if (chunk > nx) chunk = nx;
     t.chunk = chunk;
     t.nchunks = (nx + chunk - 1) / chunk;
+    size_t mat_bytes = (size_t)chunk * per_x;
+    if (narrow && op == kOpGram) { // equal chunks
+        t.chunk = (nx + t.nchunks - 1) / t.nchunks;
+        t.nchunks = (nx + t.chunk - 1) / t.chunk;
+        mat_bytes = (size_t)t.chunk * per_x;
+    } else if (narrow && t.nchunks > 1) { // symmetric: as many x paths as their own columns let in
+        t.cap_pairs = (int64_t)(cap / (per_x / (size_t)nx));
+        t.nchunks = 0;
+        int64_t most = 0;
+        for (int64_t i0 = 0, i1; i0 < nx; i0 = i1, ++t.nchunks) {
+            i1 = chunk_end(t, i0, nx);
+            if ((i1 - i0) * i1 > most) most = (i1 - i0) * i1;
+        }
+        mat_bytes = (size_t)most * (per_x / (size_t)nx);
+    }
     t.err_off = 0;
     t.bnd_off = 256;
     t.a_off = t.bnd_off + bnd_bytes; // x differences
     t.b_off = t.a_off + (diffs ? align256((size_t)nx * ncx * d * sizeof(double)) : 0); // y differences
     t.ct_off = t.b_off + (diffs ? align256((size_t)ny_paths * ncy * d * sizeof(double)) : 0);
-    t.ws_bytes = t.ct_off + align256((size_t)chunk * per_x);
+    t.ws_bytes = t.ct_off + align256(mat_bytes);
     return t;
 }
+
+// The narrow paths' matrix is an option beside kernels that need a few MB, so it takes a quarter of the room that the
+// other matrices may (ms at 1.5 / 6 GiB: 256 x 256, L = 200, d = 8, order 0: 9.12 / 8.44, fused 27.9; 200 x 170, L = 250,
+// d = 14, order 1: 7.7 / 8.1, fused 15.2; 1000 x 1000, L = 128, d = 12, order 1: 66.4 / 63.0, fused 173).
+constexpr size_t kNarrowChunkBytes = size_t(1536) << 20;
 
 TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order)
 {
@@ -865,16 +895,18 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         const int64_t pairs = op == kOpGram ? nx * ny : nx * (nx + 1) / 2;
         const bool few = order >= 2 && pairs < (int64_t)sm_count() * 6;
         if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 : d < 8 || few)) return TcPlan{};
+        const size_t cap = tc_chunk_cap(kNarrowChunkBytes);
         // not where one x path's increments alone exceed a chunk: the fused kernels need no matrix at all
-        if ((size_t)((ncx + 3) / 4 * 4) * (size_t)((op == kOpGram ? ny : nx) * ncy) * sizeof(double) > tc_chunk_cap())
+        if ((size_t)((ncx + 3) / 4 * 4) * (size_t)((op == kOpGram ? ny : nx) * ncy) * sizeof(double) > cap)
             return TcPlan{};
         // nor where the matrix comes in chunks of too few pairs: each chunk's wavefront waits for its slowest warp, and
         // several bands want more of them (ms, fused / matrix.  One band: 128 x 128, L = 120, d = 12, order 1, chunks
         // of 384 pairs 2.75 / 2.75, 512 2.75 / 2.19; 200 x 170, L = 250, d = 14, order 1, 510 15.2 / 14.1, 1170 15.2 /
         // 9.8.  Several: 80 x 80, L = 300, d = 8, order 1, 725 4.5 / 7.1, 1450 4.5 / 4.4, 2900 4.5 / 3.6; 40 x 40,
         // L = 400, d = 8, order 3, 1600 5.7 / 5.9; symmetric, 47 paths, L = 1786, d = 11, order 1, 113 22.8 / 145).
-        const TcPlan t = mat64_layout(op, nx, ny, ncx, ncy, d, order, true);
+        const TcPlan t = mat64_layout(op, nx, ny, ncx, ncy, d, order, true, sizeof(double), cap, true);
         if (t.nchunks > 1 && pairs < t.nchunks * sm_count() * (band ? 6 : 12)) return TcPlan{};
+        return t;
     }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,
     // which forms the dot products a step ahead of the cells (256 x 256, L = 64, d = 16, order 2: 1.97 vs
@@ -958,8 +990,9 @@ int run_pairs_mat64(const TcPlan &t, int op, const void *x, const void *y, int64
                             true, in64, dx, dyv, stream)))
         return st;
     dy = reinterpret_cast<double *>(dyv);
-    for (int64_t c = 0; c < t.nchunks; ++c) {
-        const int64_t i0 = c * t.chunk, i1 = (i0 + t.chunk < nx) ? i0 + t.chunk : nx, nxc = i1 - i0;
+    for (int64_t i0 = 0, i1; i0 < nx; i0 = i1) {
+        i1 = chunk_end(t, i0, nx);
+        const int64_t nxc = i1 - i0;
         DgemmIncParams gp{};
         gp.dx = dx + i0 * d * ncx;
         gp.dy = dy;
@@ -1807,6 +1840,24 @@ size_t sigk_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t len_x, int6
     return pl.ws_bytes;
 }
 
+size_t sigk_workspace_min_size(int op, int64_t n_x, int64_t n_y, int64_t len_x, int64_t len_y, int64_t dim, int order,
+                               int dtype, int precision)
+{
+    const size_t full = sigk_workspace_size(op, n_x, n_y, len_x, len_y, dim, order, dtype, precision);
+    if (full == 0 || (op != SIGK_OP_GRAM && op != SIGK_OP_GRAM_SYM) || dim < 1 || dim >= kDgMinDim) return full;
+    const int kop = op == SIGK_OP_GRAM ? kOpGram : kOpGramSym;
+    if (kop == kOpGramSym) {
+        n_y = n_x;
+        len_y = len_x;
+    }
+    const int64_t ncx = len_x - 1, ncy = len_y - 1;
+    if (is_tc(precision) && (make_fused_plan(kop, n_x, n_y, ncx, ncy, dim, order, precision).ok ||
+                             make_tc_plan(kop, n_x, n_y, ncx, ncy, dim, order, tsize_of(precision)).ok))
+        return full;
+    if (cell_prec(precision) != SIGK_PREC_FP64 || !make_mat64_plan(kop, n_x, n_y, ncx, ncy, dim, order).ok) return full;
+    return make_plan(kop, n_x, n_y, ncx, ncy, dim, order, sizeof(double), false).ws_bytes;
+}
+
 int sigk_pairwise(const void *x, const void *y, int64_t batch, int64_t len_x, int64_t len_y, int64_t dim, int dtype,
                   int order, double static_scale, const void *scale_x, const void *scale_y, void *out, int precision,
                   void *workspace, size_t workspace_bytes, sigk_stream_t stream)
@@ -2217,14 +2268,8 @@ extern "C" int sigk_gram_noalloc(const void *x, const void *y, int64_t n_x, int6
                                  sigk_stream_t stream)
 {
     size_t need = sigk_workspace_size(SIGK_OP_GRAM, n_x, n_y, len_x, len_y, dim, order, dtype, precision);
-    if (need > kNoAllocScratchBytes && dim < kDgMinDim) { // a narrow Gram's matrix, which run_pairs does without
-        const int64_t ncx = len_x - 1, ncy = len_y - 1;
-        const bool tc = is_tc(precision) &&
-                        (make_fused_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order, precision).ok ||
-                         make_tc_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order, tsize_of(precision)).ok);
-        if (!tc && cell_prec(precision) == SIGK_PREC_FP64 && make_mat64_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order).ok)
-            need = make_plan(kOpGram, n_x, n_y, ncx, ncy, dim, order, sizeof(double), false).ws_bytes;
-    }
+    if (need > kNoAllocScratchBytes)
+        need = sigk_workspace_min_size(SIGK_OP_GRAM, n_x, n_y, len_x, len_y, dim, order, dtype, precision);
     if (need > kNoAllocScratchBytes)
         return fail(SIGK_EINVAL,
                     "sigk_gram_noalloc: this Gram needs %zu bytes of scratch; the no-allocation entry point has "

@@ -184,7 +184,17 @@ class RequestHandle:
         return None if self.t_done is None else self.t_done - self.req.arrival
 
 
-def footprint_bytes(req: GramRequest, precision: str = "fp64") -> int:
+def _workspace_bytes(req: GramRequest, precision: str, lean: bool) -> int:
+    """Workspace of the request's Gram: that of its fastest route, or (lean) the least it runs with."""
+    x = req.x
+    nx, lx, d = x.shape
+    ny, ly = (nx, lx) if req.y is None else (req.y.shape[0], req.y.shape[1])
+    op = _lib.SIGK_OP_GRAM_SYM if req.y is None else _lib.SIGK_OP_GRAM
+    size = _lib.lib().sigk_workspace_min_size if lean else _lib.lib().sigk_workspace_size
+    return size(op, nx, ny, lx, ly, d, req.order, _k._dtype_code(x), _k._PREC[precision])
+
+
+def footprint_bytes(req: GramRequest, precision: str = "fp64", lean: bool = False) -> int:
     """Device bytes a request holds while in flight (paths, result, workspace, robust scratch)."""
     x = req.x
     y = x if req.y is None else req.y
@@ -194,8 +204,7 @@ def footprint_bytes(req: GramRequest, precision: str = "fp64") -> int:
     prec = _k._PREC[precision]
     dt = _k._dtype_code(x)
     sym = req.y is None
-    op = _lib.SIGK_OP_GRAM_SYM if sym else _lib.SIGK_OP_GRAM
-    ws = _lib.lib().sigk_workspace_size(op, nx, ny, lx, ly, d, req.order, dt, prec)
+    ws = _workspace_bytes(req, precision, lean)
     # resident paths are held by the server's store, not by the request
     paths = (0 if _resident(x) else x.numel() * es) + (0 if sym or _resident(y) else y.numel() * es)
     total = paths + nx * ny * es + ws
@@ -308,13 +317,13 @@ def request_cells(req: GramRequest) -> int:
 
 
 def _solve_on_stream(req: GramRequest, precision: str, device, stream, chunk_cells: int = 0, staging=None,
-                     use_store: bool = True):
+                     use_store: bool = True, workspace_limit: Optional[int] = None):
     """Enqueue copy-in, solve and copy-out of one request on `stream`.
     Returns (pinned host result, tensors to keep alive until the event).
     chunk_cells > 0 splits a large (non-symmetric or robust) Gram into row
     blocks of about that many cells, one launch each.  use_store=False treats
     a PathSet operand like a host tensor (copied in, scales recomputed): the
-    per-request baseline."""
+    per-request baseline.  workspace_limit: scratch that the Gram was admitted with."""
     with torch.cuda.stream(stream):
         x = _on_device(req.x, device, use_host=not use_store)
         y = None if req.y is None else _on_device(req.y, device, use_host=not use_store)
@@ -322,6 +331,7 @@ def _solve_on_stream(req: GramRequest, precision: str, device, stream, chunk_cel
         if req.kind not in ("gram", "robust"):
             raise ValueError(f"unknown request kind {req.kind!r}")
         k = _k.SigPDE(lin, req.order, precision=precision)
+        k._workspace_limit = workspace_limit
         sx = sy = None
         if req.kind == "robust":
             rk = _k.RobustSigPDE(lin, req.order, precision=precision)
@@ -563,6 +573,11 @@ class GramServer:
                 h._finish(error=e)
                 continue
             budget = self.budget - self._store_bytes
+            lean = False
+            if self._used + need > budget:  # the least workspace, if that lets the request run now or at all
+                least = footprint_bytes(h.req, self.precision, lean=True)
+                lean = least < need and (need > budget or self._used + least <= budget)
+                need = least if lean else need
             if need > budget:
                 self._pending.remove(h)
                 h._finish(error=MemoryError(f"request {h.req.rid} needs {need} bytes, budget is {budget}"))
@@ -575,7 +590,8 @@ class GramServer:
             try:
                 with torch.cuda.device(self.device):
                     out_host, keep = _solve_on_stream(h.req, self.precision, self.device, stream,
-                                                      self.chunk_cells, self._staging_for(stream))
+                                                      self.chunk_cells, self._staging_for(stream),
+                                                      workspace_limit=_workspace_bytes(h.req, self.precision, lean))
                     ev = torch.cuda.Event()
                     ev.record(stream)
             except Exception as e:

@@ -71,11 +71,22 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def _workspace(op, nx, ny, lx, ly, d, order, dtype_code, prec, device):
-    n = _lib.lib().sigk_workspace_size(op, nx, ny, lx, ly, d, order, dtype_code, prec)
+def _workspace(op, nx, ny, lx, ly, d, order, dtype_code, prec, device, limit=None):
+    """Scratch of one call: sigk_workspace_size bytes, or the least that the call runs with where that is more than
+    `limit` or than the device has left (a narrow float64 Gram then takes its fused kernels; the same values)."""
+    shape = (op, nx, ny, lx, ly, d, order, dtype_code, prec)
+    n = _lib.lib().sigk_workspace_size(*shape)
     if n == 0:
         return None, 0
-    return torch.empty(n, dtype=torch.uint8, device=device), n
+    if limit is not None and n > limit:
+        n = _lib.lib().sigk_workspace_min_size(*shape)
+    try:
+        return torch.empty(n, dtype=torch.uint8, device=device), n
+    except torch.OutOfMemoryError:
+        least = _lib.lib().sigk_workspace_min_size(*shape)
+        if least >= n:
+            raise
+    return torch.empty(least, dtype=torch.uint8, device=device), least
 
 
 def _broadcast_scale(s, n, like: torch.Tensor):
@@ -406,6 +417,8 @@ def _batches(n, size):
 class SigPDE:
     """Untruncated signature kernel by the Goursat PDE (sigpde/torch/kernel.py:26-171)."""
 
+    _workspace_limit = None  # bytes of scratch of a linear-kernel Gram, where it has a choice (see _workspace)
+
     def __init__(self, static_kernel, dyadic_order=0, precision="fp64"):
         if precision not in _PREC:
             raise ValueError(f"precision must be one of {sorted(_PREC)}")
@@ -495,7 +508,7 @@ class SigPDE:
                 x = x.contiguous()
                 y = y.contiguous()
                 ws, nws = _workspace(_lib.SIGK_OP_GRAM, Nx, Ny, x.shape[1], y.shape[1], x.shape[2],
-                                     self.dyadic_order, dt, prec, x.device)
+                                     self.dyadic_order, dt, prec, x.device, self._workspace_limit)
                 _lib.call("sigk_gram", _ptr(x), _ptr(y), Nx, Ny, x.shape[1], y.shape[1], x.shape[2], dt,
                           self.dyadic_order, float(self.static_kernel.scale), _ptr(sx), _ptr(sy), _ptr(result),
                           prec, _ptr(ws), nws, _stream())
@@ -524,7 +537,7 @@ class SigPDE:
             if _is_fused_linear(self.static_kernel):
                 x = x.contiguous()
                 ws, nws = _workspace(_lib.SIGK_OP_GRAM_SYM, N, N, x.shape[1], x.shape[1], x.shape[2],
-                                     self.dyadic_order, dt, prec, x.device)
+                                     self.dyadic_order, dt, prec, x.device, self._workspace_limit)
                 _lib.call("sigk_gram_sym", _ptr(x), N, x.shape[1], x.shape[2], dt, self.dyadic_order,
                           float(self.static_kernel.scale), _ptr(sx), _ptr(result), prec, _ptr(ws), nws, _stream())
                 return result

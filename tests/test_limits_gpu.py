@@ -40,3 +40,48 @@ def test_few_pairs_infinite_increments(sig, oracle, lx, ly, order, where, monkey
         np.testing.assert_array_equal(a, b)
     if (lx, ly, order, where) == (2, 2, 0, "overflow"):
         assert np.isinf(want[0]).any()
+
+
+def _narrow(oracle):
+    """A Gram whose increment matrix takes 1.5 GiB and whose differences take a few MB."""
+    x, y = oracle.brownian(256, 200, 8, 11), oracle.brownian(200, 200, 8, 12)
+    return cuda(x, torch.float32), cuda(y, torch.float32)
+
+
+def test_narrow_gram_runs_in_the_memory_that_is_left(sig, oracle):
+    """A process limited to less than the matrix: the fused kernels, with the same values."""
+    X, Y = _narrow(oracle)
+    k = sig.SigPDE(sig.kernels.LinearKernel(), 0)
+    want = [k.gram(X, Y), k.gram(X)]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (256 << 20)) / total)
+        torch.cuda.reset_peak_memory_stats()
+        got = [k.gram(X, Y), k.gram(X)]
+        torch.cuda.synchronize()
+        assert torch.cuda.max_memory_allocated() < 512 << 20
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("budget_mb", [64, 16384])
+def test_server_admits_narrow_grams_with_their_least_workspace(sig, oracle, budget_mb):
+    """Requests whose matrix exceeds the server's budget run, together, with the fused kernels."""
+    from sigpde_b200 import serving
+    X, Y = _narrow(oracle)
+    want = host(sig.SigPDE(sig.kernels.LinearKernel(), 0).gram(X, Y))
+    req = serving.GramRequest(x=X.cpu(), y=Y.cpu(), order=0)
+    least = serving.footprint_bytes(req, lean=True)
+    assert least < 32 << 20 < 1 << 30 < serving.footprint_bytes(req)
+    server = serving.GramServer(hbm_budget_bytes=budget_mb << 20, max_inflight=4)
+    with server:
+        handles = [server.submit(serving.GramRequest(x=X.cpu(), y=Y.cpu(), order=0)) for _ in range(4)]
+        for h in handles:
+            np.testing.assert_array_equal(h.wait(60).double().numpy(), want)
+    assert server.peak_bytes <= budget_mb << 20
+    if budget_mb == 64:
+        assert server.peak_inflight >= 2

@@ -37,3 +37,22 @@ def test_no_matrix_in_chunks_of_few_pairs(lib, monkeypatch, op, nx, ny, lx, ly, 
 def test_matrix_where_chunks_hold_enough_pairs(lib, monkeypatch, op, nx, ny, lx, ly, d, order):
     default, fused = sizes(lib, monkeypatch, op, nx, ny, lx, ly, d, order)
     assert default > fused
+
+
+@pytest.mark.parametrize("op,nx,ny,lx,ly,d,order", [
+    (GRAM, 256, 256, 200, 200, 8, 0), (GRAM, 1000, 1000, 128, 128, 12, 1), (SYM, 300, 300, 200, 200, 10, 0),
+    (GRAM, 80, 80, 300, 300, 8, 1), (GRAM, 400, 333, 256, 200, 15, 1), (SYM, 2000, 2000, 60, 60, 15, 1),
+    (GRAM, 64, 64, 1000, 1000, 8, 2)])
+def test_matrix_stays_an_option_of_bounded_size(lib, monkeypatch, op, nx, ny, lx, ly, d, order):
+    """At most 1.5 GiB beside the differences; the least workspace is the fused route's."""
+    default, fused = sizes(lib, monkeypatch, op, nx, ny, lx, ly, d, order)
+    assert default <= (1536 << 20) + 2 * fused + 1024
+    assert lib.sigk_workspace_min_size(op, nx, ny, lx, ly, d, order, F32, FP64) == fused
+
+
+def test_least_workspace_of_other_calls_is_the_whole(lib):
+    for op in (0, 1, 2, 3):
+        for prec in (0, 1, 2, 3):
+            for d in (0, 4, 16, 40):
+                full = lib.sigk_workspace_size(op, 20, 20, 30, 30, d, 1, F32, prec)
+                assert lib.sigk_workspace_min_size(op, 20, 20, 30, 30, d, 1, F32, prec) == full
