@@ -206,11 +206,15 @@ __device__ __forceinline__ T pick_row(const T (&left)[R], int rstar)
     return v;
 }
 
-// The D differences of column c (`at`: the path's values + G c) of a path of nc columns.
-template <typename T, int D>
+// The D differences of column c (`at`: the path's values + G c) of a path of nc columns.  SPLIT: one value a load,
+// where the register pairs of 16-byte loads leave the allocation no room.
+template <typename T, int D, bool SPLIT = false>
 __device__ __forceinline__ void stream_load_row(const T *at, int64_t nc, T (&v)[D])
 {
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (sizeof(T) == 8 && SPLIT) {
+#pragma unroll
+        for (int k = 0; k < D; ++k) v[k] = at[(k / 2) * 2 * nc + k % 2];
+    } else if constexpr (sizeof(T) == 8) {
 #pragma unroll
         for (int h = 0; h < D / 2; ++h) {
             const double2 t = reinterpret_cast<const double2 *>(at)[h * nc];
@@ -400,11 +404,11 @@ __device__ __forceinline__ Dbl2 stencil_cell<Dbl2>(Dbl2 k00, Dbl2 k01, Dbl2 k10,
 // when it has another x path, the dot products formed with the old dx are
 // discarded and redone after the dx reload (rare: a run moves to a new x path
 // at most a few times).
-template <typename T, int D, int RC>
+template <typename T, int D, int RC, bool SPLIT = false>
 __device__ __forceinline__ void stream_dot(const T (&dx)[RC][D], const T *dyr, int64_t ncy, T (&cc)[RC])
 {
     T dy[D];
-    stream_load_row<T, D>(dyr, ncy, dy);
+    stream_load_row<T, D, SPLIT>(dyr, ncy, dy);
 #pragma unroll
     for (int rc = 0; rc < RC; ++rc) cc[rc] = T(0);
 #pragma unroll
@@ -413,7 +417,7 @@ __device__ __forceinline__ void stream_dot(const T (&dx)[RC][D], const T *dyr, i
         for (int rc = 0; rc < RC; ++rc) cc[rc] = fma(dx[rc][kk], dy[kk], cc[rc]);
 }
 
-template <typename T, int D, int RC>
+template <typename T, int D, int RC, bool SPLIT = false>
 __device__ __forceinline__ void stream_load_dx(const T *dX, int64_t xi, int ncx, int ci0, T (&dx)[RC][D])
 {
     constexpr int G = sizeof(T) == 8 ? 2 : 1;
@@ -422,7 +426,7 @@ __device__ __forceinline__ void stream_load_dx(const T *dX, int64_t xi, int ncx,
     for (int rc = 0; rc < RC; ++rc) {
         const int ci = ci0 + (RC > 1 ? rc : 0);
         if (ci < ncx) {
-            stream_load_row<T, D>(src + ci * G, ncx, dx[rc]);
+            stream_load_row<T, D, SPLIT>(src + ci * G, ncx, dx[rc]);
         } else {
 #pragma unroll
             for (int kk = 0; kk < D; ++kk) dx[rc][kk] = T(0);
@@ -544,6 +548,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
     const int64_t first = idle ? p.nitems - 1 : pipe * p.per_warp;
     const int cnt = idle ? 0 : (int)((p.nitems - first) < p.per_warp ? (p.nitems - first) : p.per_warp);
     const int cnt_max = (int)((p.nitems - wfirst) < p.per_warp ? (p.nitems - wfirst) : p.per_warp);
+    // 16 coarse rows a lane take 250 of 255 registers; with 16-byte loads 252 bytes of them spilled (5 x 2 paths,
+    // L = 472 / 717, d = 2, order 0: 521 us, 383 without)
+    constexpr bool SPLIT = RC >= 16;
     const double *dX = reinterpret_cast<const double *>(p.dx);
     const double *dY = reinterpret_cast<const double *>(p.dy);
     const int ncx = (int)p.ncx, ncy = (int)p.ncy;
@@ -569,10 +576,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
     dypb = ndypb;
     double dx[RC][D];
     int64_t cur_x = nxi;
-    stream_load_dx<double, D, RC>(dX, nxi, ncx, ci0, dx);
+    stream_load_dx<double, D, RC, SPLIT>(dX, nxi, ncx, ci0, dx);
     double cca[RC], ccb[RC]; // increments of this lane's next step, entries a and b
-    stream_dot<double, D, RC>(dx, dypa, ncy, cca);
-    stream_dot<double, D, RC>(dx, dypb, ncy, ccb);
+    stream_dot<double, D, RC, SPLIT>(dx, dypa, ncy, cca);
+    stream_dot<double, D, RC, SPLIT>(dx, dypb, ncy, ccb);
 
     Dbl2 left[R];
 #pragma unroll
@@ -604,9 +611,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
                 dypb = ndypb;
                 if (xi != cur_x) { // the ahead increments used the previous x path's dx
                     cur_x = xi;
-                    stream_load_dx<double, D, RC>(dX, xi, ncx, ci0, dx);
-                    stream_dot<double, D, RC>(dx, dypa, ncy, cca);
-                    stream_dot<double, D, RC>(dx, dypb, ncy, ccb);
+                    stream_load_dx<double, D, RC, SPLIT>(dX, xi, ncx, ci0, dx);
+                    stream_dot<double, D, RC, SPLIT>(dx, dypa, ncy, cca);
+                    stream_dot<double, D, RC, SPLIT>(dx, dypb, ncy, ccb);
                 }
                 if (k + 1 < cnt) {
                     nya += 2;
@@ -626,8 +633,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 2) stream_reg_dual_kernel
             for (int rc = 0; rc < RC; ++rc) stencil_coefs(Dbl2{cca[rc], ccb[rc]}, A[rc], B[rc]);
             const int qn = (q + 1 == nsteps) ? 0 : q + 1;
             const int cjn = (O <= 3) ? qn : ((qn * C) >> p.order);
-            stream_dot<double, D, RC>(dx, ((qn == 0) ? ndypa : dypa) + (int64_t)cjn * 2, ncy, cca);
-            stream_dot<double, D, RC>(dx, ((qn == 0) ? ndypb : dypb) + (int64_t)cjn * 2, ncy, ccb);
+            stream_dot<double, D, RC, SPLIT>(dx, ((qn == 0) ? ndypa : dypa) + (int64_t)cjn * 2, ncy, cca);
+            stream_dot<double, D, RC, SPLIT>(dx, ((qn == 0) ? ndypb : dypb) + (int64_t)cjn * 2, ncy, ccb);
             stream_block<Dbl2, R, O>(left, top, corner, A, B, bot);
             if (q == nsteps - 1 && lane == lstar) {
                 const Dbl2 v = pick_row(left, rstar);
