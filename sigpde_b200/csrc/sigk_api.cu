@@ -882,30 +882,42 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
     if (d < kDgMinDim) {
         // Below that, where the fused kernels would read each lane's dx from shared memory: a streaming shape whose
         // dx tile does not fit registers (ms, fused / matrix: 80 x 80, L = 200, order 0, d = 8: 2.04 / 0.90, with the
-        // tile in registers at d = 4: 0.41 / 0.83; 128 x 128, L = 120, order 1, d = 12: 2.51 / 0.97), and several
-        // bands from d = 8 on (80 x 80, L = 300, order 1: 4.55 / 3.32 at d = 8, 2.91 / 3.18 at d = 4).  From order 2 on
-        // the increments are few beside the cells, and a warp with one pair has latencies to hide them in: with fewer
-        // than 6 pairs an SM the matrix only adds its own time (L = 239 / 154, d = 10, order 2: 588 pairs 389 / 437 us,
-        // 960 pairs 505 / 478).
+        // tile in registers at d = 4: 0.41 / 0.83; 128 x 128, L = 120, order 1, d = 12: 2.51 / 0.97; not at d = 3: 38 x 22,
+        // L = 371 / 310, order 0: 0.36 / 0.46), and several
+        // bands from d = 8 on (80 x 80, L = 300, order 1: 4.55 / 3.39 at d = 8, 2.91 / 3.18 at d = 4).
         const int64_t n = ncx << order, m = ncy << order;
         const int Rs = pick_rows(n), C = order >= 4 ? 8 : 1 << order;
         int Dp = 2;
         while (Dp < d) Dp <<= 1;
-        const bool band = n <= 32 * Rs, regs = rows_per_coarse_lane(Rs, order) * Dp <= 32;
-        const int64_t pairs = op == kOpGram ? nx * ny : nx * (nx + 1) / 2;
-        const bool few = order >= 2 && pairs < (int64_t)sm_count() * 6;
-        if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 : d < 8 || few)) return TcPlan{};
+        const bool band = n <= 32 * Rs, regs = rows_per_coarse_lane(Rs, order) * Dp <= 32, sym = op == kOpGramSym;
+        if (env_flag("SIGK_NO_REG_DX") || (band ? regs || m / C < 32 || d < 4 : d < 8)) return TcPlan{};
         const size_t cap = tc_chunk_cap(kNarrowChunkBytes);
         // not where one x path's increments alone exceed a chunk: the fused kernels need no matrix at all
-        if ((size_t)((ncx + 3) / 4 * 4) * (size_t)((op == kOpGram ? ny : nx) * ncy) * sizeof(double) > cap)
-            return TcPlan{};
-        // nor where the matrix comes in chunks of too few pairs: each chunk's wavefront waits for its slowest warp, and
-        // several bands want more of them (ms, fused / matrix.  One band: 128 x 128, L = 120, d = 12, order 1, chunks
-        // of 384 pairs 2.75 / 2.75, 512 2.75 / 2.19; 200 x 170, L = 250, d = 14, order 1, 510 15.2 / 14.1, 1170 15.2 /
-        // 9.8.  Several: 80 x 80, L = 300, d = 8, order 1, 725 4.5 / 7.1, 1450 4.5 / 4.4, 2900 4.5 / 3.6; 40 x 40,
-        // L = 400, d = 8, order 3, 1600 5.7 / 5.9; symmetric, 47 paths, L = 1786, d = 11, order 1, 113 22.8 / 145).
+        if ((size_t)((ncx + 3) / 4 * 4) * (size_t)((sym ? nx : ny) * ncy) * sizeof(double) > cap) return TcPlan{};
         const TcPlan t = mat64_layout(op, nx, ny, ncx, ncy, d, order, true, sizeof(double), cap, true);
-        if (t.nchunks > 1 && pairs < t.nchunks * sm_count() * (band ? 6 : 12)) return TcPlan{};
+        const int64_t pairs = sym ? nx * (nx + 1) / 2 : nx * ny, sms = sm_count();
+        const bool multi = t.nchunks > 1;
+        if (!band) {
+            // A warp solves a pair of several bands, and one with few pairs beside it has latencies to hide the
+            // increments in; from order 2 on they are few beside the cells (us, fused / matrix: 24 x 12, L = 765 / 580,
+            // d = 8, order 0 1823 / 2232; symmetric, 14 paths, L = 667, d = 11, order 0 2602 / 2504; 34 x 34, L = 153 /
+            // 173, d = 8, order 2 452 / 491, 60 x 60 symmetric, L = 200 845 / 773; order 2, L = 239 / 154, d = 10: 588
+            // pairs 389 / 437, 960 505 / 478).  At few dimensions they are worth no matrix at order 3, and at order 2
+            // none in several chunks (d = 8: 40 x 40, L = 150, order 3 1114 / 1159; 90 x 90, L = 300, order 2 6393 /
+            // 6919; symmetric, 120 paths, L = 200, order 2 2612 / 2908; but 100 x 90, L = 180 / 200, d = 9, order 2 3520 /
+            // 3200; symmetric, 120 paths, L = 80, order 4 4392 / 4048).
+            const int least = order >= 2 ? (d < 11 ? 12 : 6) : d < 10 ? 6 : 0;
+            if (pairs < sms * least || (order == 3 && d < 11) || (order == 2 && multi && d < (sym ? 11 : 9)))
+                return TcPlan{};
+        }
+        // Nor where the matrix comes in chunks of too few pairs: each chunk's wavefront waits for its slowest warp, and
+        // more rows a lane or several bands want more of them (ms, fused / matrix.  One band: 128 x 128, L = 120,
+        // d = 12, order 1, chunks of 384 pairs 2.75 / 2.75, 512 2.75 / 2.19; 200 x 170, L = 250, d = 14, order 1, 1170
+        // 15.2 / 9.8; 93 x 114, L = 377 / 420, d = 5, order 0, 1178 5.1 / 6.3.  Several: 80 x 80, L = 300, d = 8, order 1,
+        // 725 4.5 / 7.1, 1450 4.5 / 4.4, 2133 4.5 / 3.4; symmetric, 47 paths, L = 1786, d = 11, order 1, 113 22.8 / 145;
+        // symmetric, 120 paths, L = 250, d = 11, order 3, 2420 9.9 / 10.8).
+        const int least = band && Rs < 16 ? 6 : sym && !band && order >= 2 ? 24 : 12;
+        if (multi && pairs < t.nchunks * sms * least) return TcPlan{};
         return t;
     }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,
