@@ -1598,8 +1598,9 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
     if (precision == SIGK_PREC_FP64) {
         q = make_pair_wave_plan(op, nx, ny, lx - 1, ly - 1, d, order);
         TcPlan t = make_mat64_plan(op, nx, ny, lx - 1, ly - 1, d, order);
-        // the narrow paths' matrix is a choice: a smaller workspace that holds the fused route's differences takes that
-        if (t.ok && d < kDgMinDim && ws && ws_bytes < t.ws_bytes &&
+        // the narrow paths' matrix is a choice: a workspace that is smaller or less aligned than it needs, but serves
+        // the fused route, takes that
+        if (t.ok && d < kDgMinDim && ws && (ws_bytes < t.ws_bytes || ((uintptr_t)ws & 255) != 0) &&
             ws_bytes >= make_plan(op, nx, ny, lx - 1, ly - 1, d, order, sizeof(double), false).ws_bytes)
             t.ok = false;
         if (t.ok) {

@@ -85,3 +85,28 @@ def test_server_admits_narrow_grams_with_their_least_workspace(sig, oracle, budg
     assert server.peak_bytes <= budget_mb << 20
     if budget_mb == 64:
         assert server.peak_inflight >= 2
+
+
+@pytest.mark.parametrize("op,dim", [("gram", 8), ("gram", 12), ("sym", 8)])
+def test_narrow_grams_take_a_16_byte_aligned_workspace(sig, oracle, op, dim, monkeypatch):
+    """The C entry points accept 16-byte alignment wherever the fused kernels serve, whatever the size given."""
+    from sigpde_b200 import _lib
+    monkeypatch.setenv("SIGK_NO_PAIR_WAVE", "1")
+    lib, n, L = _lib.lib(), 40, 200
+    X = cuda(oracle.brownian(n, L, dim, 21), torch.float32)
+    stream = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for shift in (0, 16, 128):
+        size = lib.sigk_workspace_size(2 if op == "sym" else 1, n, n, L, L, dim, 0, 0, 0)
+        assert size > lib.sigk_workspace_min_size(2 if op == "sym" else 1, n, n, L, L, dim, 0, 0, 0)
+        ws = torch.empty(size + 256, dtype=torch.uint8, device="cuda")
+        out = torch.full((n, n), float("nan"), device="cuda")
+        if op == "sym":
+            st = lib.sigk_gram_sym(X.data_ptr(), n, L, dim, 0, 0, 1.0, None, out.data_ptr(), 0, ws.data_ptr() + shift,
+                                   size, stream)
+        else:
+            st = lib.sigk_gram(X.data_ptr(), X.data_ptr(), n, n, L, L, dim, 0, 0, 1.0, None, None, out.data_ptr(), 0,
+                               ws.data_ptr() + shift, size, stream)
+        assert st == 0, _lib.last_error()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
