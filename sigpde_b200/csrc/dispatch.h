@@ -57,6 +57,8 @@ struct NormKernel {
 };
 // smem_tile, smem_bnd: increments, bottom rows in shared memory (a tile there only with the rows)
 NormKernel get_norm_kernel(int R, int O, bool smem_tile, bool smem_bnd);
+// the same, one path a warp (norm_warp.cuh); mode: kNormDelta, kNormGiven or kNormTile; in64: the given increments' type
+NormFn get_norm_warp_kernel(bool in64, int mode, int R, int O);
 // few pairs, one CTA each (pair_wave.cuh): R in {2,4,8} rows a lane; fn null where not built
 struct PairWaveKernel {
     PairWaveFn fn;

@@ -36,7 +36,9 @@ struct NormParams {
     int col0;            // tile column of coarse column 0 (1: a zero column before it)
     int64_t tile;        // values of a tile
     double *tiles;       // one tile a CTA, where it is not in shared memory
-    double *bnd;         // C ones and nw rows a CTA, where they are not in shared memory
+    double *bnd;         // C ones and nw rows a CTA, where they are not in shared memory; norm_warp_kernel: a row a warp
+    int64_t bnd_stride;  // norm_warp_kernel: values of a row, and of a warp's shared memory
+    int64_t smem_values;
     double *knorm;       // builtin: output (may be null); external: input
     const double *fnorm; // null: builtin f(s) = 2 - 1/(1 + log s)
     double tol;
@@ -331,7 +333,7 @@ __device__ __forceinline__ double norm_solve(const P &p, const double *tile, dou
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
                             const double l = left[r], a = A[cc][NS::rc_of(r)], bb = B[cc][NS::rc_of(r)];
-                            up = CHAIN ? fma(up, a, fma(l, a, -(dg * bb))) : stencil_cell(dg, up, l, a, bb);
+                            up = CHAIN ? stencil_chain(dg, up, l, a, bb) : stencil_cell(dg, up, l, a, bb);
                             dg = l;
                             left[r] = up;
                         }

@@ -22,6 +22,7 @@
 #include "ragged.cuh"
 #include "stream.cuh"
 #include "tc.cuh"
+#include "norm_warp.cuh"
 #include "pair_wave.cuh"
 #include "second_diff.cuh"
 #include "dgemm_inc.cuh"
@@ -1722,6 +1723,12 @@ int run_pairs(int op, const void *x, const void *y, int64_t nx, int64_t ny, int6
 // tile and the bands' bottom rows live, and the workspace (float64 differences |
 // tiles | rows).
 struct NormPlan {
+    double cost; // cycles, up to a factor
+    bool capped; // fewer CTAs than fit, for their tiles
+    bool warp;   // one path a warp
+    int mode;    // of that: where the increments come from
+    int64_t bnd_stride;
+    size_t smem_warp;
     NormKernel k;
     int R, O, nbands, nw, nsteps, pitch, col0, threads;
     int64_t tile; // values
@@ -1733,7 +1740,47 @@ struct NormPlan {
 constexpr size_t kNormSmemBytes = 226 * 1024;      // of the 227 KB a CTA may have (its static word)
 constexpr size_t kNormTileCap = size_t(1) << 30;   // of all resident CTAs' tiles in the workspace
 
-NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
+// One path a warp (norm_warp.cuh): workspace boundary rows | differences.  Its cost in the unit of norm_cta_plan, for
+// paths whose increments are formed as the wavefront goes: a warp's steps of a solve, each at its issue slots times the
+// warps that share a sub-partition, or at a lone warp's slots and latencies.  Fitted to 430 shapes, n = 8 - 20000,
+// L = 80 - 4000, d = 1 - 64, orders 0 - 4 (given increments: 21): the chosen route's time is 1.014 of the better one's on
+// average, 1.33 of this one's at most.
+NormPlan norm_warp_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
+{
+    NormPlan q{};
+    q.warp = true;
+    const int64_t pitch = nc | 1; // odd: neighbouring lanes' rows fall in different banks
+    const size_t tile = (size_t)nc * (size_t)pitch * sizeof(double);
+    q.mode = from_inc ? kNormGiven : tile <= kNormWarpTileBytes ? kNormTile : kNormDelta;
+    // only the difference mode stages rows of dx (and may shrink R to fit them)
+    const Plan pl = make_plan(SIGK_OP_NORMALIZE, n, n, nc, nc, d, order, 8, q.mode != kNormDelta);
+    q.R = pl.R;
+    q.O = pl.O;
+    q.nbands = pl.nbands;
+    q.bnd_stride = pl.bnd_stride;
+    q.pitch = (int)pitch;
+    q.smem_warp = q.mode == kNormTile ? tile : q.mode == kNormDelta ? pl.stage_bytes_per_warp : 0;
+    q.dx_off = align256(pl.ws_bytes);
+    q.ws_bytes = q.dx_off + (from_inc ? 0 : align256((size_t)n * (size_t)d * (size_t)nc * sizeof(double)));
+
+    const int sms = sm_count(), C = order >= 4 ? 8 : 1 << order, rc = rows_per_coarse_lane(q.R, order);
+    double warps = q.R == 16 ? 12 : 16; // an SM
+    if (q.smem_warp) {
+        const double fit = 4 * (double)((227 * 1024) / (q.smem_warp * kWarpsPerBlock + 1024));
+        if (fit < warps) warps = fit;
+    }
+    const double per_sm = (double)((n + sms - 1) / sms), together = per_sm < warps ? per_sm : warps;
+    const double steps = (double)q.nbands * (double)((nc << order) / C + 31);
+    const double incs = from_inc ? 4.0 * rc : q.smem_warp ? 4.9 * d * (rc + 2.1) : 30.5 * d * (rc + 1.0);
+    const double slots = 1.26 * (6.0 * q.R * C + 10.0 * rc + incs + 120.0);
+    const double alone = slots + (from_inc ? 500.0 + 75.0 * rc : q.smem_warp ? 225.0 + 12.0 * d : 225.0);
+    const double shared = slots * together / 4.0, rounds = (double)n / (sms * warps);
+    q.cost = (rounds > 1.0 ? rounds : 1.0) * steps * (shared > alone ? shared : alone);
+    return q;
+}
+
+// One path a CTA (norm_wave.cuh).
+NormPlan norm_cta_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
 {
     const int sms = sm_count();
     const int64_t nref = nc << order;
@@ -1780,13 +1827,27 @@ NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
             const double steps = (double)((q.nbands + q.nw - 1) / q.nw) * (q.nsteps + 31 + (q.nw - 1) * kNormLag);
             const double slots = 1.15 * (6.0 * R * q.k.cols + (smem_tile ? 10.0 : 22.0) * q.k.rc * q.k.ccols + 50.0);
             const double shared = slots * (double)((together * q.nw + 3) / 4), alone = slots + (smem_tile ? 130.0 : 230.0);
-            const double cost = (double)((paths + together - 1) / together) * steps * (shared > alone ? shared : alone);
-            if (best_cost >= 0 && cost >= best_cost) continue;
+            double cost = (double)((paths + together - 1) / together) * steps * (shared > alone ? shared : alone);
             q.grid = n < sms * res ? n : sms * res;
+            const bool capped = !smem_tile && (size_t)q.grid * tile > kNormTileCap;
+            if (capped) q.grid = (int64_t)(kNormTileCap / tile) > 0 ? (int64_t)(kNormTileCap / tile) : 1;
+            // the same without whole rounds, and with the CTAs that there are
+            const double ctas = n > q.grid ? (double)q.grid / sms : (double)((q.grid + sms - 1) / sms);
+            const double busy = slots * (ctas * q.nw > 4.0 ? ctas * q.nw / 4.0 : 1.0);
+            double solve = steps * (busy > alone ? busy : alone);
             if (!smem_tile) {
-                const int64_t fit = (int64_t)(kNormTileCap / tile), most = fit > 0 ? fit : 1;
-                if (q.grid > most) q.grid = most;
+                // a tile's columns reach an SM at 12 bytes a cycle, and all of them at 1300 from memory: tiles that the L2
+                // does not hold, from 40 MB on in part, from 80 MB on all
+                const double tiles = (double)q.grid * (double)tile, over = tiles / 40e6 - 1.0;
+                const double l2 = ctas * (double)tile / 12.0;
+                const double hbm = tiles * (over < 0.0 ? 0.0 : over > 1.0 ? 1.0 : over) / 1300.0;
+                if (solve < l2) solve = l2;
+                if (solve < hbm) solve = hbm;
             }
+            q.cost = (n > q.grid ? (double)n / (double)q.grid : 1.0) * solve;
+            if (capped) cost = q.cost;
+            q.capped = capped;
+            if (best_cost >= 0 && cost >= best_cost) continue;
             q.dx_off = 0;
             q.tile_off = from_inc ? 0 : align256((size_t)n * (size_t)d * (size_t)nc * sizeof(double));
             q.bnd_off = q.tile_off + (smem_tile ? 0 : align256((size_t)q.grid * tile));
@@ -1796,6 +1857,36 @@ NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
         }
     }
     return best;
+}
+
+// A path a CTA, or a path a warp where there are more paths than CTAs make good use of (SIGK_NORM_WARP=1: a warp always,
+// 0: never).
+NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
+{
+    const char *force = getenv("SIGK_NORM_WARP");
+    const NormPlan w = norm_warp_plan(n, nc, d, order, from_inc);
+    if (force && force[0]) return force[0] != '0' ? w : norm_cta_plan(n, nc, d, order, from_inc);
+    // a CTA's tile alone exceeds what all of them may take: only a path a warp needs no storage of nc squared
+    if ((size_t)nc * (size_t)nc * sizeof(double) > kNormTileCap) return w;
+    if (w.mode == kNormTile) {
+        // Increments in shared memory either way.  A path of one to a few bands leaves most of a CTA's threads without
+        // work, which costs from 16 paths an SM on (us, CTA / warp, order 0, 1, 2: n = 13000 - 16000, L = 16 - 21
+        // 1051 / 761, 1009 / 751, 1064 / 760; n = 2500 - 2900, L = 14 - 16 145 / 145, 153 / 145, 234 / 188; n = 1200 -
+        // 1300, L = 22 - 28 189 / 267, 222 / 214, 222 / 214).  Fewer points than that leave the root-find's own
+        // arithmetic, at 32 lanes a path (n = 18771, L = 5, order 1 515 / 569); more, and order 3, a CTA's bands.
+        const int64_t per_sm = n / sm_count();
+        const bool many = per_sm >= (order == 0 ? 16 : 12) && nc >= 9 && nc <= 32;
+        const bool most = per_sm >= 64 && nc > 32 && nc <= (order == 0 ? 40 : 48);
+        return (order <= 2 && many) || (order <= 1 && most)
+                   ? w
+                   : norm_cta_plan(n, nc, d, order, from_inc);
+    }
+    // The rest: the cheaper one, and this one in doubt where the CTAs' tiles are at their cap, since it needs none (ms,
+    // CTA / warp: 512 paths, L = 4000, d = 3, order 0, eight tiles at a time, 2776 / 220; 64 of them 357 / 218; 1052,
+    // L = 727, d = 2, order 1 19.3 / 14.2; 476, L = 2335, d = 32, order 1 942 / 1308; 24, L = 220, d = 8, order 1
+    // 0.53 / 4.1).
+    const NormPlan c = norm_cta_plan(n, nc, d, order, from_inc);
+    return w.cost < (c.capped ? 1.6 : 0.95) * c.cost ? w : c;
 }
 
 } // namespace
@@ -2124,6 +2215,13 @@ static int normalize_impl(const void *x, const void *inc, int64_t n, int64_t nc,
     p.maxit = maxit;
     p.lam = lam;
     p.iters = iters;
+    if (q.warp) {
+        p.bnd = q.nbands > 1 ? reinterpret_cast<double *>(wsb) : nullptr;
+        p.bnd_stride = q.bnd_stride;
+        p.smem_values = (int64_t)(q.smem_warp / sizeof(double));
+        return launch(get_norm_warp_kernel(dtype == SIGK_F64, q.mode, q.R, q.O), p, n, q.smem_warp * kWarpsPerBlock,
+                      stream);
+    }
     int nb = 0; // opts the kernel in to its shared memory
     if ((st = blocks_per_sm((const void *)q.k.fn, q.smem, &nb, q.threads))) return st;
     q.k.fn<<<(unsigned)q.grid, q.threads, q.smem, stream>>>(p);

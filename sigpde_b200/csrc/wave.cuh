@@ -294,10 +294,17 @@ struct GivenIncs {
     }
 };
 
+// The cell in one dependent operation down a column instead of two: other roundings (float64 cells only).
+template <typename T>
+__device__ __forceinline__ T stencil_chain(T k00, T k01, T k10, T A, T B)
+{
+    return fma(k01, A, fma(k10, A, -(k00 * B)));
+}
+
 // Solve one pair with the warp.  Returns K[n][m] in every lane.
 // bnd: per-warp boundary row buffer of m + 1 values (only touched when the
-// pair has more than one band).
-template <typename T, int R, int O, class Src>
+// pair has more than one band).  CHAIN: stencil_chain cells.
+template <typename T, int R, int O, bool CHAIN = false, class Src>
 __device__ T warp_solve(const SolveGeom &g, Src &src, T *bnd)
 {
     using BS = BlockShape<R, O>;
@@ -352,7 +359,8 @@ __device__ T warp_solve(const SolveGeom &g, Src &src, T *bnd)
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         const T l = left[r];
-                        const T v = stencil_cell(dg, up, l, A[BS::rc_of(r)], B[BS::rc_of(r)]);
+                        const T v = CHAIN ? stencil_chain(dg, up, l, A[BS::rc_of(r)], B[BS::rc_of(r)])
+                                          : stencil_cell(dg, up, l, A[BS::rc_of(r)], B[BS::rc_of(r)]);
                         dg = l;
                         up = v;
                         left[r] = v;

@@ -110,3 +110,42 @@ def test_narrow_grams_take_a_16_byte_aligned_workspace(sig, oracle, op, dim, mon
         assert st == 0, _lib.last_error()
         outs.append(out)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("n,L,d,order", [(5, 10, 3, 0), (3, 33, 4, 1), (4, 79, 5, 1), (3, 80, 5, 1), (3, 130, 2, 0),
+                                         (2, 66, 40, 2), (2, 70, 2, 4), (3, 40, 130, 1), (2, 40, 3, 6), (2, 301, 4, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("given", [False, True])
+def test_normalization_one_path_a_warp(sig, oracle, n, L, d, order, dtype, given, monkeypatch):
+    """A path a warp (SIGK_NORM_WARP=1) and a path a CTA (0): the same scales bit for bit, from a tile in shared memory,
+    from the differences and from the caller's increments, at the edges of bands and of the staged dimensions."""
+    class Increments:  # the linear kernel as a static kernel the device does not know
+        def pairwise(self, x, y):
+            return x @ y.transpose(1, 2)
+
+    x = oracle.brownian(n, L, d, 31 + L, scale=np.linspace(0.8, 3.0, n) / np.sqrt(d))
+    X = cuda(x, dtype)
+    rk = sig.RobustSigPDE(Increments() if given else sig.kernels.LinearKernel(), order)
+    got = []
+    for route in ("1", "0"):
+        monkeypatch.setenv("SIGK_NORM_WARP", route)
+        got.append(host(rk.normalization(X)))
+    np.testing.assert_array_equal(got[0], got[1])
+    tol = dict(rtol=1e-6, atol=1e-9) if dtype == torch.float64 and not given else dict(rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(got[0], oracle.normalization(host(X), order), **tol)
+
+
+@pytest.mark.parametrize("n,L,d,order", [(8, 1100, 3, 2), (8, 260, 2, 4), (17, 2061, 2, 0), (150, 1500, 2, 0),
+                                         (2600, 20, 3, 1)])
+def test_normalization_of_long_paths_and_many(sig, oracle, n, L, d, order, monkeypatch):
+    """Thousands of points, more bands than warps a CTA, more tiles than the workspace holds, many short paths: the
+    default route within the oracle's bound, and the other one the same."""
+    x = oracle.brownian(n, L, d, 41 + L, scale=np.linspace(0.8, 2.5, n))
+    X = cuda(x)
+    rk = sig.RobustSigPDE(sig.kernels.LinearKernel(), order)
+    lam = host(rk.normalization(X))
+    idx = np.unique(np.linspace(0, n - 1, 3).astype(int))
+    np.testing.assert_allclose(lam[idx], oracle.normalization(x[idx], order), rtol=1e-6, atol=1e-9)
+    for route in ("1", "0"):
+        monkeypatch.setenv("SIGK_NORM_WARP", route)
+        np.testing.assert_array_equal(host(rk.normalization(X)), lam)
