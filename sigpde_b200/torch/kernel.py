@@ -174,6 +174,14 @@ def _second_diff_forward(G, order, dtype):
     return _second_diff(0, G, G.shape, G.stride(), order, inc)
 
 
+def _second_diff_adjoint(grad_inc, shape, strides, dtype, order):
+    """dL/dG from dL/dinc, laid out as G (a Gram's axes are permuted), so that the static kernel's own backward reads
+    both alike."""
+    gG = (torch.empty_strided(shape, strides, dtype=dtype, device=grad_inc.device) if _dense(shape, strides)
+          else torch.empty(shape, dtype=dtype, device=grad_inc.device))
+    return _second_diff(1, grad_inc.detach().contiguous(), shape, gG.stride(), order, gG)
+
+
 class _SecondDiff(torch.autograd.Function):
     """Coarse increments from the static Gram G in one launch, and dL/dG in one
     (linear in G, so nothing is saved)."""
@@ -185,12 +193,22 @@ class _SecondDiff(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_inc):
-        shape, strides, dtype, order = ctx.meta
-        grad_inc = grad_inc.detach().contiguous()
-        # laid out as G (a Gram's axes are permuted), so that the static kernel's own backward reads both alike
-        gG = (torch.empty_strided(shape, strides, dtype=dtype, device=grad_inc.device) if _dense(shape, strides)
-              else torch.empty(shape, dtype=dtype, device=grad_inc.device))
-        return _second_diff(1, grad_inc, shape, gG.stride(), order, gG), None, None
+        if torch.is_grad_enabled() and grad_inc.requires_grad:  # create_graph: dL/dinc may depend on the scales
+            return _SecondDiffAdjoint.apply(grad_inc, *ctx.meta), None, None
+        return _second_diff_adjoint(grad_inc, *ctx.meta), None, None
+
+
+class _SecondDiffAdjoint(torch.autograd.Function):
+    """dL/dG from dL/dinc; its own adjoint is the second difference."""
+
+    @staticmethod
+    def forward(ctx, grad_inc, shape, strides, dtype, order):
+        ctx.meta = (order, grad_inc.dtype)
+        return _second_diff_adjoint(grad_inc, shape, strides, dtype, order)
+
+    @staticmethod
+    def backward(ctx, grad_G):
+        return _SecondDiff.apply(grad_G, *ctx.meta), None, None, None, None
 
 
 def _increments(x, y, static_kernel, dyadic_order, pairwise, dtype):

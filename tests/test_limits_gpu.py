@@ -149,3 +149,24 @@ def test_normalization_of_long_paths_and_many(sig, oracle, n, L, d, order, monke
     for route in ("1", "0"):
         monkeypatch.setenv("SIGK_NORM_WARP", route)
         np.testing.assert_array_equal(host(rk.normalization(X)), lam)
+
+
+@pytest.mark.parametrize("op", ["pairwise", "gram"])
+def test_gradient_with_a_graph_reaches_the_scales(sig, oracle, op, monkeypatch):
+    """create_graph on a static kernel's gradient: what depends on the scales outside the solver keeps its graph, as
+    with torch's own second difference."""
+    from sigpde_b200.torch import kernel
+    x, y = oracle.brownian(4, 12, 3, 51), oracle.brownian(4, 10, 3, 52)
+    k = sig.SigPDE(sig.kernels.RBFKernel(1.0), 1)
+
+    def second():
+        X, Y = cuda(x).requires_grad_(), cuda(y).requires_grad_()
+        s = cuda(np.linspace(0.7, 1.3, 4)).requires_grad_()
+        v = k.pairwise(X, Y, s, s) if op == "pairwise" else k.gram(X, Y, s, s)
+        gx, gy = torch.autograd.grad(v.sum(), (X, Y), create_graph=True)
+        return torch.autograd.grad((gx ** 2).sum() + (gy ** 2).sum(), (s, X, Y))
+
+    got = second()
+    monkeypatch.setattr(kernel, "_takes_second_diff", lambda G, dim: False)
+    for a, b in zip(got, second()):
+        np.testing.assert_allclose(host(a), host(b), rtol=1e-9, atol=1e-12)
