@@ -237,3 +237,12 @@ def test_route_choices_by_workspace(built_lib, monkeypatch):
     assert c3 < (1 << 30) + (64 << 20) < (2 << 30) < ws(S, 512, 512, 64, 64, 16, 1, TC64, SIGK_TC_CHUNK_MB="6144")
     assert ws(S, 512, 512, 128, 128, 8, 0, TC64) > 4 << 30
     assert ws(S, 512, 512, 128, 128, 8, 1, TC64) > 4 << 30
+
+
+def test_stream_lookup_without_the_private_function(monkeypatch):
+    """torch._C._cuda_getCurrentRawStream is private: without it the public stream object gives the handle."""
+    from types import SimpleNamespace
+    from sigpde_b200.torch import kernel
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=100 + device))
+    assert kernel._raw_stream_lookup()(3) == 103
