@@ -16,6 +16,7 @@
 #include <mutex>
 #include <string>
 #include <unordered_map>
+#include <utility>
 
 #include "../../include/sigk.h"
 #include "dispatch.h"
@@ -1159,6 +1160,23 @@ bool grad_shape(GradPlan &g, int64_t nx, int64_t items_per_x, int64_t ncx, int64
     return true;
 }
 
+// Pairs whose backward pass runs with the sides exchanged, k(x, y) = k(y, x): long x paths against a few columns, whose
+// bands wait out the least period (kGradMinPeriod) with most of its steps empty, where the other side as rows takes fewer
+// steps (us a training step: 8 pairs, L = 1485 / 10, d = 1, order 1 1196 / 680 exchanged; 50, L = 1485 / 30, d = 3
+// 1526 / 925).
+bool grad_exchange(int64_t npairs, int64_t ncx, int64_t ncy, int order)
+{
+    GradPlan a, b;
+    if (!grad_shape(a, npairs, 1, ncx, ncy, order) || a.nb == 1 || a.nsteps >= kGradMinPeriod ||
+        !grad_shape(b, npairs, 1, ncy, ncx, order))
+        return false;
+    auto steps = [&](const GradPlan &g) {
+        const int64_t run = grad_per_warp(npairs, get_grad_kernels(g.R, order, g.wide).ctas);
+        return grad_warp_steps(run, g.nb, g.period);
+    };
+    return steps(b) < steps(a);
+}
+
 // Increment matrix, records and boundary rows of a chunk from offset `off` on; returns the end.
 size_t grad_wave_layout(GradPlan &g, int64_t items, int64_t ncy, size_t off)
 {
@@ -2053,7 +2071,10 @@ size_t sigk_backward_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t le
     (void)dtype;
     if (op != SIGK_OP_PAIRWISE && op != SIGK_OP_GRAM) return 0;
     if (len_x < 2 || len_y < 2 || order < 0 || order > 12 || dim < 1 || n_x < 1 || n_y < 1) return 0;
-    if (op == SIGK_OP_PAIRWISE) n_y = n_x;
+    if (op == SIGK_OP_PAIRWISE) {
+        n_y = n_x;
+        if (grad_exchange(n_x, len_x - 1, len_y - 1, order)) std::swap(len_x, len_y);
+    }
     GradPlan g = make_grad_plan(op == SIGK_OP_PAIRWISE ? kOpPairwise : kOpGram, n_x, n_y, len_x - 1, len_y - 1, dim,
                                 order);
     return g.ok ? g.ws_bytes : 0;
@@ -2083,6 +2104,12 @@ int sigk_backward(int op, const void *x, const void *y, int64_t n_x, int64_t n_y
         (st = check_dev(scale_y, "scale_y", true)))
         return st;
     const int kop = op == SIGK_OP_PAIRWISE ? kOpPairwise : kOpGram;
+    if (kop == kOpPairwise && grad_exchange(n_x, len_x - 1, len_y - 1, order)) {
+        std::swap(x, y);
+        std::swap(len_x, len_y);
+        std::swap(scale_x, scale_y);
+        std::swap(grad_x, grad_y);
+    }
     GradPlan g = make_grad_plan(kop, n_x, n_y, len_x - 1, len_y - 1, dim, order);
     if (!g.ok) return fail(SIGK_EUNSUPPORTED, "no backward plan");
     if (!workspace || workspace_bytes < g.ws_bytes)
@@ -2096,6 +2123,7 @@ int sigk_backward(int op, const void *x, const void *y, int64_t n_x, int64_t n_y
 size_t sigk_backward_inc_workspace_size(int64_t npairs, int64_t nc_x, int64_t nc_y, int order)
 {
     if (npairs < 1 || nc_x < 1 || nc_y < 1 || order < 0 || order > kGradMaxOrder) return 0;
+    if (grad_exchange(npairs, nc_x, nc_y, order)) std::swap(nc_x, nc_y);
     GradPlan g = make_grad_inc_plan(npairs, nc_x, nc_y, order);
     return g.ok ? g.ws_bytes : 0;
 }
@@ -2116,6 +2144,11 @@ int sigk_backward_inc(const void *inc, int64_t npairs, int64_t nc_x, int64_t nc_
         (st = check_dev(grad_inc, "grad_inc", false)) || (st = check_dev(scale_x, "scale_x", true)) ||
         (st = check_dev(scale_y, "scale_y", true)))
         return st;
+    if (grad_exchange(npairs, nc_x, nc_y, order)) {
+        std::swap(nc_x, nc_y);
+        std::swap(s1, s2);
+        std::swap(g1, g2);
+    }
     GradPlan g = make_grad_inc_plan(npairs, nc_x, nc_y, order);
     if (!g.ok) return fail(SIGK_EUNSUPPORTED, "no backward plan");
     if (!workspace || workspace_bytes < g.ws_bytes)

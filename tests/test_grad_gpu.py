@@ -317,3 +317,33 @@ def test_second_difference_kernel(sig, shape, types):
         w = torch.randint(-16, 17, tuple(want.shape), generator=g).to(types[1]).cuda()
         (wa,), (wb,) = torch.autograd.grad(want, Ga, w), torch.autograd.grad(got, Gb, w)
         assert wb.dtype == types[0] and torch.equal(wa, wb)
+
+
+@pytest.mark.parametrize("shape,exchanged", [((3, 599, 12, 3, 1), True), ((8, 1485, 10, 1, 1), True),
+                                             ((2, 1100, 30, 4, 0), False), ((2, 600, 6, 5, 2), True)])
+def test_long_against_short_gradients(sig, oracle, shape, exchanged):
+    """Long x paths against a few points: where that takes fewer steps the sides are exchanged inside, so that both
+    orders of the arguments are the same computation; scales, and increments that torch builds, included."""
+    B, lx, ly, d, o = shape
+    x, y = oracle.brownian(B, lx, d, 31), oracle.brownian(B, ly, d, 32)
+    w, sx, sy = np.linspace(-1.0, 1.5, B), np.linspace(0.6, 1.4, B), np.linspace(1.2, 0.7, B)
+
+    class Increments:  # the linear kernel as a static kernel the device does not know
+        scale = None
+
+        def pairwise(self, a, b):
+            return 0.8 * a @ b.transpose(1, 2)
+
+    def grads(kernel, a, b, sa, sb):
+        A, C = cuda(a, grad=True), cuda(b, grad=True)
+        return [host(g) for g in torch.autograd.grad(
+            (sig.SigPDE(kernel, o).pairwise(A, C, cuda(sa), cuda(sb)) * cuda(w)).sum(), (A, C))]
+
+    want = oracle.grad_pairwise(x, y, o, w, sx, sy, static_scale=0.8)
+    for kernel in (sig.kernels.LinearKernel(0.8), Increments()):
+        got, other = grads(kernel, x, y, sx, sy), grads(kernel, y, x, sy, sx)
+        for g, ref, name in zip(got, want, "xy"):
+            close(g, ref, TOL64, f"grad {name}")
+        if exchanged and kernel.scale is not None:
+            np.testing.assert_array_equal(got[0], other[1])
+            np.testing.assert_array_equal(got[1], other[0])
