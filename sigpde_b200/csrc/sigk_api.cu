@@ -1160,21 +1160,21 @@ bool grad_shape(GradPlan &g, int64_t nx, int64_t items_per_x, int64_t ncx, int64
     return true;
 }
 
-// Pairs whose backward pass runs with the sides exchanged, k(x, y) = k(y, x): long x paths against a few columns, whose
-// bands wait out the least period (kGradMinPeriod) with most of its steps empty, where the other side as rows takes fewer
-// steps (us a training step: 8 pairs, L = 1485 / 10, d = 1, order 1 1196 / 680 exchanged; 50, L = 1485 / 30, d = 3
-// 1526 / 925).
+// Pairs whose backward pass runs with the sides exchanged, k(x, y) = k(y, x): a few pairs of long x paths against a few
+// columns, whose bands wait out the least period (kGradMinPeriod) with most of its steps empty, where the other side as
+// rows takes fewer of them, each at a lone warp's latencies and its cells (us a training step, as they are / exchanged:
+// 8 pairs, L = 1485 / 10, d = 1, order 1 1196 / 680; 50, L = 1485 / 30, d = 3 1526 / 925; 143, L = 548 / 2, d = 20, order 1
+// 746 / 692; but 722, L = 164 / 3, order 2 411 / 480; 1948, L = 1006 / 10, order 1, two pairs a warp 2625 / 2748).
 bool grad_exchange(int64_t npairs, int64_t ncx, int64_t ncy, int order)
 {
     GradPlan a, b;
-    if (!grad_shape(a, npairs, 1, ncx, ncy, order) || a.nb == 1 || a.nsteps >= kGradMinPeriod ||
-        !grad_shape(b, npairs, 1, ncy, ncx, order))
+    if (npairs > 4ll * sm_count() || !grad_shape(a, npairs, 1, ncx, ncy, order) || a.nb == 1 ||
+        a.nsteps >= kGradMinPeriod || !grad_shape(b, npairs, 1, ncy, ncx, order))
         return false;
-    auto steps = [&](const GradPlan &g) {
-        const int64_t run = grad_per_warp(npairs, get_grad_kernels(g.R, order, g.wide).ctas);
-        return grad_warp_steps(run, g.nb, g.period);
+    auto cost = [&](const GradPlan &g) {
+        return (double)grad_warp_steps(1, g.nb, g.period) * (58.0 + g.R * get_grad_kernels(g.R, order, g.wide).cols);
     };
-    return steps(b) < steps(a);
+    return 1.3 * cost(b) < cost(a);
 }
 
 // Increment matrix, records and boundary rows of a chunk from offset `off` on; returns the end.

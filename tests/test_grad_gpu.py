@@ -320,7 +320,7 @@ def test_second_difference_kernel(sig, shape, types):
 
 
 @pytest.mark.parametrize("shape,exchanged", [((3, 599, 12, 3, 1), True), ((8, 1485, 10, 1, 1), True),
-                                             ((2, 1100, 30, 4, 0), False), ((2, 600, 6, 5, 2), True)])
+                                             ((2, 1100, 30, 4, 0), False), ((2, 600, 6, 5, 2), False)])
 def test_long_against_short_gradients(sig, oracle, shape, exchanged):
     """Long x paths against a few points: where that takes fewer steps the sides are exchanged inside, so that both
     orders of the arguments are the same computation; scales, and increments that torch builds, included."""
