@@ -1891,11 +1891,13 @@ NormPlan norm_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_inc)
         // work, which costs from 16 paths an SM on (us, CTA / warp, order 0, 1, 2: n = 13000 - 16000, L = 16 - 21
         // 1051 / 761, 1009 / 751, 1064 / 760; n = 2500 - 2900, L = 14 - 16 145 / 145, 153 / 145, 234 / 188; n = 1200 -
         // 1300, L = 22 - 28 189 / 267, 222 / 214, 222 / 214).  Fewer points than that leave the root-find's own
-        // arithmetic, at 32 lanes a path (n = 18771, L = 5, order 1 515 / 569); more, and order 3, a CTA's bands.
+        // arithmetic, at 32 lanes a path (n = 18771, L = 5, d = 3, order 1 515 / 569), unless the dot products outweigh it
+        // (n = 21176, L = 8, d = 50, order 0 939 / 713); more, and order 3, a CTA's bands.
         const int64_t per_sm = n / sm_count();
         const bool many = per_sm >= (order == 0 ? 16 : 12) && nc >= 9 && nc <= 32;
         const bool most = per_sm >= 64 && nc > 32 && nc <= (order == 0 ? 40 : 48);
-        return (order <= 2 && many) || (order <= 1 && most)
+        const bool wide = per_sm >= 16 && nc >= 4 && nc <= 8 && d >= 32;
+        return (order <= 2 && many) || (order <= 1 && most) || (order <= 3 && wide)
                    ? w
                    : norm_cta_plan(n, nc, d, order, from_inc);
     }
