@@ -813,7 +813,8 @@ __global__ void grad_gy_kernel(GradContractParams p)
 // kGyRows rows and 8 dimensions; its lanes take two neighbouring m each (16-byte
 // loads, the next ones in flight), the differences of a tile of m come from
 // shared memory (dimension-major [k][m], two tiles), and the lanes' sums meet in
-// a fixed shuffle tree.  grad_gy_reduce_kernel adds the ranges of m in order.
+// a fixed shuffle tree.  grad_points_kernel adds the ranges of m in order, in a
+// call of several chunks of x paths grad_gy_reduce_kernel first.
 // (One fma per shared-memory load, or the differences read from the L2 by each
 // warp, cost 2.39 and 1.76 ms for the 2.1 GB of a 128 x 128 gradient.)
 constexpr int kGyRows = 8;

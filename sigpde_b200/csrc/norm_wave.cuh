@@ -10,11 +10,13 @@
 // path, into shared memory where they fit, else into a tile in the workspace
 // that stays in the L2.  Measured, before (one warp a path, increments re-formed
 // each solve above 48 KB; or bands that poll each other through global memory)
-// and now, us a call: 24 paths, L = 220, d = 8, order 1: 4067, 565; 512 paths,
-// L = 64, d = 16, order 1: 297, 163; 8 paths, L = 256, d = 32, order 2: 15640,
-// 1183; 32 paths, L = 128, d = 32, order 1: 1644, 320.
+// and now, us a call: 24 paths, L = 220, d = 8, order 1: 4069, 553; 512 paths,
+// L = 64, d = 16, order 1: 297, 152; 8 paths, L = 256, d = 32, order 2: 16185,
+// 1191; 32 paths, L = 128, d = 32, order 1: 1642, 301.  Calls of many short paths,
+// or of long ones in number, take a warp a path instead (norm_warp.cuh).
 //
-// The increments' sums are those of the other kernels, in the same order.
+// The increments' sums are those of the other kernels, in the same order; the
+// root-find's cells are stencil_chain's, whose roundings differ from theirs.
 #pragma once
 
 #include "sigk_kernels.cuh"

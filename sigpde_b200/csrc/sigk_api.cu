@@ -340,10 +340,14 @@ struct TcPlan {
     size_t err_off, a_off, b_off, ct_off, ws_bytes;
 };
 
-// Float matrices read by half-warp pipelines at order 1 (at most 128 refined rows) run faster in
-// chunks of at most 1 GiB: RobustSigPDE.gram N=512, L=64, d=16, tc64 2.23 -> 2.04 ms; a 512 x 512
-// order-1 Gram 3.64 -> 3.33 ms (tc32 symmetric 1.93 -> 1.73 ms).  Orders 0 and 2 and float64
-// matrices measured slower with small chunks, so they keep kTcChunkBytes.
+// Float matrices read by half-warp pipelines at order 1 (at most 128 refined rows) come in chunks of
+// at most 1 GiB.  With float32 cells that is faster (ms, 6 GiB / 1 GiB: 512 x 512, L = 64, d = 16,
+// tc32 3.08 / 2.54, symmetric 1.67 / 1.39); with float64 cells it costs a little since the reader
+// takes several columns a step (tc64 2.54 / 2.67, symmetric 1.43 / 1.47; 1000 x 1000, L = 65 9.6 /
+// 10.5) and keeps the call's memory down.  Orders 0 and 2 and float64 matrices measured slower with
+// small chunks (symmetric 512, L = 128, d = 8, order 0, tc64 3.66 / 4.31; 256 x 256, L = 128, d = 8,
+// order 2, tc32 4.69 / 4.92; symmetric 512, L = 64, d = 16, order 1, fp64 2.14 / 2.40), so they keep
+// kTcChunkBytes.
 constexpr size_t kTcChunkBytesHalfWarpO1 = size_t(1) << 30;
 
 size_t tc_chunk_cap(size_t by_default = kTcChunkBytes)
@@ -545,9 +549,11 @@ int consume_matrix(const TcPlan &t, int op, const void *mat, bool mat64, int64_t
     }
     const bool f64 = cell_prec(precision) == SIGK_PREC_FP64;
     // pairs of at most 128 refined rows run as half-warp pipelines (two pairs a warp, twice the rows a
-    // lane, half the pipeline fill): measured faster except for float64 matrices at order 0 (one
-    // column a step, where twice the rows a lane doubles each step's loads: 1.11 vs 1.02 ms at
-    // N=128 L=128 d=32)
+    // lane, half the pipeline fill): us, whole / half warps, 512 x 512, L = 64, d = 16, order 1, tc64
+    // 3435 / 2672; 256 x 256, L = 65, d = 32, order 1, fp64 1691 / 1595.  Float64 matrices at order 0 keep
+    // whole warps, where twice the rows a lane doubles each step's loads: alike or slower near 128 rows
+    // (128 x 128, L = 128, d = 32 1472 / 1485; symmetric 300, L = 100, d = 16 1902 / 1941; the half warp
+    // is faster at 64: 256 x 256, L = 64, d = 24 1764 / 1295)
     const int64_t nrows = ncx << order;
     int W = 32, R = t.R;
     if (nrows <= 128 && !(mat64 && order == 0) && !env_flag("SIGK_NO_HALF_WARP")) {
@@ -601,9 +607,11 @@ struct FtPlan {
 FtPlan make_fused_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order, int precision)
 {
     FtPlan f;
-    // The route where it is eligible and the order is 2 or more (cells outweigh the per-chunk boundary: config 2
-    // 5.15 ms fused vs 5.59 two-phase; at orders 0-1 the two-phase route measured faster).  SIGK_FUSED_TC=1
-    // takes it at every eligible order, SIGK_FUSED_TC=0 never.
+    // The route where it is eligible and the order is 2 or more (cells outweigh the per-chunk boundary: 256 x 256,
+    // L = 128, d = 8, order 2 4.97 ms fused, 5.22 two-phase; 2.73 and 2.50 at order 1), and where it needs no matrix:
+    // two-phase readers of at most 64 rows a half warp overtook it (L = 64, d = 16, order 2 1.77 and 1.51, 512 x 512 6.82
+    // and 5.86; L = 64, d = 32, order 3 4.20 and 4.13), with 1 to 4 GB of it.  SIGK_FUSED_TC=1 takes it at every eligible
+    // order, SIGK_FUSED_TC=0 never.
     const char *force = getenv("SIGK_FUSED_TC");
     const int mode = (force && force[0]) ? (force[0] != '0' ? 1 : 0) : -1;
     if (op != kOpGram || precision != SIGK_PREC_TC64 || d > 32 || order > 3 || mode == 0 || (mode < 0 && order < 2))
@@ -618,7 +626,7 @@ FtPlan make_fused_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
     const int ring = fused_tc_smem(rc, kpd, 16) <= kFtMaxSmem ? 16 : fused_tc_smem(rc, kpd, 8) <= kFtMaxSmem ? 8 : 0;
     if (!ring || !get_fused_tc_kernel(R, order, ring)) return f;
     // at 4 coarse rows a lane the 8-step boundary's copy outweighs the matrix round trip (256 x 256, L = 128,
-    // d = 16, order 2: 5.93 vs 5.63 ms two-phase); at 2 it wins (L = 64, d = 32, order 3: 4.30 vs 4.44 ms)
+    // d = 16, order 2: 5.74 ms, 5.25 two-phase); at 2 they are alike (above)
     if (mode < 0 && ring == 8 && rc > 2) return f;
     f.ok = true;
     f.R = R;
@@ -1833,8 +1841,8 @@ NormPlan norm_cta_plan(int64_t n, int64_t nc, int64_t d, int order, bool from_in
             // paths an SM works on together, and the time of all of its paths: the steps of a solve, each at the issue
             // slots of a warp's step (two for each of 3 float64 operations a cell and 5 a coarse cell) times the warps
             // that share a sub-partition, or a lone warp's slots and latencies (a tile in the L2 costs its loads too).
-            // Rows a lane, us: 24 paths, L = 220, d = 8, order 1: 617 / 565 / 680 with 2 / 4 / 8; 512, L = 64, d = 16,
-            // order 1: 210 / 163 / 205; 512, L = 256, d = 8, order 2: 5984 / 3702 / 2654 (16: 4312)
+            // Rows a lane, us: 24 paths, L = 220, d = 8, order 1: 605 / 553 / 664 with 2 / 4 / 8; 512, L = 64, d = 16,
+            // order 1: 199 / 152 / 192; 512, L = 256, d = 8, order 2: 4586 / 3646 / 2665 (16: 4284)
             int64_t res = (int64_t)((228 * 1024) / (q.smem + 1024));
             const int64_t by_regs = 65536 / ((int64_t)q.threads * q.k.regs);
             if (res > by_regs) res = by_regs;
