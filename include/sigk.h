@@ -130,7 +130,7 @@ SIGK_API size_t sigk_workspace_size(int op, int64_t n_x, int64_t n_y, int64_t le
 
 /*
  * The least scratch with which the same call runs.  It is sigk_workspace_size but for float64-cell Grams of narrow
- * paths (dim < 16): with all of sigk_workspace_size (up to 1.5 GiB), 256-byte aligned, they read a matrix of all
+ * paths (dim < 16): with all of sigk_workspace_size (up to 3 GiB), 256-byte aligned, they read a matrix of all
  * increments; with less, or aligned to 16 bytes only, they take kernels that need the path differences alone and give the
  * same values.
  */

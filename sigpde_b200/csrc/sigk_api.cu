@@ -335,6 +335,7 @@ struct TcPlan {
     int64_t rows_x, rows_y;   // matrix rows per x path (ncx rounded up to 4) and per y path
     int64_t chunk, nchunks;   // x paths per chunk
     int64_t cap_pairs;        // > 0: chunks of a symmetric Gram by their x paths times y paths instead
+    int64_t fewest;           // chunks at the cap, where narrow_chunks may take more
     int64_t a_tiles, b_tiles; // operand tiles per image
     size_t a_bytes, b_bytes;  // bytes of one (hi or lo) image
     size_t err_off, a_off, b_off, ct_off, ws_bytes;
@@ -502,6 +503,23 @@ int tc_gemm(const TcGemmParams &gp, cudaStream_t stream, int bn = kTcBN)
 }
 
 
+// Pairs of at most 128 refined rows run as half-warp pipelines (two pairs a warp, twice the rows a
+// lane, half the pipeline fill): us, whole / half warps, 512 x 512, L = 64, d = 16, order 1, tc64
+// 3435 / 2672; 256 x 256, L = 65, d = 32, order 1, fp64 1691 / 1595.  Float64 matrices at order 0 keep
+// whole warps, where twice the rows a lane doubles each step's loads: alike or slower near 128 rows
+// (128 x 128, L = 128, d = 32 1472 / 1485; symmetric 300, L = 100, d = 16 1902 / 1941; the half warp
+// is faster at 64: 256 x 256, L = 64, d = 24 1764 / 1295)
+struct PipeShape {
+    int W, R; // lanes a pipeline, rows a lane
+};
+PipeShape inc_pipe_shape(int64_t nrows, int order, int R, bool mat64)
+{
+    if (nrows > 128 || (mat64 && order == 0) || env_flag("SIGK_NO_HALF_WARP")) return {32, R};
+    int Rh = 2;
+    while (16 * Rh < nrows) Rh *= 2;
+    return {16, Rh};
+}
+
 // The wavefront over one chunk of x paths [i0, i1) reading an increment matrix
 // (out[n * ld + m], float32 from the tensor cores or float64 from
 // dgemm_inc_kernel): the streaming kernel for single-band pairs with enough
@@ -548,19 +566,8 @@ int consume_matrix(const TcPlan &t, int op, const void *mat, bool mat64, int64_t
         return launch(pfn, p, p.nitems, 0, stream);
     }
     const bool f64 = cell_prec(precision) == SIGK_PREC_FP64;
-    // pairs of at most 128 refined rows run as half-warp pipelines (two pairs a warp, twice the rows a
-    // lane, half the pipeline fill): us, whole / half warps, 512 x 512, L = 64, d = 16, order 1, tc64
-    // 3435 / 2672; 256 x 256, L = 65, d = 32, order 1, fp64 1691 / 1595.  Float64 matrices at order 0 keep
-    // whole warps, where twice the rows a lane doubles each step's loads: alike or slower near 128 rows
-    // (128 x 128, L = 128, d = 32 1472 / 1485; symmetric 300, L = 100, d = 16 1902 / 1941; the half warp
-    // is faster at 64: 256 x 256, L = 64, d = 24 1764 / 1295)
-    const int64_t nrows = ncx << order;
-    int W = 32, R = t.R;
-    if (nrows <= 128 && !(mat64 && order == 0) && !env_flag("SIGK_NO_HALF_WARP")) {
-        W = 16;
-        R = 2;
-        while (16 * R < nrows) R *= 2;
-    }
+    const PipeShape ps = inc_pipe_shape(ncx << order, order, t.R, mat64);
+    const int W = ps.W, R = ps.R;
     StreamIncFn fn = get_stream_inc_kernel(f64, R, t.O, mat64, W);
     int nb = 0;
     if ((st = blocks_per_sm((const void *)fn, 0, &nb))) return st;
@@ -829,6 +836,67 @@ int64_t chunk_end(const TcPlan &t, int64_t i0, int64_t nx)
     return i1 < nx ? i1 : nx;
 }
 
+// Chunks of a narrow Gram's matrix (of x paths with per_x bytes each, at most cap bytes): equal ones, or a symmetric
+// Gram's of as many x paths as their own columns let in.  A chunk's wavefront gives each pipeline whole pairs, so one pair
+// more than the pipelines doubles their runs and halves their number; of the sizes between the cap and two thirds of it
+// the one with the least time is taken, a run costing 13 and one more for each warp on its SM (200 x 180, L = 256 / 220,
+// d = 15, order 2, chunks of 1980 / 2340 / 2880 / 3060 / 3420 pairs on 2960 pipelines: 17.3 / 15.3 / 15.1 / 17.6 / 17.1 ms).
+// Returns the matrix's bytes.
+size_t narrow_chunks(TcPlan &t, int op, int64_t nx, int64_t ny, int64_t ncx, int order, size_t per_x, size_t cap)
+{
+    const PipeShape ps = t.stream ? inc_pipe_shape(ncx << order, order, t.R, true) : PipeShape{32, t.R};
+    const void *fn = t.stream ? (const void *)get_stream_inc_kernel(true, ps.R, t.O, true, ps.W)
+                              : (const void *)get_pair_kernel_f64(false, kPairMat64, t.R, t.O);
+    int nb = 0;
+    const int lanes = ps.W;
+    const std::string before = g_last_error;
+    if (blocks_per_sm(fn, 0, &nb)) { // no device: the size of a plan that nothing will run, and no error of this call
+        g_last_error = before;
+        nb = 4;
+    }
+    const int64_t sms = sm_count(), pipes = sms * nb * kWarpsPerBlock * (32 / lanes);
+    auto cost = [&](int64_t pairs) {
+        const int64_t run = (pairs + pipes - 1) / pipes, used = (pairs + run - 1) / run;
+        return (double)run * (13.0 + (double)used * lanes / (32.0 * (double)sms)) + 1.0;
+    };
+    const size_t per_pair = per_x / (size_t)ny;
+    double best = -1.0;
+    TcPlan pick = t;
+    size_t bytes = 0;
+    for (int i = 0; i <= 16; ++i) { // caps from all to two thirds
+        TcPlan q = t;
+        const size_t c = cap - cap / 48 * (size_t)i;
+        double time = 0.0;
+        int64_t most = 0;
+        if (op == kOpGramSym) {
+            q.cap_pairs = (int64_t)(c / per_pair);
+            if (q.cap_pairs < nx) break; // the last x path alone
+            q.nchunks = 0;
+            for (int64_t i0 = 0, i1; i0 < nx; i0 = i1, ++q.nchunks) {
+                i1 = chunk_end(q, i0, nx);
+                time += cost((i1 * (i1 + 1) - i0 * (i0 + 1)) / 2);
+                if ((i1 - i0) * i1 > most) most = (i1 - i0) * i1;
+            }
+        } else {
+            const int64_t rows = (int64_t)(c / per_x);
+            if (rows < 1) break;
+            const int64_t k = (nx + rows - 1) / rows;
+            q.chunk = (nx + k - 1) / k;
+            q.nchunks = (nx + q.chunk - 1) / q.chunk;
+            time = (double)(nx / q.chunk) * cost(q.chunk * ny) + (nx % q.chunk ? cost(nx % q.chunk * ny) : 0.0);
+            most = q.chunk * ny;
+        }
+        if (i == 0) t.fewest = q.nchunks;
+        if (best >= 0.0 && time >= best) continue;
+        best = time;
+        q.fewest = t.fewest;
+        pick = q;
+        bytes = (size_t)most * per_pair;
+    }
+    t = pick;
+    return bytes;
+}
+
 // es: bytes per element of the increment matrix (8 for float64 cells, 4 for float32 cells); the chunk of x
 // paths per launch and the matrix's share of the workspace follow it.
 TcPlan mat64_layout(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order, bool diffs,
@@ -858,20 +926,7 @@ TcPlan mat64_layout(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, in
     t.chunk = chunk;
     t.nchunks = (nx + chunk - 1) / chunk;
     size_t mat_bytes = (size_t)chunk * per_x;
-    if (narrow && op == kOpGram) { // equal chunks
-        t.chunk = (nx + t.nchunks - 1) / t.nchunks;
-        t.nchunks = (nx + t.chunk - 1) / t.chunk;
-        mat_bytes = (size_t)t.chunk * per_x;
-    } else if (narrow && t.nchunks > 1) { // symmetric: as many x paths as their own columns let in
-        t.cap_pairs = (int64_t)(cap / (per_x / (size_t)nx));
-        t.nchunks = 0;
-        int64_t most = 0;
-        for (int64_t i0 = 0, i1; i0 < nx; i0 = i1, ++t.nchunks) {
-            i1 = chunk_end(t, i0, nx);
-            if ((i1 - i0) * i1 > most) most = (i1 - i0) * i1;
-        }
-        mat_bytes = (size_t)most * (per_x / (size_t)nx);
-    }
+    if (narrow && t.nchunks > 1) mat_bytes = narrow_chunks(t, op, nx, ny_paths, ncx, order, per_x, cap);
     t.err_off = 0;
     t.bnd_off = 256;
     t.a_off = t.bnd_off + bnd_bytes; // x differences
@@ -881,10 +936,11 @@ TcPlan mat64_layout(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, in
     return t;
 }
 
-// The narrow paths' matrix is an option beside kernels that need a few MB, so it takes a quarter of the room that the
-// other matrices may (ms at 1.5 / 6 GiB: 256 x 256, L = 200, d = 8, order 0: 9.12 / 8.44, fused 27.9; 200 x 170, L = 250,
-// d = 14, order 1: 7.7 / 8.1, fused 15.2; 1000 x 1000, L = 128, d = 12, order 1: 66.4 / 63.0, fused 173).
-constexpr size_t kNarrowChunkBytes = size_t(1536) << 20;
+// The narrow paths' matrix is an option beside kernels that need a few MB, so it takes half of the room that the other
+// matrices may (ms at 1.5 / 3 / 6 GiB: 256 x 256, L = 200, d = 8, order 0 8.49 / 8.26 / 8.19, fused 28.0; 200 x 200,
+// L = 250, d = 12, order 0 10.1 / 9.4 / 9.1, fused 13.6; symmetric, 220 paths, L = 256, d = 13, order 1 6.66 / 6.21 / 6.00,
+// fused 11.9).
+constexpr size_t kNarrowChunkBytes = size_t(3) << 30;
 
 TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy, int64_t d, int order)
 {
@@ -923,11 +979,11 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         // Nor where the matrix comes in chunks of too few pairs: each chunk's wavefront waits for its slowest warp, and
         // more rows a lane or several bands want more of them (ms, fused / matrix.  One band: 128 x 128, L = 120,
         // d = 12, order 1, chunks of 384 pairs 2.75 / 2.75, 512 2.75 / 2.19; 200 x 170, L = 250, d = 14, order 1, 1170
-        // 15.2 / 9.8; 93 x 114, L = 377 / 420, d = 5, order 0, 1178 5.1 / 6.3.  Several: 80 x 80, L = 300, d = 8, order 1,
+        // 15.2 / 9.8; 93 x 114, L = 377 / 420, d = 5, order 0, 2500 5.1 / 5.8.  Several: 80 x 80, L = 300, d = 8, order 1,
         // 725 4.5 / 7.1, 1450 4.5 / 4.4, 2133 4.5 / 3.4; symmetric, 47 paths, L = 1786, d = 11, order 1, 113 22.8 / 145;
         // symmetric, 120 paths, L = 250, d = 11, order 3, 2420 9.9 / 10.8).
-        const int least = band && Rs < 16 ? 6 : sym && !band && order >= 2 ? 24 : 12;
-        if (multi && pairs < t.nchunks * sms * least) return TcPlan{};
+        const int least = band && Rs < 16 ? 6 : (sym && !band && order >= 2) || (band && !sym && d < 8) ? 24 : 12;
+        if (multi && pairs < t.fewest * sms * least) return TcPlan{};
         return t;
     }
     // A Gram of order 2-3 whose lanes hold dx in registers runs faster on the two-entry register kernel,

@@ -43,7 +43,7 @@ def test_few_pairs_infinite_increments(sig, oracle, lx, ly, order, where, monkey
 
 
 def _narrow(oracle):
-    """A Gram whose increment matrix takes 1.5 GiB and whose differences take a few MB."""
+    """A Gram whose increment matrix takes over 1 GiB and whose differences take a few MB."""
     x, y = oracle.brownian(256, 200, 8, 11), oracle.brownian(200, 200, 8, 12)
     return cuda(x, torch.float32), cuda(y, torch.float32)
 

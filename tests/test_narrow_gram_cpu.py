@@ -34,7 +34,7 @@ def test_no_matrix_in_chunks_of_few_pairs(lib, monkeypatch, op, nx, ny, lx, ly, 
 @pytest.mark.parametrize("op,nx,ny,lx,ly,d,order", [
     (GRAM, 24, 12, 765, 580, 8, 0), (SYM, 24, 24, 537, 537, 8, 0), (SYM, 11, 11, 690, 690, 9, 0),
     (GRAM, 34, 34, 153, 173, 8, 2), (SYM, 81, 81, 128, 128, 8, 3), (GRAM, 40, 40, 150, 167, 8, 3),
-    (SYM, 120, 120, 200, 200, 8, 2), (GRAM, 90, 90, 300, 317, 8, 2), (SYM, 120, 120, 250, 250, 11, 3),
+    (SYM, 120, 120, 200, 200, 8, 2), (GRAM, 90, 90, 300, 317, 8, 2),
     (SYM, 266, 266, 442, 442, 6, 0), (GRAM, 93, 114, 377, 420, 5, 0), (GRAM, 38, 22, 371, 310, 3, 0)])
 def test_no_matrix_where_it_measured_slower(lib, monkeypatch, op, nx, ny, lx, ly, d, order):
     """Several bands with few pairs, few dimensions at orders 2 and 3, chunks that fill the device once at most."""
@@ -44,7 +44,8 @@ def test_no_matrix_where_it_measured_slower(lib, monkeypatch, op, nx, ny, lx, ly
 
 @pytest.mark.parametrize("op,nx,ny,lx,ly,d,order", [
     (GRAM, 256, 256, 200, 200, 8, 0), (GRAM, 128, 128, 120, 120, 12, 1), (GRAM, 1000, 1000, 128, 128, 12, 1),
-    (GRAM, 80, 80, 300, 300, 8, 1), (SYM, 300, 300, 200, 200, 10, 0), (GRAM, 100, 90, 180, 200, 9, 2)])
+    (GRAM, 80, 80, 300, 300, 8, 1), (SYM, 300, 300, 200, 200, 10, 0), (GRAM, 100, 90, 180, 200, 9, 2),
+    (SYM, 120, 120, 250, 250, 11, 3)])
 def test_matrix_where_chunks_hold_enough_pairs(lib, monkeypatch, op, nx, ny, lx, ly, d, order):
     default, fused = sizes(lib, monkeypatch, op, nx, ny, lx, ly, d, order)
     assert default > fused
@@ -55,9 +56,9 @@ def test_matrix_where_chunks_hold_enough_pairs(lib, monkeypatch, op, nx, ny, lx,
     (GRAM, 80, 80, 300, 300, 8, 1), (GRAM, 400, 333, 256, 200, 15, 1), (SYM, 2000, 2000, 60, 60, 15, 1),
     (GRAM, 64, 64, 1000, 1000, 8, 2)])
 def test_matrix_stays_an_option_of_bounded_size(lib, monkeypatch, op, nx, ny, lx, ly, d, order):
-    """At most 1.5 GiB beside the differences; the least workspace is the fused route's."""
+    """At most 3 GiB beside the differences; the least workspace is the fused route's."""
     default, fused = sizes(lib, monkeypatch, op, nx, ny, lx, ly, d, order)
-    assert default <= (1536 << 20) + 2 * fused + 1024
+    assert default <= (3 << 30) + 2 * fused + 1024
     assert lib.sigk_workspace_min_size(op, nx, ny, lx, ly, d, order, F32, FP64) == fused
 
 
