@@ -965,14 +965,14 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         const bool multi = t.nchunks > 1;
         if (!band) {
             // A warp solves a pair of several bands, and one with few pairs beside it has latencies to hide the
-            // increments in; from order 2 on they are few beside the cells (us, fused / matrix: 24 x 12, L = 765 / 580,
-            // d = 8, order 0 1823 / 2232; symmetric, 14 paths, L = 667, d = 11, order 0 2602 / 2504; 34 x 34, L = 153 /
+            // increments in; from order 2 on they are few beside the cells (us, fused / matrix: 37 x 24, L = 554 / 605,
+            // d = 8, order 0 2116 / 2633; symmetric, 14 paths, L = 667, d = 11, order 0 2602 / 2504; 34 x 34, L = 153 /
             // 173, d = 8, order 2 452 / 491, 60 x 60 symmetric, L = 200 845 / 773; order 2, L = 239 / 154, d = 10: 588
             // pairs 389 / 437, 960 505 / 478).  At few dimensions they are worth no matrix at order 3, and at order 2
             // none in several chunks (d = 8: 40 x 40, L = 150, order 3 1114 / 1159; 90 x 90, L = 300, order 2 6393 /
             // 6919; symmetric, 120 paths, L = 200, order 2 2612 / 2908; but 100 x 90, L = 180 / 200, d = 9, order 2 3520 /
             // 3200; symmetric, 120 paths, L = 80, order 4 4392 / 4048).
-            const int least = order >= 2 ? (d < 11 ? 12 : 6) : d < 10 ? 6 : 0;
+            const int least = order >= 2 ? (d < 11 ? 12 : 6) : d < 10 ? 9 : 0;
             if (pairs < sms * least || (order == 3 && d < 11) || (order == 2 && multi && d < (sym ? 11 : 9)))
                 return TcPlan{};
         }
@@ -982,7 +982,7 @@ TcPlan make_mat64_plan(int op, int64_t nx, int64_t ny, int64_t ncx, int64_t ncy,
         // 15.2 / 9.8; 93 x 114, L = 377 / 420, d = 5, order 0, 2500 5.1 / 5.8.  Several: 80 x 80, L = 300, d = 8, order 1,
         // 725 4.5 / 7.1, 1450 4.5 / 4.4, 2133 4.5 / 3.4; symmetric, 47 paths, L = 1786, d = 11, order 1, 113 22.8 / 145;
         // symmetric, 120 paths, L = 250, d = 11, order 3, 2420 9.9 / 10.8).
-        const int least = band && Rs < 16 ? 6 : (sym && !band && order >= 2) || (band && !sym && d < 8) ? 24 : 12;
+        const int least = band && Rs < 16 ? 6 : (sym && !band && order >= 2) || (band && d < 8) ? 24 : 12;
         if (multi && pairs < t.fewest * sms * least) return TcPlan{};
         return t;
     }

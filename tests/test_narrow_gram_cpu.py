@@ -35,7 +35,8 @@ def test_no_matrix_in_chunks_of_few_pairs(lib, monkeypatch, op, nx, ny, lx, ly, 
     (GRAM, 24, 12, 765, 580, 8, 0), (SYM, 24, 24, 537, 537, 8, 0), (SYM, 11, 11, 690, 690, 9, 0),
     (GRAM, 34, 34, 153, 173, 8, 2), (SYM, 81, 81, 128, 128, 8, 3), (GRAM, 40, 40, 150, 167, 8, 3),
     (SYM, 120, 120, 200, 200, 8, 2), (GRAM, 90, 90, 300, 317, 8, 2),
-    (SYM, 266, 266, 442, 442, 6, 0), (GRAM, 93, 114, 377, 420, 5, 0), (GRAM, 38, 22, 371, 310, 3, 0)])
+    (SYM, 266, 266, 442, 442, 6, 0), (GRAM, 93, 114, 377, 420, 5, 0), (GRAM, 38, 22, 371, 310, 3, 0),
+    (GRAM, 37, 24, 554, 605, 8, 0), (GRAM, 27, 36, 625, 608, 8, 0), (SYM, 178, 178, 399, 399, 5, 0)])
 def test_no_matrix_where_it_measured_slower(lib, monkeypatch, op, nx, ny, lx, ly, d, order):
     """Several bands with few pairs, few dimensions at orders 2 and 3, chunks that fill the device once at most."""
     default, fused = sizes(lib, monkeypatch, op, nx, ny, lx, ly, d, order)
